@@ -269,8 +269,8 @@ def _head_depth(width, height, camera):
     def dev(a):
         return torch.as_tensor(a, device="cuda", dtype=torch.float64)
 
-    vp = dev(M.to_rows(camera.proj(width, height)) @ M.to_rows(camera.view()))
-    inv = torch.linalg.inv(vp)
+    vp = M.to_rows(camera.proj(width, height)) @ M.to_rows(camera.view())
+    vp, inv = dev(vp), dev(np.linalg.inv(vp))
     xs = (torch.arange(width, device="cuda", dtype=torch.float64) + 0.5) / width * 2.0 - 1.0
     ys = 1.0 - (torch.arange(height, device="cuda", dtype=torch.float64) + 0.5) / height * 2.0
     y, x = torch.meshgrid(ys, xs, indexing="ij")
