@@ -118,6 +118,47 @@ __device__ __forceinline__ RowSpan makeRowSpan(const ProjSeg& s) {
   return r;
 }
 
+// The pixels of a row of a box that can pass the four edge tests, for the
+// kernels that share a box's rows out over lanes.  Along a row an edge bounds x
+// on one side at o.x + (y - o.y) * slope, slope = e.x / e.y: from below where
+// e.y > 0, from above where e.y < 0.  A segment keeps up to two bounds of each
+// kind as lines a + row * s in the box's (or tile's) own pixel coordinates; an
+// edge that is nearly level (|slope| > 64) or far from the box is left out,
+// which only widens the span.  The bounds are moved out by 1/64 px: with
+// |slope| <= 64 and every term below 8,192 the errors of the approximate slope,
+// of the line's evaluation and of the fp32 edge test itself add up to less than
+// 0.01 px, so every pixel the exact test accepts is in the span, and the exact
+// test still decides each pixel of it.
+constexpr float SPAN_MARGIN = 1.0f / 64.0f;
+struct SpanLines { float4 lo, hi; };  // (a, s) of two lower bounds; of two upper ones
+__device__ __forceinline__ SpanLines spanLines(const f2 (&o)[4], const f2 (&d)[4], float x0, float y0, float rows) {
+  SpanLines L;
+  L.lo = make_float4(-1e9f, 0.0f, -1e9f, 0.0f);
+  L.hi = make_float4(1e9f, 0.0f, 1e9f, 0.0f);
+  bool lo1 = false, hi1 = false;  // the first slot is taken
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const float s = __fdividef(d[i].x, d[i].y), dy = y0 - o[i].y, dx = o[i].x - x0;
+    const float a = dx + dy * s;
+    const bool use = fabsf(d[i].x) <= 64.0f * fabsf(d[i].y) && fabsf(d[i].y) > 1e-9f && fabsf(dx) < 8192.0f &&
+                     (fabsf(dy) + rows) * fabsf(s) < 8192.0f;
+    if (!use) continue;
+    if (d[i].y > 0.0f) {
+      if (!lo1) { L.lo.x = a - SPAN_MARGIN; L.lo.y = s; } else { L.lo.z = a - SPAN_MARGIN; L.lo.w = s; }
+      lo1 = true;
+    } else {
+      if (!hi1) { L.hi.x = a + SPAN_MARGIN; L.hi.y = s; } else { L.hi.z = a + SPAN_MARGIN; L.hi.w = s; }
+      hi1 = true;
+    }
+  }
+  return L;
+}
+// Row r's span within [x0, x1] (x0 > x1: empty).
+__device__ __forceinline__ void spanOf(const float4& lo, const float4& hi, float r, int& x0, int& x1) {
+  x0 = max(x0, __float2int_ru(fmaxf(__fmaf_rn(r, lo.y, lo.x), __fmaf_rn(r, lo.w, lo.z))));
+  x1 = min(x1, __float2int_rd(fminf(__fmaf_rn(r, hi.y, hi.x), __fmaf_rn(r, hi.w, hi.z))));
+}
+
 // Block-wide exclusive prefix (all threads call; total = block sum).
 __device__ __forceinline__ uint32_t blockExclusiveScan(uint32_t v, uint32_t* warpSums, uint32_t& total) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -180,6 +221,7 @@ struct TrShared {
   float dp[4][TR_SEGS];                                                 // depthsProj
   float qsx[TR_SEGS], qsy[TR_SEGS], qax[TR_SEGS], qay[TR_SEGS], qd2[TR_SEGS], qlse[TR_SEGS], qws[TR_SEGS],
       qwe[TR_SEGS], qd22[TR_SEGS];                                      // QuadConst
+  float yd2[TR_SEGS], ylse[TR_SEGS], yd22[TR_SEGS];                     // QuadRecip
   uint32_t cx0[TR_SEGS], cy0[TR_SEGS], cw[TR_SEGS];  // candidate rectangle origin and width
   uint32_t tminx[TR_SEGS], tminy[TR_SEGS], tsx[TR_SEGS];
   float blo[TR_SEGS], bhi[TR_SEGS];  // depth range over which the bin follows from the depth alone
@@ -387,6 +429,8 @@ __device__ __forceinline__ void tilesRasterBody(const HfbUniforms& U, uint32_t P
       const QuadConst q = quadConst(s);
       sh.qsx[tid] = q.sm.x; sh.qsy[tid] = q.sm.y; sh.qax[tid] = q.ab.x; sh.qay[tid] = q.ab.y;
       sh.qd2[tid] = q.d2; sh.qlse[tid] = q.lse; sh.qws[tid] = q.wS; sh.qwe[tid] = q.wE; sh.qd22[tid] = q.d22;
+      const QuadRecip y = quadRecip(q);
+      sh.yd2[tid] = y.d2; sh.ylse[tid] = y.lse; sh.yd22[tid] = y.d22;
     }
   }
   // accumulators of the block's (segment, tile) pairs; segments beyond them walk alone
@@ -509,7 +553,7 @@ __device__ __forceinline__ void tilesRasterBody(const HfbUniforms& U, uint32_t P
       qc.d2 = sh.qd2[k]; qc.lse = sh.qlse[k]; qc.wS = sh.qws[k]; qc.wE = sh.qwe[k];
       qc.ab2 = mk2(sh.ex[3][k], sh.ey[3][k]);
       qc.d22 = sh.qd22[k];
-      const f2 wq = interpolateHairQuadPre(qc, mk2(sh.ox[3][k], sh.oy[3][k]), p);
+      const f2 wq = interpolateHairQuadPre(qc, {sh.yd2[k], sh.ylse[k], sh.yd22[k]}, mk2(sh.ox[3][k], sh.oy[3][k]), p);
       const float hd = interpolateHairF32(wq, mk4(sh.dp[0][k], sh.dp[1][k], sh.dp[2][k], sh.dp[3][k]));
       const float zb = loadTex2DClamp(depth, W, H, (int)x, (int)H - (int)y);
       if (hd > zb) continue;  // depth test, :193-195
@@ -1004,17 +1048,24 @@ tileSortKernel(uint32_t T, uint32_t NB, uint32_t bucketSize, const uint32_t* __r
 // STAGE segments -- short bins share a round, a long bin spans several -- and
 // each round runs in three phases:
 //   A1  one thread per (segment, row of the segment's tile-local bounding
-//       box): the four edge tests of processHairSegment (:5-20) on every
-//       pixel of the row into a bit mask; the passing pixels that are not
-//       done are appended to a list, one shared atomic per warp;
-//   A2  one thread per passing pair: segment-space interpolation, the depth
+//       box): the row's span (spanOf) without the pixels that are done; the
+//       spans' pixels are listed in (segment, row, x) order through a block
+//       scan of their counts;
+//   A2  one thread per listed pixel: the four edge tests of
+//       processHairSegment (:5-20), segment-space interpolation, the depth
 //       test and the fragment colour (:21-53), rounded through f16 like
 //       pack2x16float (hairSlicesDataBuffer.ts:50-63);
 //   B   one thread per pixel: the pixel's fragments in list order, found
-//       through a per-pixel bit mask over the round's segments.
-// A pixel covers ~4 of the ~25 pixels of a segment's box at 1080p, so the
-// pair phases keep the lanes busy where a pixel-per-thread walk of the list
-// would idle most of them.  Each slice of a pixel keeps the closed form of
+//       through a per-pixel bit mask over the round's segments and the place
+//       of its row's span in the list.
+// A segment covers ~4 of the ~25 pixels of its box at 1080p, so the list holds
+// what the edge tests accept and little else, and the phases keep the lanes
+// busy where a pixel-per-thread walk of the segments would idle most of them.
+// The kernel is bound by issue and by the barriers between the phases: what
+// counts is instructions per record and full rounds.  Against edge tests of every
+// box pixel, with rounds cut at PAIRS box pixels: 150 -> 109 us (10,000 x 32 at
+// 1920x1080, 16 px tiles), 222 -> 154 us (11,400 x 16, 8 px tiles, 8 slices), 320 ->
+// 176 us (7,001 x 23 at 1361x767, 32 px), 7.2 -> 4.2 ms (200,000 x 32 at 4K).  Each slice of a pixel keeps the closed form of
 // its front-to-back blend in registers: fragments arrive back to front
 // (descending key) and acc = f + (1 - f.a) * acc, which equals the
 // reference's per-slice linked list reduced front to back
@@ -1035,9 +1086,36 @@ constexpr uint32_t RUN_ENDS = 1u << 31;
 constexpr uint32_t FINE_SPLIT_MIN = 256;  // records: tiles below this are never split
 
 template <int TS> struct FineDims;
-template <> struct FineDims<8> { static constexpr uint32_t STAGE = 64, PAIRS = 768; };
-template <> struct FineDims<16> { static constexpr uint32_t STAGE = 128, PAIRS = 2048; };  // 96: 2-3 % slower, 160: 4 % slower
-template <> struct FineDims<32> { static constexpr uint32_t STAGE = 256, PAIRS = 4096; };
+// PAIRS: listed pixels of a round (and, in a careful group, box pixels: fineTile); ROWS:
+// box rows (a few per thread); CTAS: CTAs per SM that fineScheduleBody shares a frame's
+// records out over, by slices (4, 8, 16) -- a constant, not the occupancy, so that where
+// a tile is split, and with it the last bits of its pixels, does not depend on the build
+template <> struct FineDims<8> {
+  static constexpr uint32_t STAGE = 64, PAIRS = 768, ROWS = 512, CTAS[3] = {8, 6, 6};
+};
+template <> struct FineDims<16> {
+  static constexpr uint32_t STAGE = 128, PAIRS = 2048, ROWS = 2048, CTAS[3] = {3, 2, 2};  // 96: 2-3 % slower, 160: 4 % slower
+};
+template <> struct FineDims<32> {
+  static constexpr uint32_t STAGE = 256, PAIRS = 4096, ROWS = 4096, CTAS[3] = {1, 1, 1};
+};
+
+// A box row's place in the round's list: the row's listed pixels (bit x), and
+// the list index of the first.
+template <int TS> struct FineRow {
+  uint32_t v;  // pixels | first << 16
+  __device__ __forceinline__ void set(uint32_t pixels, uint32_t first) { v = pixels | (first << 16); }
+  __device__ __forceinline__ uint32_t pixels() const { return v & 0xffffu; }
+  __device__ __forceinline__ uint32_t at(uint32_t x) const {
+    return (v >> 16) + (uint32_t)__popc(v & ((1u << x) - 1u));
+  }
+};
+template <> struct FineRow<32> {
+  uint32_t p, f;
+  __device__ __forceinline__ void set(uint32_t pixels, uint32_t first) { p = pixels; f = first; }
+  __device__ __forceinline__ uint32_t pixels() const { return p; }
+  __device__ __forceinline__ uint32_t at(uint32_t x) const { return f + (uint32_t)__popc(p & ((1u << x) - 1u)); }
+};
 
 // Shared inputs of the fine pass.
 struct FineArgs {
@@ -1055,23 +1133,27 @@ struct FineArgs {
 
 template <int TS>
 struct FineSmem {
-  static constexpr uint32_t NT = TS * TS, STAGE = FineDims<TS>::STAGE, PAIRS = FineDims<TS>::PAIRS;
-  static_assert(PAIRS >= NT, "a segment box covers up to TS*TS pairs");
+  static constexpr uint32_t NT = TS * TS, STAGE = FineDims<TS>::STAGE, PAIRS = FineDims<TS>::PAIRS, ROWS = FineDims<TS>::ROWS;
+  static_assert(PAIRS >= NT && ROWS >= TS, "any one segment fits in a round");
+  static_assert(PAIRS <= 65536 && ROWS % NT == 0, "FineRow's first index is 16 bits; rows per thread");
   static_assert(2 * 6 * STAGE * sizeof(float) <= PAIRS * sizeof(uint2), "stagePoint's scratch fits in frag");
   float4 shade[STAGE][NSHADE];   // the shading entries each staged segment can sample
-  uint2 frag[PAIRS];             // A1: pixel | segment << 16 of a passing pair; A2: its colour as 4 x f16
-  uint32_t pairInfo[PAIRS];      // per box pair with a fragment (pixMask): fragment index | slice << 16
+  uint2 frag[PAIRS];             // A1: pixel | segment << 16 of a listed pixel; A2: its fragment's colour as 4 x f16
+  float4 spanLo[STAGE], spanHi[STAGE];  // SpanLines in tile pixels
+  uint8_t slice[PAIRS];          // A2: the fragment's slice
+  FineRow<TS> row[ROWS];         // the box rows of the staged segments, segment after segment
   // staged segments, one array per quantity (consecutive segments in consecutive banks)
   float ox[4][STAGE], oy[4][STAGE];  // first vertex of the four edge tests: v01, v11, v10, v00
   float ex[4][STAGE], ey[4][STAGE];  // second - first vertex of each edge test
   float dp[4][STAGE];                // depthsProj
   float qsx[STAGE], qsy[STAGE], qax[STAGE], qay[STAGE], qd2[STAGE], qlse[STAGE], qws[STAGE], qwe[STAGE],
       qd22[STAGE];                   // QuadConst
-  uint32_t strand[STAGE], segIdx[STAGE], listIdx[STAGE];
+  float yd2[STAGE], ylse[STAGE], yd22[STAGE];  // QuadRecip
+  uint32_t enc[STAGE], listIdx[STAGE];  // strand | segment << 24, place in the list
   uint32_t box[STAGE];               // tile-local pixel box x0 | y0 << 8 | x1 << 16 | y1 << 24
   uint32_t shadeBase[STAGE];         // first staged shading index | count << 16 | depth bin << 24
-  uint32_t pairBase[STAGE + 1];      // exclusive prefix of the box areas
   uint32_t rowBase[STAGE + 1];       // exclusive prefix of the box heights (A1's items)
+  uint32_t rowOff[STAGE];            // rowBase minus the box's first row: tile row y is row[rowOff + y]
   uint32_t cntEdge[STAGE], cntFrag[STAGE];
   uint32_t pixMask[STAGE / 32][NT];  // bit k of pixel p: staged segment k left a fragment at p
   // the tile
@@ -1086,7 +1168,7 @@ struct FineSmem {
   // the work item's instance (written by one thread per item): read where used, so that none of
   // it stays in registers across the tile's rounds
   FineArgs args;
-  uint32_t nRuns, nStaged, nSeg, passCount, queueIdx, bad, tileMode, total, walkNext;
+  uint32_t nRuns, nStaged, nSeg, passCount, segLimit, edgePasses, queueIdx, bad, tileMode, total, walkNext;
   uint32_t mode, cutSeg, cutSlots, roundFrags, e0, eLast, arrive;
 };
 
@@ -1140,11 +1222,11 @@ __device__ __forceinline__ uint32_t stageShade(FineSmem<TS>& sh, uint32_t k, uin
 // pixel-independent part of interpolateHairQuad, and the tile-local box of
 // the pixels that can pass the edge tests ([floor(min), ceil(max)] of the
 // vertices).  shade: first | count << 16 of its staged shading entries
-// (stageShade).  Returns the box area.
+// (stageShade).  Returns the box height (0: no pixel).
 template <int TS>
 __device__ __forceinline__ uint32_t stageFromProjection(FineSmem<TS>& sh, uint32_t k, uint32_t bin, const ProjSeg& s,
                                                         uint32_t shade, uint32_t x0, uint32_t y0) {
-  uint32_t box = EMPTY_BOX, area = 0, shadeBase = bin << 24;
+  uint32_t box = EMPTY_BOX, rows = 0, shadeBase = bin << 24;
   float mnx = floorf(fminf(fminf(s.v00.x, s.v01.x), fminf(s.v10.x, s.v11.x))) - (float)x0;
   float mny = floorf(fminf(fminf(s.v00.y, s.v01.y), fminf(s.v10.y, s.v11.y))) - (float)y0;
   float mxx = ceilf(fmaxf(fmaxf(s.v00.x, s.v01.x), fmaxf(s.v10.x, s.v11.x))) - (float)x0;
@@ -1153,17 +1235,20 @@ __device__ __forceinline__ uint32_t stageFromProjection(FineSmem<TS>& sh, uint32
     const uint32_t bx0 = (uint32_t)fmaxf(mnx, 0.0f), by0 = (uint32_t)fmaxf(mny, 0.0f);
     const uint32_t bx1 = (uint32_t)fminf(mxx, (float)(TS - 1)), by1 = (uint32_t)fminf(mxy, (float)(TS - 1));
     box = bx0 | (by0 << 8) | (bx1 << 16) | (by1 << 24);
-    area = (bx1 - bx0 + 1u) * (by1 - by0 + 1u);
+    rows = by1 - by0 + 1u;
     // edge tests in the order insideQuad evaluates them
     const f2 o[4] = {s.v01, s.v11, s.v10, s.v00};
-    const f2 e[4] = {s.v00, s.v01, s.v11, s.v10};
+    const f2 d[4] = {sub2(s.v00, s.v01), sub2(s.v01, s.v11), sub2(s.v11, s.v10), sub2(s.v10, s.v00)};
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       sh.ox[i][k] = o[i].x;
       sh.oy[i][k] = o[i].y;
-      sh.ex[i][k] = fsub(e[i].x, o[i].x);
-      sh.ey[i][k] = fsub(e[i].y, o[i].y);
+      sh.ex[i][k] = d[i].x;
+      sh.ey[i][k] = d[i].y;
     }
+    const SpanLines sl = spanLines(o, d, (float)x0, (float)y0, (float)TS);
+    sh.spanLo[k] = sl.lo;
+    sh.spanHi[k] = sl.hi;
     sh.dp[0][k] = s.depthsProj.x;
     sh.dp[1][k] = s.depthsProj.y;
     sh.dp[2][k] = s.depthsProj.z;
@@ -1171,13 +1256,15 @@ __device__ __forceinline__ uint32_t stageFromProjection(FineSmem<TS>& sh, uint32
     const QuadConst q = quadConst(s);
     sh.qsx[k] = q.sm.x; sh.qsy[k] = q.sm.y; sh.qax[k] = q.ab.x; sh.qay[k] = q.ab.y;
     sh.qd2[k] = q.d2; sh.qlse[k] = q.lse; sh.qws[k] = q.wS; sh.qwe[k] = q.wE; sh.qd22[k] = q.d22;
+    const QuadRecip y = quadRecip(q);
+    sh.yd2[k] = y.d2; sh.ylse[k] = y.lse; sh.yd22[k] = y.d22;
     shadeBase |= shade;
   }
   sh.box[k] = box;
   sh.shadeBase[k] = shadeBase;
   sh.cntEdge[k] = 0;
   sh.cntFrag[k] = 0;
-  return area;
+  return rows;
 }
 
 // Projects staged segment k (both points, projectSegment) and stages it.
@@ -1186,7 +1273,7 @@ __device__ __forceinline__ uint32_t stageSegment(FineSmem<TS>& sh, uint32_t k, u
                                                  const float4* __restrict__ pos, const float4* __restrict__ tan,
                                                  const float4* __restrict__ shading, uint32_t S, uint32_t P,
                                                  uint32_t SP, f2 size, uint32_t x0, uint32_t y0) {
-  const uint32_t st = sh.strand[k], sg = sh.segIdx[k];
+  const uint32_t st = sh.enc[k] & 0x00ffffffu, sg = sh.enc[k] >> 24;
   if (st < S && sg + 1u < P) {  // otherwise not a segment of this hair: covers no pixel
     const ProjSeg s = projectSegment(U, pos, tan, P, st, sg, size);
     return stageFromProjection<TS>(sh, k, bin, s, stageShade<TS>(sh, k, st, sg, shading, P, SP), x0, y0);
@@ -1203,7 +1290,7 @@ template <int TS>
 __device__ __forceinline__ uint32_t stageCached(FineSmem<TS>& sh, uint32_t k, uint32_t bin,
                                                 const float4* __restrict__ proj, const float4* __restrict__ shading,
                                                 uint32_t S, uint32_t P, uint32_t SP, uint32_t x0, uint32_t y0) {
-  const uint32_t st = sh.strand[k], sg = sh.segIdx[k];
+  const uint32_t st = sh.enc[k] & 0x00ffffffu, sg = sh.enc[k] >> 24;
   if (st < S && sg + 1u < P) {
     const float4* q = proj + ((size_t)st * (P - 1u) + sg) * SEG_PROJ_VEC4;
     const float4 a = __ldg(HFB_G(&q[0])), b = __ldg(HFB_G(&q[1])), d = __ldg(HFB_G(&q[2]));
@@ -1233,7 +1320,7 @@ __device__ __forceinline__ void stagePoint(FineSmem<TS>& sh, uint32_t k, uint32_
                                            f2 size) {
   constexpr uint32_t STAGE = FineSmem<TS>::STAGE;
   float* pt = reinterpret_cast<float*>(sh.frag) + end * 6u * STAGE;  // [6][STAGE] per end
-  const uint32_t st = sh.strand[k], sg = sh.segIdx[k];
+  const uint32_t st = sh.enc[k] & 0x00ffffffu, sg = sh.enc[k] >> 24;
   if (!(st < S && sg + 1u < P)) return;
   const size_t i = (size_t)st * P + sg + end;
   f2 o0, o1;
@@ -1254,7 +1341,7 @@ template <int TS>
 __device__ __forceinline__ uint32_t stageFromPoints(FineSmem<TS>& sh, uint32_t k, uint32_t bin, uint32_t S,
                                                     uint32_t P, uint32_t x0, uint32_t y0) {
   constexpr uint32_t STAGE = FineSmem<TS>::STAGE;
-  const uint32_t st = sh.strand[k], sg = sh.segIdx[k];
+  const uint32_t st = sh.enc[k] & 0x00ffffffu, sg = sh.enc[k] >> 24;
   if (!(st < S && sg + 1u < P)) {
     sh.box[k] = EMPTY_BOX;
     sh.shadeBase[k] = bin << 24;
@@ -1284,7 +1371,7 @@ __device__ __forceinline__ uint2 fragmentColour(const FineSmem<TS>& sh, uint32_t
   float alpha = fsub(1.0f, fabsf(fsub(fmul(w.x, 2.0f), 1.0f)));
   if (alphaQuadratic) alpha = sqrtf(alpha);
   alpha = sat(fmul(alpha, alphaMul));
-  const float tFull = fadd((float)sh.segIdx[k], w.y) / (float)(P - 1u);
+  const float tFull = fadd((float)(sh.enc[k] >> 24), w.y) / (float)(P - 1u);
   uint32_t i0, i1;
   const float fr = remapToIndices(SP, tFull, i0, i1);
   const uint32_t sbase = sh.shadeBase[k];
@@ -1294,7 +1381,7 @@ __device__ __forceinline__ uint2 fragmentColour(const FineSmem<TS>& sh, uint32_t
     c0 = sh.shade[k][i0 - e0];
     c1 = sh.shade[k][i1 - e0];
   } else {
-    const size_t sb = (size_t)sh.strand[k] * SP;
+    const size_t sb = (size_t)(sh.enc[k] & 0x00ffffffu) * SP;
     c0 = __ldg(HFB_G(&shading[sb + i0]));
     c1 = __ldg(HFB_G(&shading[sb + i1]));
   }
@@ -1309,7 +1396,8 @@ __device__ __forceinline__ uint2 fragmentColour(const FineSmem<TS>& sh, uint32_t
 __device__ __forceinline__ float halfLo(uint32_t v) { return __half2float(__ushort_as_half((unsigned short)(v & 0xffffu))); }
 __device__ __forceinline__ float halfHi(uint32_t v) { return __half2float(__ushort_as_half((unsigned short)(v >> 16))); }
 
-// acc[slice] = f + (1 - f.a) * acc[slice]
+// acc[slice] = f + (1 - f.a) * acc[slice], the colours with one rounding; alpha, which decides
+// when a pixel is done, with the two of the reference's product and sum
 template <int MAXL>
 __device__ __forceinline__ void blendFragment(f4 (&acc)[MAXL], uint32_t sl, uint2 h) {
   const f4 q = mk4(halfLo(h.x), halfHi(h.x), halfLo(h.y), halfHi(h.y));
@@ -1317,9 +1405,9 @@ __device__ __forceinline__ void blendFragment(f4 (&acc)[MAXL], uint32_t sl, uint
 #pragma unroll
   for (int si = 0; si < MAXL; si++) {
     if ((uint32_t)si == sl) {
-      acc[si].x = fadd(q.x, fmul(kk, acc[si].x));
-      acc[si].y = fadd(q.y, fmul(kk, acc[si].y));
-      acc[si].z = fadd(q.z, fmul(kk, acc[si].z));
+      acc[si].x = __fmaf_rn(kk, acc[si].x, q.x);
+      acc[si].y = __fmaf_rn(kk, acc[si].y, q.y);
+      acc[si].z = __fmaf_rn(kk, acc[si].z, q.z);
       acc[si].w = fadd(q.w, fmul(kk, acc[si].w));
     }
   }
@@ -1357,15 +1445,24 @@ __device__ __forceinline__ uint32_t buildRuns(FineSmem<TS>& sh, uint32_t B, uint
 // Rasterizes depth bins [b0, b1) of tile tileIdx in order, every pixel
 // starting from an empty colour (processTile per bin + reduceHairSlices,
 // hairFinePass.wgsl.ts:205-288), and leaves each pixel's colour in fin.
-// With `independent`, the bins are a later part of a split tile: every pixel
-// in view takes part, and the call gives up (returns false) as soon as a bin
-// could fill its fragment pool, whose cut would depend on which pixels the
-// earlier bins finished.
+// With `part` IN_ORDER the bins start the tile.  Otherwise they are a later part
+// of a split tile: every pixel in view takes part, and the call gives up
+// (FINE_UNSAFE) where a bin could fill its fragment pool, whose cut would depend
+// on which pixels the earlier bins finished.  Where it gives up decides whether
+// the tile is merged from its parts or drawn in order, which shows in the pixels
+// (up to the 0.001 that a finished pixel still lacks), so the decision must not
+// depend on how tight the listed pixels are: CAREFUL takes rounds of at most
+// PAIRS box pixels and counts what the edge tests accept, and its running bound
+// exceeds a bin's own count by less than PAIRS.  QUICK takes full rounds and
+// counts listed pixels; while a bin's count stays PAIRS below the pool, CAREFUL
+// would not give up either; past that it returns FINE_AGAIN, for CAREFUL to decide.
+enum FinePart : uint32_t { FINE_IN_ORDER = 0, FINE_QUICK, FINE_CAREFUL };
+enum FineEnd : uint32_t { FINE_OK = 0, FINE_UNSAFE, FINE_AGAIN };
 template <int TS, int MAXL>
-__device__ __forceinline__ bool fineTile(FineSmem<TS>& sh, const HfbUniforms& U, const FineArgs& a,
-                                         uint32_t tileIdx, uint32_t b0, uint32_t b1, bool independent, f4& fin) {
+__device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms& U, const FineArgs& a,
+                                         uint32_t tileIdx, uint32_t b0, uint32_t b1, FinePart part, f4& fin) {
   using SM = FineSmem<TS>;
-  constexpr uint32_t NT = SM::NT, STAGE = SM::STAGE, PAIRS = SM::PAIRS, NW = NT / 32u;
+  constexpr uint32_t NT = SM::NT, STAGE = SM::STAGE, PAIRS = SM::PAIRS, ROWS = SM::ROWS, NW = NT / 32u;
   constexpr uint32_t MODE_FAST = 0, MODE_TIGHTEN = 1, MODE_ABORT = 2;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const uint32_t lx = tid % TS, ly = tid / TS;
@@ -1475,8 +1572,7 @@ __device__ __forceinline__ bool fineTile(FineSmem<TS>& sh, const HfbUniforms& U,
         const uint32_t b = sh.runBin[r] & 0xffu;
         const uint32_t idx = sh.head[b].z - 1u - (sh.runOff[r] + k - sh.runK0[r]);
         const uint32_t enc = HFB_EXPECT(idx < maxDrawn) ? __ldg(HFB_G(&a.segBuf[1u + 2u * idx])) : 0xffffffffu;
-        sh.strand[k] = enc & 0x00ffffffu;
-        sh.segIdx[k] = enc >> 24;
+        sh.enc[k] = enc;
         sh.listIdx[k] = idx;
       }
     } else {
@@ -1508,8 +1604,7 @@ __device__ __forceinline__ bool fineTile(FineSmem<TS>& sh, const HfbUniforms& U,
           }
           const uint32_t cnt = firstIn ? first + 1u : first;
           if (lane < cnt) {
-            sh.strand[m + lane] = e.x & 0x00ffffffu;
-            sh.segIdx[m + lane] = e.x >> 24;
+            sh.enc[m + lane] = e.x;
             sh.listIdx[m + lane] = cand;
           }
           m += cnt;
@@ -1546,7 +1641,7 @@ __device__ __forceinline__ bool fineTile(FineSmem<TS>& sh, const HfbUniforms& U,
         for (uint32_t k = tid; k < nStaged; k += NT) {
           uint32_t r = 0;
           while (r + 1u < nRuns && sh.runK0[r + 1u] <= k) r++;
-          sh.pairBase[k] = stageCached<TS>(sh, k, sh.runBin[r] & 0xffu, a.proj, a.shading, a.S, a.P, a.SP, tbp.x0,
+          sh.rowBase[k] = stageCached<TS>(sh, k, sh.runBin[r] & 0xffu, a.proj, a.shading, a.S, a.P, a.SP, tbp.x0,
                                            tbp.y0);
         }
       } else if constexpr (2u * STAGE <= NT) {
@@ -1559,23 +1654,23 @@ __device__ __forceinline__ bool fineTile(FineSmem<TS>& sh, const HfbUniforms& U,
         for (uint32_t k = tid; k < nStaged; k += NT) {
           uint32_t r = 0;
           while (r + 1u < nRuns && sh.runK0[r + 1u] <= k) r++;
-          sh.pairBase[k] = stageFromPoints<TS>(sh, k, sh.runBin[r] & 0xffu, a.S, a.P, tbp.x0, tbp.y0);
+          sh.rowBase[k] = stageFromPoints<TS>(sh, k, sh.runBin[r] & 0xffu, a.S, a.P, tbp.x0, tbp.y0);
         }
       } else {
         for (uint32_t k = tid; k < nStaged; k += NT) {
           uint32_t r = 0;
           while (r + 1u < nRuns && sh.runK0[r + 1u] <= k) r++;
-          sh.pairBase[k] = stageSegment<TS>(sh, k, sh.runBin[r] & 0xffu, U, a.pos, a.tan, a.shading, a.S, a.P,
+          sh.rowBase[k] = stageSegment<TS>(sh, k, sh.runBin[r] & 0xffu, U, a.pos, a.tan, a.shading, a.S, a.P,
                                             a.SP, size, tbp.x0, tbp.y0);
         }
       }
       __syncthreads();
-      // exclusive prefix of the areas; the round keeps the longest prefix
-      // of segments whose pairs fit
+      // exclusive prefix of the box heights (low half) and areas (high half) together, all
+      // chunks of 32 segments at once (independent shuffle chains); the halves cannot carry
+      // into each other: at most STAGE * TS * TS and STAGE * TS, below 2^16 up to 16 px
+      // tiles.  The round keeps the longest prefix of segments whose rows fit (and, in a
+      // CAREFUL part, at most PAIRS box pixels)
       if (warp == 0) {
-        // the box areas (high half) and heights (low half) scanned together, all chunks of
-        // 32 segments at once (independent shuffle chains); the halves cannot carry into each
-        // other: at most STAGE * TS * TS and STAGE * TS, below 2^16 up to 16 px tiles
         using V = std::conditional_t<(TS <= 16), uint32_t, unsigned long long>;
         constexpr uint32_t SH = TS <= 16 ? 16u : 32u, NC = STAGE / 32u;
         constexpr V LOW = ((V)1 << SH) - 1u;
@@ -1583,9 +1678,8 @@ __device__ __forceinline__ bool fineTile(FineSmem<TS>& sh, const HfbUniforms& U,
 #pragma unroll
         for (uint32_t c = 0; c < NC; c++) {
           const uint32_t k = c * 32u + lane;
-          const uint32_t a = k < nStaged ? sh.pairBase[k] : 0u;
-          const uint32_t rows = a ? (sh.box[k] >> 24) - ((sh.box[k] >> 8) & 0xffu) + 1u : 0u;
-          val[c] = ((V)a << SH) | rows;
+          const uint32_t rows = k < nStaged ? sh.rowBase[k] : 0u, box = k < nStaged ? sh.box[k] : 0u;
+          val[c] = ((V)(rows ? rows * (((box >> 16) & 0xffu) - (box & 0xffu) + 1u) : 0u) << SH) | rows;
           incl[c] = val[c];
         }
 #pragma unroll
@@ -1596,150 +1690,143 @@ __device__ __forceinline__ bool fineTile(FineSmem<TS>& sh, const HfbUniforms& U,
             if (lane >= (uint32_t)o) incl[c] += y;
           }
         }
-        V carryBoth = 0;
+        V carry = 0;
         uint32_t nSeg = nStaged;
 #pragma unroll
         for (uint32_t c = 0; c < NC; c++) {
           const uint32_t k = c * 32u + lane;
-          const V ex = carryBoth + incl[c] - val[c];
+          const uint32_t ex = (uint32_t)((carry + incl[c] - val[c]) & LOW);
           if (k < nStaged) {
-            sh.pairBase[k] = (uint32_t)(ex >> SH);
-            sh.rowBase[k] = (uint32_t)(ex & LOW);
+            sh.rowBase[k] = ex;
+            sh.rowOff[k] = ex - ((sh.box[k] >> 8) & 0xffu);
           }
-          const uint32_t over =
-              __ballot_sync(0xffffffffu, k < nStaged && (uint32_t)((carryBoth + incl[c]) >> SH) > PAIRS);
+          const V end = carry + incl[c];
+          const uint32_t over = __ballot_sync(0xffffffffu, k < nStaged && ((uint32_t)(end & LOW) > ROWS ||
+                                                                           (part == FINE_CAREFUL && (uint32_t)(end >> SH) > PAIRS)));
           if (over && nSeg == nStaged) nSeg = c * 32u + (uint32_t)(__ffs(over) - 1);
-          carryBoth += __shfl_sync(0xffffffffu, incl[c], 31);
+          carry += __shfl_sync(0xffffffffu, incl[c], 31);
         }
-        const uint32_t carry = (uint32_t)(carryBoth >> SH), carryRows = (uint32_t)(carryBoth & LOW);
         if (lane == 0) {
-          sh.pairBase[nStaged] = carry;
-          sh.rowBase[nStaged] = carryRows;
-          sh.passCount = 0;
-          if (nSeg < nStaged) {  // drop the segments from nSeg on
-            if (tileMode) {
-              uint32_t used;
-              sh.nRuns = buildRuns<TS>(sh, b1, bin, off, nSeg, used);
-            } else {
-              sh.runK1[0] = nSeg;
-              sh.runBin[0] &= ~RUN_ENDS;
-            }
-          }
+          sh.rowBase[nStaged] = (uint32_t)(carry & LOW);
           sh.nSeg = nSeg;
+          sh.segLimit = nSeg;
+          sh.passCount = 0xffffffffu;
+          sh.edgePasses = 0;
         }
       }
       __syncthreads();
     }
     uint32_t nSeg = sh.nSeg;
-    nRuns = sh.nRuns;
-    const uint32_t nPairs = sh.pairBase[nSeg];
 
-    // ---------------- A1: edge tests, one thread per (segment, box row) ----------------
-    // A thread tests every pixel of a box row (the row term of edgeFunction,
-    // swRasterizeHair.wgsl.ts:128-130, formed once) into a bit mask, drops the
-    // pixels that are done, and appends the rest with one shared atomic per warp.
+    // ---------------- A1: the box rows' spans, one thread per (segment, row) ----------------
+    // Each thread takes consecutive rows: it counts its rows' pixels that are in their
+    // span and not done, a block scan places them, and it writes them to the list.  A
+    // segment whose pixels do not fit any more ends the round (any first one fits).
     {
       const uint32_t nRows = sh.rowBase[nSeg];
-      const uint32_t per = divCeil(nRows, NT);
-      uint32_t it0 = tid * per;
-      const uint32_t itEnd = min(it0 + per, nRows);
-      uint32_t k = 0, ry = 0, myCnt = 0, bx0 = 0, bx1 = 0, by0 = 0, bh = 0;
-      float eox[4], eey[4];
-      auto loadSeg = [&](uint32_t kk) {
-        const uint32_t bx = sh.box[kk];
-        bx0 = bx & 0xffu;
-        by0 = (bx >> 8) & 0xffu;
-        bx1 = (bx >> 16) & 0xffu;
-        bh = (bx >> 24) - by0 + 1u;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          eox[i] = sh.ox[i][kk]; eey[i] = sh.ey[i][kk];
-        }
-      };
-      if (it0 < itEnd) {
-        uint32_t lo = 0, hi = nSeg;  // last k with rowBase[k] <= it0
+      const uint32_t per = divCeil(nRows, NT);  // at most ROWS / NT
+      const uint32_t r0 = min(tid * per, nRows), r1 = min(r0 + per, nRows);
+      uint32_t k = 0, kFirst = 0, cnt = 0;
+      if (r0 < r1) {
+        uint32_t lo = 0, hi = nSeg;  // last k with rowBase[k] <= r0
         while (hi - lo > 1u) {
           const uint32_t mid = (lo + hi) >> 1;
-          if (sh.rowBase[mid] <= it0) lo = mid; else hi = mid;
+          if (sh.rowBase[mid] <= r0) lo = mid; else hi = mid;
         }
-        k = lo;
-        loadSeg(k);
-        ry = it0 - sh.rowBase[k];
-      }
-      for (uint32_t it = 0; it < per; it++) {
-        const bool valid = it0 < itEnd;
-        uint32_t live = 0, rowPix = 0;
-        if (valid) {
-          const uint32_t qy = by0 + ry;
-          const float py = (float)(tbp.y0 + qy);
-          float rowT[4];
-#pragma unroll
-          for (int i = 0; i < 4; i++) rowT[i] = fmul(fsub(py, sh.oy[i][k]), sh.ex[i][k]);
-          uint32_t bits = 0;
-#pragma unroll
-          for (uint32_t qx = 0; qx < (uint32_t)TS; qx++) {
-            if (qx < bx0 || qx > bx1) continue;
-            const float px = (float)(tbp.x0 + qx);
-            bool pass = true;
-#pragma unroll
-            for (int i = 0; i < 4; i++) {  // edgeFunction >= 0
-              const float C = fsub(fmul(fsub(px, eox[i]), eey[i]), rowT[i]);
-              pass = pass && C >= 0.0f;
-            }
-            bits |= pass ? 1u << qx : 0u;
+        k = kFirst = lo;
+        uint32_t end = sh.rowBase[k + 1u], box = sh.box[k];
+        float4 sLo = sh.spanLo[k], sHi = sh.spanHi[k];
+        uint32_t off = sh.rowOff[k];
+        for (uint32_t r = r0; r < r1; r++) {
+          if (r >= end) {  // next segment with rows
+            do { end = sh.rowBase[++k + 1u]; } while (end <= r);
+            box = sh.box[k];
+            sLo = sh.spanLo[k];
+            sHi = sh.spanHi[k];
+            off = sh.rowOff[k];
           }
-          rowPix = qy * TS;
-          const uint32_t rowDone = (sh.doneMask[rowPix >> 5] >> (rowPix & 31u)) &
-                                   (TS == 32 ? 0xffffffffu : ((1u << (TS & 31)) - 1u));
-          live = bits & ~rowDone;
+          const uint32_t qy = r - off;
+          int xa = (int)(box & 0xffu), xb = (int)((box >> 16) & 0xffu);
+          spanOf(sLo, sHi, (float)qy, xa, xb);
+          uint32_t live = 0;
+          if (xa <= xb) {
+            const uint32_t rowPix = qy * TS;
+            live = (0xffffffffu << xa) & (0xffffffffu >> (31 - xb)) & ~(sh.doneMask[rowPix >> 5] >> (rowPix & 31u));
+          }
+          sh.row[r].set(live, 0u);
+          cnt += (uint32_t)__popc(live);
         }
-        // warp-aggregated append of the row's pixels
-        const uint32_t n = (uint32_t)__popc(live);
-        uint32_t incl = n;
+      }
+      // exclusive prefix of the counts in thread order
+      uint32_t incl = cnt;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= (uint32_t)o) incl += y;
-        }
-        const uint32_t warpTotal = __shfl_sync(0xffffffffu, incl, 31);
-        if (warpTotal) {
-          uint32_t base = 0;
-          if (lane == 31) base = atomicAdd(&sh.passCount, warpTotal);
-          base = __shfl_sync(0xffffffffu, base, 31) + incl - n;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+      }
+      if (lane == 31) sh.red[warp] = incl;
+      __syncthreads();
+      uint32_t pos = incl - cnt;
+      for (uint32_t w = 0; w < warp; w++) pos += sh.red[w];
+      if (tid == NT - 1u) atomicMin(&sh.passCount, pos + cnt);  // the total: every row's, unless the list fills up
+      if (r0 < r1) {
+        uint32_t end = sh.rowBase[kFirst + 1u], off = sh.rowOff[kFirst], myCnt = 0;
+        k = kFirst;
+        for (uint32_t r = r0; r < r1; r++) {
+          if (r >= end) {
+            if (myCnt && part != FINE_CAREFUL) atomicAdd(&sh.cntEdge[k], myCnt);
+            myCnt = 0;
+            do { end = sh.rowBase[++k + 1u]; } while (end <= r);
+            off = sh.rowOff[k];
+          }
+          uint32_t live = sh.row[r].pixels();
+          const uint32_t n = (uint32_t)__popc(live);
+          if (pos + n > PAIRS) {  // the rows before this one fit
+            atomicMin(&sh.segLimit, k);
+            atomicMin(&sh.passCount, pos);
+            break;
+          }
+          sh.row[r].set(live, pos);
+          const uint32_t tag = (r - off) * TS | (k << 16);
           while (live) {
             const uint32_t qx = (uint32_t)(__ffs(live) - 1);
             live &= live - 1u;
-            if (HFB_EXPECT(base < PAIRS)) sh.frag[base].x = (rowPix + qx) | (k << 16);
-            base++;
+            if (HFB_EXPECT(pos < PAIRS)) sh.frag[pos].x = tag + qx;
+            pos++;
           }
+          myCnt += n;
         }
-        myCnt += n;
-        if (valid) {
-          it0++;
-          if (++ry == bh) {  // segment done
-            if (myCnt) atomicAdd(&sh.cntEdge[k], myCnt);
-            myCnt = 0;
-            if (it0 < itEnd) {
-              while (sh.rowBase[k + 1u] <= it0) k++;  // next segment with rows
-              loadSeg(k);
-              ry = 0;
-            }
-          }
-        }
+        if (myCnt && part != FINE_CAREFUL) atomicAdd(&sh.cntEdge[k], myCnt);
       }
-      if (myCnt) atomicAdd(&sh.cntEdge[k], myCnt);
     }
     __syncthreads();
+    nSeg = sh.segLimit;
+    if (nSeg < sh.nStaged) {  // uniform: drop the segments from nSeg on
+      if (tid == 0) {
+        sh.nSeg = nSeg;
+        if (tileMode) {
+          uint32_t used;
+          sh.nRuns = buildRuns<TS>(sh, b1, bin, off, nSeg, used);
+        } else {
+          sh.runK1[0] = nSeg;
+          sh.runBin[0] &= ~RUN_ENDS;
+        }
+      }
+      __syncthreads();
+    }
+    nRuns = sh.nRuns;
 
     // ---------------- can a bin fill its pool in this round? ----------------
-    // The edge-test passes bound the fragments: when the passes of the whole
-    // round, on top of what the cursor's bin may already hold, fit in a pool,
-    // no bin can fill its pool and nothing needs counting (the common case:
-    // every thread sees passCount after the barrier above).  Otherwise one
-    // warp sums the passes run by run.  e0 / eLast carry the bounds of the
-    // first and last run (the round's total where it is enough).
+    // The listed pixels bound the fragments: when those of the whole round, on
+    // top of what the cursor's bin may already hold, fit in a pool, no bin can
+    // fill its pool and nothing needs counting (the common case: every thread
+    // sees passCount after the barrier above).  Otherwise one warp sums the
+    // listed pixels run by run.  e0 / eLast carry the bounds of the first and
+    // last run (the round's total where it is enough).  A CAREFUL part checks
+    // after A2, which counts what the edge tests accept.
+    const uint32_t cap = part == FINE_QUICK ? (a.CAP > PAIRS ? a.CAP - PAIRS : 0u) : a.CAP;
     uint32_t mode = MODE_FAST, e0 = sh.passCount, eLast = e0;
-    if (runningUB + e0 > a.CAP) {
+    auto sumRuns = [&]() {  // by run, with the warp 0; all threads call
       if (warp == 0) {
         uint32_t wmode = MODE_FAST, keep = nRuns, we0 = 0, weLast = 0;
         for (uint32_t r = 0; r < nRuns; r++) {
@@ -1748,13 +1835,13 @@ __device__ __forceinline__ bool fineTile(FineSmem<TS>& sh, const HfbUniforms& U,
           e = __reduce_add_sync(0xffffffffu, e);
           const uint32_t base = r == 0u ? runningUB : 0u;
           if (r == 0u) we0 = e;
-          if (base + e > a.CAP) {
+          if (base + e > cap) {
             if (r == 0u) { wmode = MODE_TIGHTEN; keep = 1; } else { keep = r; }
             break;
           }
           weLast = e;
         }
-        if (independent && (wmode == MODE_TIGHTEN || keep < nRuns)) wmode = MODE_ABORT;
+        if (part != FINE_IN_ORDER && (wmode == MODE_TIGHTEN || keep < nRuns)) wmode = MODE_ABORT;
         if (lane == 0) {
           sh.mode = wmode;
           sh.e0 = we0;
@@ -1770,9 +1857,12 @@ __device__ __forceinline__ bool fineTile(FineSmem<TS>& sh, const HfbUniforms& U,
       mode = sh.mode;
       e0 = sh.e0;
       eLast = sh.eLast;
-      if (mode == MODE_ABORT) return false;  // a pool could fill: this group cannot stand alone
       nRuns = sh.nRuns;
       nSeg = sh.nSeg;
+    };
+    if (part != FINE_CAREFUL && runningUB + e0 > cap) {
+      sumRuns();
+      if (mode == MODE_ABORT) return FINE_AGAIN;
     }
     bool exact = false;
     if (mode == MODE_TIGHTEN) {
@@ -1782,13 +1872,14 @@ __device__ __forceinline__ bool fineTile(FineSmem<TS>& sh, const HfbUniforms& U,
       exact = runningUB + e0 > a.CAP;
     }
 
-    // ---------------- A2: fragments, one thread per passing pair ----------------
+    // ---------------- A2: fragments, one thread per listed pixel ----------------
     {
       // the arguments this phase reads, in registers for the phase only
       const uint32_t P = a.P, SP = a.SP, L = a.L, alphaQuadratic = a.alphaQuadratic;
       const float alphaMul = a.alphaMul;
       const float4* __restrict__ shading = a.shading;
       const uint32_t nPass = sh.passCount;
+      uint32_t accepted = 0;
       for (uint32_t i = tid; i < nPass; i += NT) {
         const uint32_t e = sh.frag[i].x;
         const uint32_t pix = e & 0xffffu, k = e >> 16;
@@ -1796,13 +1887,22 @@ __device__ __forceinline__ bool fineTile(FineSmem<TS>& sh, const HfbUniforms& U,
         if (!HFB_EXPECT(i < PAIRS && k < STAGE && pix < NT)) continue;
         const uint32_t qx = pix % TS, qy = pix / TS;
         const f2 pf = mk2((float)(tbp.x0 + qx), (float)(tbp.y0 + qy));
+        bool inside = true;
+#pragma unroll
+        for (int j = 0; j < 4; j++)  // edgeFunction >= 0
+          inside = inside && fsub(fmul(fsub(pf.x, sh.ox[j][k]), sh.ey[j][k]), fmul(fsub(pf.y, sh.oy[j][k]), sh.ex[j][k])) >= 0.0f;
+        if (!inside) continue;
+        if (part == FINE_CAREFUL) {
+          accepted++;
+          atomicAdd(&sh.cntEdge[k], 1u);
+        }
         QuadConst qc;
         qc.sm = mk2(sh.qsx[k], sh.qsy[k]);
         qc.ab = mk2(sh.qax[k], sh.qay[k]);
         qc.d2 = sh.qd2[k]; qc.lse = sh.qlse[k]; qc.wS = sh.qws[k]; qc.wE = sh.qwe[k];
         qc.ab2 = mk2(sh.ex[3][k], sh.ey[3][k]);
         qc.d22 = sh.qd22[k];
-        const f2 w = interpolateHairQuadPre(qc, mk2(sh.ox[3][k], sh.oy[3][k]), pf);
+        const f2 w = interpolateHairQuadPre(qc, {sh.yd2[k], sh.ylse[k], sh.yd22[k]}, mk2(sh.ox[3][k], sh.oy[3][k]), pf);
         const float hd = interpolateHairF32(w, mk4(sh.dp[0][k], sh.dp[1][k], sh.dp[2][k], sh.dp[3][k]));
         if (!(hd < sh.zbuf[pix])) continue;  // depth test with GL_LESS (skip when >=)
         const uint32_t kb = sh.shadeBase[k] >> 24;
@@ -1811,14 +1911,20 @@ __device__ __forceinline__ bool fineTile(FineSmem<TS>& sh, const HfbUniforms& U,
         const uint2 col = fragmentColour<TS>(sh, k, w, hd, P, SP, L, td0, td1, alphaQuadratic, alphaMul, shading,
                                              slice);
         sh.frag[i] = col;
-        const uint32_t bx = sh.box[k];
-        sh.pairInfo[sh.pairBase[k] + (qy - ((bx >> 8) & 0xffu)) * (((bx >> 16) & 0xffu) - (bx & 0xffu) + 1u) +
-                    (qx - (bx & 0xffu))] = i | (slice << 16);
+        sh.slice[i] = (uint8_t)slice;
         atomicOr(&sh.pixMask[k >> 5][pix], 1u << (k & 31u));
         if (exact) atomicAdd(&sh.cntFrag[k], 1u);
       }
+      if (accepted) atomicAdd(&sh.edgePasses, accepted);
     }
     __syncthreads();
+    if (part == FINE_CAREFUL) {
+      e0 = eLast = sh.edgePasses;
+      if (runningUB + e0 > cap) {
+        sumRuns();
+        if (mode == MODE_ABORT) return FINE_UNSAFE;  // a pool could fill: this part cannot stand alone
+      }
+    }
 
     // ---------------- exact accounting: the segment that fills the pool ----------------
     if (exact) {
@@ -1858,7 +1964,7 @@ __device__ __forceinline__ bool fineTile(FineSmem<TS>& sh, const HfbUniforms& U,
       const uint32_t cut = sh.cutSeg;
       if (cut != INVALID_PTR) {  // slots of the filling segment in pixel order
         const uint32_t b = sh.box[cut], bxa = b & 0xffu, bya = (b >> 8) & 0xffu;
-        const uint32_t bw = ((b >> 16) & 0xffu) - bxa + 1u, area = sh.pairBase[cut + 1u] - sh.pairBase[cut];
+        const uint32_t bw = ((b >> 16) & 0xffu) - bxa + 1u, area = bw * ((b >> 24) - bya + 1u);
         const uint32_t pix = tid < area ? (bya + tid / bw) * TS + bxa + tid % bw : 0u;
         const uint32_t bit = 1u << (cut & 31u);
         const bool has = tid < area && (sh.pixMask[cut >> 5][pix] & bit) != 0u;
@@ -1880,12 +1986,9 @@ __device__ __forceinline__ bool fineTile(FineSmem<TS>& sh, const HfbUniforms& U,
           while (bits) {
             const uint32_t j = w * 32u + (uint32_t)(__ffs(bits) - 1);
             bits &= bits - 1u;
-            const uint32_t b = sh.box[j];
-            const uint32_t bx0 = b & 0xffu, by0 = (b >> 8) & 0xffu;
-            const uint32_t info =
-                sh.pairInfo[sh.pairBase[j] + (ly - by0) * (((b >> 16) & 0xffu) - bx0 + 1u) + (lx - bx0)];
-            if (HFB_EXPECT((info & 0xffffu) < PAIRS)) {
-              blendFragment<MAXL>(acc, info >> 16, sh.frag[info & 0xffffu]);
+            const uint32_t at = sh.row[sh.rowOff[j] + ly].at(lx);
+            if (HFB_EXPECT(at < PAIRS)) {
+              blendFragment<MAXL>(acc, sh.slice[at], sh.frag[at]);
               nFrag++;
               pending++;
             }
@@ -1957,7 +2060,7 @@ __device__ __forceinline__ bool fineTile(FineSmem<TS>& sh, const HfbUniforms& U,
     if (__syncthreads_and(done)) break;
     if (bin >= b1) break;
   }
-  return true;
+  return FINE_OK;
 }
 
 // Builds the work list of the fine pass: one item per drawn tile, in the
@@ -2087,9 +2190,16 @@ __device__ __forceinline__ void fineItem(FineSmem<TS>& sh, const HfbUniforms& U,
       return;
     }
     f4 fin;
+    FinePart part = split && g > 0u ? FINE_QUICK : FINE_IN_ORDER;
     while (true) {
-      const bool ok = fineTile<TS, MAXL>(sh, U, a, tileIdx, b0, b1, split && g > 0u, fin);
+      const FineEnd end = fineTile<TS, MAXL>(sh, U, a, tileIdx, b0, b1, part, fin);
+      if (end == FINE_AGAIN) {  // uniform
+        part = FINE_CAREFUL;
+        __syncthreads();
+        continue;
+      }
       if (!split) break;
+      const bool ok = end == FINE_OK;
       // a group of a split tile: publish its composite; the last to arrive merges
       (*HFB_G(&fs.groups[(size_t)(item.z + g) * NT + tid])) = make_float4(fin.x, fin.y, fin.z, fin.w);
       __threadfence();
@@ -2107,6 +2217,7 @@ __device__ __forceinline__ void fineItem(FineSmem<TS>& sh, const HfbUniforms& U,
         b0 = 0;
         b1 = a.B;
         split = false;
+        part = FINE_IN_ORDER;
         continue;
       }
       __threadfence();
@@ -2201,6 +2312,13 @@ fineBatch(BatchView b, FineArgs base, HfbConfig cfgParam) {
   }
 }
 
+// CTAs that the schedule shares a frame's records out over.
+template <int TS, int MAXL>
+uint32_t fineShare(const HfbCtx* c) {
+  return c->cfg.processorCount ? c->cfg.processorCount
+                               : FineDims<TS>::CTAS[MAXL == 4 ? 0 : MAXL == 8 ? 1 : 2] * (uint32_t)c->smCount;
+}
+
 template <int TS, int MAXL>
 cudaError_t launchFineT(HfbCtx* c, const HfbUniforms& u, const HfbHairData& h, const float* pos,
                         const float* tan, const float* shading, const float* depth, HfbRasterBuffers& rb,
@@ -2217,12 +2335,13 @@ cudaError_t launchFineT(HfbCtx* c, const HfbUniforms& u, const HfbHairData& h, c
     if (perSM < 1) return cudaErrorInvalidConfiguration;
   }
   const uint32_t grid = cfg.processorCount ? cfg.processorCount : (uint32_t)(perSM * c->smCount);
+  const uint32_t share = fineShare<TS, MAXL>(c);
   const uint32_t T = divCeil(rb.width, TS) * divCeil(rb.height, TS);
   const uint32_t dispMode = u.displayMode & 0xffu;
   const bool dbg = dispMode == 4u && ((u.displayMode >> 8) & 0xffffu) != 0u;
   FineScratch fs = fineScratchLayout(rb.scratch, cfg, rb.width, rb.height);
   fineScheduleKernel<<<1, 1024, 0, c->stream>>>(rb.tileList, rb.segmentCountPerTile, (const uint4*)rb.tiles, T,
-                                                cfg.tileDepthBins, grid, rb.maxDrawnSegments,
+                                                cfg.tileDepthBins, share, rb.maxDrawnSegments,
                                                 h.strandsCount * h.pointsPerStrand, dbg ? 0u : 1u, fs,
                                                 (DeviceCounters*)c->dCounters);
   HFB_AFTER_LAUNCH(c, "fineScheduleKernel");
@@ -2391,7 +2510,7 @@ cudaError_t launchFineBatchT(HfbCtx* c, const BatchView& b) {
   DeviceCounters* dc = (DeviceCounters*)c->dCounters;
   uint32_t& sgrid = c->batchGrid[BK_SCHEDULE];
   if (!sgrid) sgrid = c->smCount;
-  fineScheduleBatch<<<batchLaunchGrid(c, sgrid), 1024, 0, c->stream>>>(b, cfg, batchLaunchGrid(c, grid), dc);
+  fineScheduleBatch<<<batchLaunchGrid(c, sgrid), 1024, 0, c->stream>>>(b, cfg, batchLaunchGrid(c, fineShare<TS, MAXL>(c)), dc);
   HFB_AFTER_LAUNCH(c, "fineScheduleBatch");
   fineItemPrefixBatch<<<1, 1024, 0, c->stream>>>(b, cfg);
   HFB_AFTER_LAUNCH(c, "fineItemPrefixBatch");

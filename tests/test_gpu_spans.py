@@ -1,0 +1,43 @@
+"""The kernels that list a segment's pixels row by row from conservative spans
+(raster.cu spanLines): at sizes where the lists, the rounds and the split
+tiles' decisions have their edges, against the CPU oracle."""
+import numpy as np
+import pytest
+
+from helpers import small_instance
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA GPU", allow_module_level=True)
+
+from test_gpu_parity import _fine_vs_oracle, oracle  # noqa: E402,F401
+
+
+@pytest.mark.parametrize("tile,slices", [(8, 4), (8, 8), (16, 4), (16, 8), (32, 4), (32, 8)])
+@pytest.mark.parametrize("fiber,strands", [(2e-2, 400), (2e-3, 1500), (2e-5, 1500)])
+def test_fine_pass_segments_of_every_width(oracle, tile, slices, fiber, strands):  # noqa: F811
+    """Segments that cover whole tiles (a round's list fills up before its
+    segments do), ordinary ones, and ones thinner than a pixel (most rows'
+    spans are empty); a ragged viewport, so edge tiles are partial."""
+    inst = small_instance(strands=strands, width=301, height=217, tile_size=tile, slices=slices, fiber_radius=fiber,
+                          avg_segments_per_tile=2048)
+    cnt, g, o = _fine_vs_oracle(oracle, inst)
+    err = np.abs(g - o)
+    assert err.max() <= 1.0 / 255.0, f"max pixel error {err.max():.4g} (> 1/255)"
+    assert np.array_equal(g[:, 3] > 0, o[:, 3] > 0), "coverage differs"
+
+
+@pytest.mark.parametrize("tile", [8, 16])
+@pytest.mark.parametrize("avg", [4, 9])
+def test_fine_pass_split_tiles_near_a_full_pool(oracle, tile, avg):  # noqa: F811
+    """Split tiles whose bins hold about a pool's worth of fragments: parts
+    that stay clear of it, that are taken again with exact counts, and that
+    send the tile to the in-order walk."""
+    inst = small_instance(strands=6000, points=32, width=320, height=240, tile_size=tile, depth_bins=4, slices=4)
+    inst.cfg.avg_fragments_per_slice = avg
+    cnt, g, o = _fine_vs_oracle(oracle, inst)
+    assert cnt["fineSplitTiles"] > 0, "no tile was split: the test does not test"
+    err = np.abs(g - o)
+    assert err.max() <= 1.0 / 255.0, f"max pixel error {err.max():.4g} (> 1/255)"
