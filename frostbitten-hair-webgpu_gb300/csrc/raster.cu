@@ -190,47 +190,65 @@ __device__ __forceinline__ uint32_t blockExclusiveScan(uint32_t v, uint32_t* war
 // ---------------------------------------------------------------------------
 // 1. tilesRaster: HairTilesPass.main + processTile, hairTilesPass.wgsl.ts:70-238
 //
-// A block takes TR_SEGS consecutive segments.  The candidate pixels of a
-// segment are its bounding rectangle clipped to the pixels the tiles cover
-// ([0, W - 1) x [0, H - 1): getTileBoundsPx clamps the tile ends to W - 1 /
-// H - 1), each belonging to tile (x / TS, y / TS).  The block then runs:
-//   A1  one thread per (segment, candidate pixel) pair: the edge tests;
-//       passing pairs are appended to the warp's region of a list;
-//   A2  one thread per passing pixel: interpolated depth, the depth test
-//       against the scene and, where the bin does not follow from the depth
-//       range (binRange), the view-space depth bin, folded into the
-//       (segment, tile) accumulators with shared-memory atomics (min / max
-//       over an order-preserving u32 image of the depth, min of the bin):
-//       the result does not depend on the order;
-//   E   one thread per (segment, tile): the record, as processTile stores
-//       it (:220-237).
-// A segment whose tiles do not fit the block's accumulators is walked by its
-// own thread, tile by tile (rasterSegmentSerial).
+// A warp takes 32 consecutive segments, one per lane, and needs no other warp:
+// there is no block barrier.  The candidate pixels of a segment are its bounding
+// rectangle clipped to the pixels the tiles cover ([0, W - 1) x [0, H - 1):
+// getTileBoundsPx clamps the tile ends to W - 1 / H - 1), each belonging to tile
+// (x / TS, y / TS).  After projecting, the warp works in rounds of as many of its
+// segments as have room for their (segment, tile) accumulators:
+//   R  the rectangles' rows are shared out over the lanes (the owner of row i
+//      found by a search over the lanes' row counts), each narrowed to its span
+//      (spanOf);
+//   P  the spans' pixels are shared out over the lanes the same way: the edge
+//      tests, interpolated depth, the depth test against the scene and, where the
+//      bin does not follow from the depth range (binRange), the view-space depth
+//      bin, folded into the (segment, tile) accumulators with shared-memory
+//      atomics (min / max over an order-preserving u32 image of the depth, min of
+//      the bin): the result does not depend on the order;
+//   E  one lane per (segment, tile): the record, as processTile stores it
+//      (:220-237).
+// A segment whose tiles do not fit the accumulators alone, or whose rectangle is
+// enormous, is walked by its own lane, tile by tile (rasterSegmentSerial).
+//
+// Bound by issue: an fp32 projection with IEEE roots and quotients per segment,
+// then what each row and each covered pixel costs.  Against edge tests of every
+// rectangle pixel, four warps sharing one list between block barriers: 92 -> 58 us
+// (10,000 x 32 at 1920x1080, 16 px tiles), 98 -> 64 us (11,400 x 16, 8 px tiles),
+// 2.65 -> 1.58 ms (200,000 x 32 at 4K), 3.14 -> 2.43 ms (64 instances).
 // ---------------------------------------------------------------------------
 constexpr uint32_t TR_SEGS = TILES_RASTER_SEGS;  // segments (and threads) per block
-// (segment, tile) accumulators per block and list entries per A1 / A2 round: the
-// single-instance kernel keeps more of a large frame's long segments in
-// shared memory (768, 2,048: 6 CTAs per SM); the batched one, whose
-// instances are smaller, trades them for a seventh CTA (512, 1,024).
-constexpr uint32_t TR_SLOTS = 768, TR_CHUNK = 2048;
-constexpr uint32_t TR_SLOTS_BATCH = 512, TR_CHUNK_BATCH = 1024;
+constexpr uint32_t TR_SLOTS = 256;               // (segment, tile) accumulators per warp
 
-template <uint32_t TR_SLOTS, uint32_t TR_CHUNK>
 struct TrShared {
-  float ox[4][TR_SEGS], oy[4][TR_SEGS], ex[4][TR_SEGS], ey[4][TR_SEGS];  // edge tests (insideQuad order)
-  float dp[4][TR_SEGS];                                                 // depthsProj
-  float qsx[TR_SEGS], qsy[TR_SEGS], qax[TR_SEGS], qay[TR_SEGS], qd2[TR_SEGS], qlse[TR_SEGS], qws[TR_SEGS],
-      qwe[TR_SEGS], qd22[TR_SEGS];                                      // QuadConst
-  float yd2[TR_SEGS], ylse[TR_SEGS], yd22[TR_SEGS];                     // QuadRecip
-  uint32_t cx0[TR_SEGS], cy0[TR_SEGS], cw[TR_SEGS];  // candidate rectangle origin and width
-  uint32_t tminx[TR_SEGS], tminy[TR_SEGS], tsx[TR_SEGS];
-  float blo[TR_SEGS], bhi[TR_SEGS];  // depth range over which the bin follows from the depth alone
-  uint32_t pairBase[TR_SEGS + 1], slotBase[TR_SEGS + 1];
-  uint32_t accMin[TR_SLOTS], accMax[TR_SLOTS], accBin[TR_SLOTS];
-  uint32_t pass[TR_CHUNK];  // segment | column in the rectangle << 7 | row << 19, one region per warp
-  uint32_t warpSums[32];
-  uint32_t regionCount[TR_SEGS / 32];  // entries in each warp's region of pass
+  float4 ox[TR_SEGS], oy[TR_SEGS], ex[TR_SEGS], ey[TR_SEGS];  // edge tests (insideQuad order)
+  float4 dp[TR_SEGS];                                         // depthsProj
+  float4 q0[TR_SEGS], q1[TR_SEGS], q2[TR_SEGS];  // QuadConst: sm, ab | d2, lse, wS, wE | d22, QuadRecip
+  float4 spanLo[TR_SEGS], spanHi[TR_SEGS];       // SpanLines in the rectangle's pixels
+  float2 bin[TR_SEGS];       // depth range over which the bin follows from the depth alone
+  uint4 rect[TR_SEGS];       // first column and row, width, tiles per row
+  uint2 tile[TR_SEGS];       // first tile's column and row
+  uint32_t slotBase[TR_SEGS];
+  uint32_t accMin[TR_SEGS / 32][TR_SLOTS], accMax[TR_SEGS / 32][TR_SLOTS], accBin[TR_SEGS / 32][TR_SLOTS];
 };
+
+// Inclusive prefix over the warp.
+__device__ __forceinline__ uint32_t warpInclusive(uint32_t v, uint32_t lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= (uint32_t)o) v += y;
+  }
+  return v;
+}
+// The lane that owns item i when the lanes' inclusive item counts are incl: the
+// number of lanes with incl <= i (31 past the last item).  All lanes call it.
+__device__ __forceinline__ uint32_t warpOwner(uint32_t incl, uint32_t i) {
+  uint32_t o = 0;
+#pragma unroll
+  for (uint32_t s = 16; s > 0; s >>= 1)
+    if (__shfl_sync(0xffffffffu, incl, o + s - 1u) <= i) o += s;
+  return o;
+}
 
 // order-preserving u32 image of a float (NaN excluded by the caller)
 __device__ __forceinline__ uint32_t orderedBits(float f) {
@@ -353,16 +371,15 @@ __device__ void rasterSegmentSerial(const HfbUniforms& U, const ProjSeg& s, uint
   }
 }
 
-template <uint32_t TR_SLOTS, uint32_t TR_CHUNK>
 __device__ __forceinline__ void tilesRasterBody(const HfbUniforms& U, uint32_t P, uint32_t nStrands, uint32_t TS,
                                                 uint32_t B, uint32_t threshold, float4 bsphere,
                                                 const float4* __restrict__ pos, const float4* __restrict__ tan,
                                                 const float* __restrict__ depth, uint4* __restrict__ tiles,
                                                 uint32_t* __restrict__ segBuf, uint32_t* __restrict__ segCount,
                                                 uint32_t* __restrict__ binCount,
-                                                DeviceCounters* __restrict__ counters, TrShared<TR_SLOTS, TR_CHUNK>& sh,
+                                                DeviceCounters* __restrict__ counters, TrShared& sh,
                                                 uint32_t blk, float4* __restrict__ projOut) {
-  const uint32_t tid = threadIdx.x, lane = tid & 31u;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, w0 = tid & ~31u;  // w0: the warp's first segment in sh
   const uint32_t segsPerStrand = P - 1u;
   const uint32_t nSeg = nStrands * segsPerStrand;
   const uint32_t gid = blk * TR_SEGS + tid;
@@ -373,11 +390,13 @@ __device__ __forceinline__ void tilesRasterBody(const HfbUniforms& U, uint32_t P
   // getHairDepthBoundsVS, :242-246
   const f4 bsVS = m4v(U.modelViewMat.m, mk4(bsphere.x, bsphere.y, bsphere.z, 1.0f));
   const float dv0 = fsub(bsVS.z, bsphere.w), dv1 = fadd(bsVS.z, bsphere.w);
-  const bool binRows = binRowsFromDepth(U.projMatrixInv.m);
   const uint32_t tsShift = (uint32_t)(__ffs((int)TS) - 1);  // TS is 8, 16 or 32
+  uint32_t* const accMin = sh.accMin[tid >> 5];
+  uint32_t* const accMax = sh.accMax[tid >> 5];
+  uint32_t* const accBin = sh.accBin[tid >> 5];
 
-  // ---- project this thread's segment ----
-  uint32_t pairs = 0, slots = 0, key = 0;
+  // ---- project this lane's segment ----
+  uint32_t rows = 0, slots = 0, key = 0;
   bool serial = false;
   ProjSeg s;
   uint32_t ux0 = 0, uy0 = 0, ux1 = 0, uy1 = 0;
@@ -397,205 +416,143 @@ __device__ __forceinline__ void tilesRasterBody(const HfbUniforms& U, uint32_t P
     const float bx0 = fmaxf(floorf(fminf(fminf(s.v00.x, s.v01.x), fminf(s.v10.x, s.v11.x))), 0.0f);
     const float by0 = fmaxf(floorf(fminf(fminf(s.v00.y, s.v01.y), fminf(s.v10.y, s.v11.y))), 0.0f);
     ux0 = f2u(bx0); uy0 = f2u(by0); ux1 = f2u(bx1); uy1 = f2u(by1);
-    const uint32_t tminx = ux0 / TS, tminy = uy0 / TS, tmaxx = ux1 / TS, tmaxy = uy1 / TS;
+    const uint32_t tminx = ux0 >> tsShift, tminy = uy0 >> tsShift, tmaxx = ux1 >> tsShift, tmaxy = uy1 >> tsShift;
     const uint32_t tsx = (tmaxx - tminx) + 1u, tsy = (tmaxy - tminy) + 1u;
     if (tsx * tsy <= threshold) {  // degenerate segment rejection, :111-117
       const uint32_t cx1 = min(ux1 + 1u, W - 1u), cy1 = min(uy1 + 1u, H - 1u);
       const uint32_t cwid = cx1 > ux0 ? cx1 - ux0 : 0u, chei = cy1 > uy0 ? cy1 - uy0 : 0u;
       if (cwid && chei) {
-        if ((uint64_t)cwid * chei >= (1ull << 24) || cwid > 4096u || chei > 8192u) {
-          serial = true;  // beyond the pair encoding: its own walk
+        if (cwid > 4096u || chei > 4096u || tsx * tsy > TR_SLOTS) {
+          serial = true;  // its own walk
         } else {
-          pairs = cwid * chei;
+          rows = chei;
           slots = tsx * tsy;
         }
       }
-      sh.cx0[tid] = ux0; sh.cy0[tid] = uy0; sh.cw[tid] = max(cwid, 1u);
-      sh.tminx[tid] = tminx; sh.tminy[tid] = tminy; sh.tsx[tid] = tsx;
-      const f2 o[4] = {s.v01, s.v11, s.v10, s.v00};  // the edge tests in insideQuad's order
-      const f2 e[4] = {s.v00, s.v01, s.v11, s.v10};
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        sh.ox[i][tid] = o[i].x;
-        sh.oy[i][tid] = o[i].y;
-        sh.ex[i][tid] = fsub(e[i].x, o[i].x);
-        sh.ey[i][tid] = fsub(e[i].y, o[i].y);
+      if (rows) {
+        const f2 o[4] = {s.v01, s.v11, s.v10, s.v00};  // the edge tests in insideQuad's order
+        const f2 d[4] = {sub2(s.v00, s.v01), sub2(s.v01, s.v11), sub2(s.v11, s.v10), sub2(s.v10, s.v00)};
+        sh.ox[tid] = make_float4(o[0].x, o[1].x, o[2].x, o[3].x);
+        sh.oy[tid] = make_float4(o[0].y, o[1].y, o[2].y, o[3].y);
+        sh.ex[tid] = make_float4(d[0].x, d[1].x, d[2].x, d[3].x);
+        sh.ey[tid] = make_float4(d[0].y, d[1].y, d[2].y, d[3].y);
+        sh.dp[tid] = make_float4(s.depthsProj.x, s.depthsProj.y, s.depthsProj.z, s.depthsProj.w);
+        const SpanLines sl = spanLines(o, d, (float)ux0, (float)uy0, (float)chei);
+        sh.spanLo[tid] = sl.lo;
+        sh.spanHi[tid] = sl.hi;
+        const QuadConst q = quadConst(s);
+        const QuadRecip y = quadRecip(q);
+        sh.q0[tid] = make_float4(q.sm.x, q.sm.y, q.ab.x, q.ab.y);
+        sh.q1[tid] = make_float4(q.d2, q.lse, q.wS, q.wE);
+        sh.q2[tid] = make_float4(q.d22, y.d2, y.lse, y.d22);
+        float blo, bhi;
+        binRange(U.projMatrixInv.m, binRowsFromDepth(U.projMatrixInv.m), s.depthsProj, blo, bhi);
+        sh.bin[tid] = make_float2(blo, bhi);
+        sh.rect[tid] = make_uint4(ux0, uy0, cwid, tsx);
+        sh.tile[tid] = make_uint2(tminx, tminy);
       }
-      sh.dp[0][tid] = s.depthsProj.x; sh.dp[1][tid] = s.depthsProj.y;
-      sh.dp[2][tid] = s.depthsProj.z; sh.dp[3][tid] = s.depthsProj.w;
-      float blo, bhi;
-      binRange(U.projMatrixInv.m, binRows, s.depthsProj, blo, bhi);
-      sh.blo[tid] = blo; sh.bhi[tid] = bhi;
-      const QuadConst q = quadConst(s);
-      sh.qsx[tid] = q.sm.x; sh.qsy[tid] = q.sm.y; sh.qax[tid] = q.ab.x; sh.qay[tid] = q.ab.y;
-      sh.qd2[tid] = q.d2; sh.qlse[tid] = q.lse; sh.qws[tid] = q.wS; sh.qwe[tid] = q.wE; sh.qd22[tid] = q.d22;
-      const QuadRecip y = quadRecip(q);
-      sh.yd2[tid] = y.d2; sh.ylse[tid] = y.lse; sh.yd22[tid] = y.d22;
     }
   }
-  // accumulators of the block's (segment, tile) pairs; segments beyond them walk alone
-  uint32_t slotTotal;
-  const uint32_t slotEx = blockExclusiveScan(slots, sh.warpSums, slotTotal);
-  if (slots && slotEx + slots > TR_SLOTS) {
-    serial = true;
-    pairs = 0;
-    slots = 0;
-  }
-  sh.slotBase[tid] = slotEx;
-  uint32_t pairTotal;
-  sh.pairBase[tid] = blockExclusiveScan(pairs, sh.warpSums, pairTotal);
-  if (tid == 0) sh.pairBase[TR_SEGS] = pairTotal;
-  for (uint32_t i = tid; i < TR_SLOTS; i += TR_SEGS) {
-    sh.accMin[i] = 0xffffffffu;
-    sh.accMax[i] = 0u;
-    sh.accBin[i] = B;
-  }
-  __syncthreads();
+  const uint32_t slotIncl = warpInclusive(slots, lane);
 
-  // Each thread walks one contiguous range of the block's pairs.  A round's
-  // A1 appends passing pairs to its warp's region of the list (a count kept
-  // in registers: no atomic) until a region is full; the warp then stops,
-  // its lanes at the pairs they have not yet appended, which the next round
-  // retests.  A2 then has a full list to share out, and the block meets at
-  // its barriers about once per TR_CHUNK passing pixels rather than once per
-  // TR_CHUNK candidate pairs.
-  // edgeFunction (swRasterizeHair.wgsl.ts:128-130) is (x - ox) * ey - (y - oy) * ex: the
-  // second product is the same along a row and is formed once per row (the same values)
-  constexpr uint32_t REGION = TR_CHUNK / (TR_SEGS / 32);
-  const uint32_t warp = tid >> 5;
-  const uint32_t per = divCeil(pairTotal, TR_SEGS);
-  uint32_t p = tid * per;
-  const uint32_t pEnd = min(p + per, pairTotal);
-  uint32_t k = 0, rx = 0, ry = 0, w = 1, x0 = 0, y0 = 0;
-  float eox[4], eey[4], rowT[4];
-  auto loadSeg = [&](uint32_t kk) {
-    x0 = sh.cx0[kk]; y0 = sh.cy0[kk]; w = sh.cw[kk];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      eox[i] = sh.ox[i][kk]; eey[i] = sh.ey[i][kk];
+  // rounds of the lanes [first, end) whose accumulators fit together
+  for (uint32_t first = 0; first < 32u;) {
+    const uint32_t base = first ? __shfl_sync(0xffffffffu, slotIncl, first - 1u) : 0u;
+    const uint32_t fit = __ballot_sync(0xffffffffu, lane >= first && slotIncl - base <= TR_SLOTS);
+    const uint32_t end = 32u - (uint32_t)__clz((int)fit);  // slotIncl grows: the fitting lanes are first .. end - 1
+    const uint32_t nSlots = __shfl_sync(0xffffffffu, slotIncl, end - 1u) - base;
+    const bool mine = lane >= first && lane < end;
+    const uint32_t rowIncl = warpInclusive(mine ? rows : 0u, lane);
+    const uint32_t nRows = __shfl_sync(0xffffffffu, rowIncl, 31);
+    if (mine) sh.slotBase[tid] = slotIncl - slots - base;
+    for (uint32_t i = lane; i < nSlots; i += 32u) {
+      accMin[i] = 0xffffffffu;
+      accMax[i] = 0u;
+      accBin[i] = B;
     }
-  };
-  auto setRow = [&]() {
-    const float py = (float)(y0 + ry);
-#pragma unroll
-    for (int i = 0; i < 4; i++) rowT[i] = fmul(fsub(py, sh.oy[i][k]), sh.ex[i][k]);
-  };
-  if (p < pEnd) {
-    uint32_t lo = 0, hi = TR_SEGS;  // last k with pairBase[k] <= p
-    while (hi - lo > 1u) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (sh.pairBase[mid] <= p) lo = mid; else hi = mid;
-    }
-    k = lo;
-    loadSeg(k);
-    const uint32_t r = p - sh.pairBase[k];
-    ry = r / w;
-    rx = r - ry * w;
-    setRow();
-  }
-  while (__syncthreads_or(p < pEnd)) {
-    // ---- A1: edge tests along the thread's range until the warp's region is full ----
-    uint32_t* const region = sh.pass + warp * REGION;
-    uint32_t cnt = 0;  // the warp's entries (the same in every lane)
-    while (cnt < REGION) {
-      const bool act = p < pEnd;
-      if (!__any_sync(0xffffffffu, act)) break;
-      bool pass = false;
-      if (act) {
-        const float px = (float)(x0 + rx);
-        pass = true;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {  // edgeFunction >= 0
-          const float C = fsub(fmul(fsub(px, eox[i]), eey[i]), rowT[i]);
-          pass = pass && C >= 0.0f;
-        }
+    __syncwarp();
+    for (uint32_t r0 = 0; r0 < nRows; r0 += 32u) {
+      // ---- R: one row per lane ----
+      const uint32_t ri = r0 + lane;
+      const uint32_t ro = warpOwner(rowIncl, ri) & 31u;
+      const uint32_t row = ri - __shfl_sync(0xffffffffu, rowIncl - (mine ? rows : 0u), ro);
+      int xa = 0, xb = -1;
+      if (ri < nRows) {
+        xb = (int)sh.rect[w0 + ro].z - 1;
+        spanOf(sh.spanLo[w0 + ro], sh.spanHi[w0 + ro], (float)row, xa, xb);
       }
-      const uint32_t bal = __ballot_sync(0xffffffffu, pass);
-      const uint32_t at = cnt + __popc(bal & ((1u << lane) - 1u));
-      const bool fits = !pass || at < REGION;  // else the region is full: the pair goes first next round
-      if (pass && fits && HFB_EXPECT(k < TR_SEGS)) region[at] = k | (rx << 7) | (ry << 19);
-      cnt = min(cnt + (uint32_t)__popc(bal), REGION);
-      if (act && fits) {
-        p++;
-        if (++rx == w) {
-          rx = 0;
-          ry++;
-          if (p < pEnd && p >= sh.pairBase[k + 1u]) {  // next segment with pairs
-            while (sh.pairBase[k + 1u] <= p) k++;
-            loadSeg(k);
-            ry = 0;
-          }
-          if (p < pEnd) setRow();
+      const uint32_t n = xb >= xa ? (uint32_t)(xb - xa + 1) : 0u;
+      const uint32_t incl = warpInclusive(n, lane);
+      const uint32_t nPix = __shfl_sync(0xffffffffu, incl, 31);
+      const uint32_t tag = ro | (row << 5);
+      const uint32_t xShift = (uint32_t)xa - (incl - n);
+      // ---- P: one pixel per lane ----
+      for (uint32_t c0 = 0; c0 < nPix; c0 += 32u) {
+        const uint32_t c = c0 + lane;
+        const uint32_t src = warpOwner(incl, c) & 31u;
+        const uint32_t t = __shfl_sync(0xffffffffu, tag, src), rx = __shfl_sync(0xffffffffu, xShift, src) + c;
+        if (c >= nPix) continue;
+        const uint32_t k = w0 + (t & 31u);
+        const uint4 rect = sh.rect[k];
+        const uint32_t x = rect.x + rx, y = rect.y + (t >> 5);
+        const f2 p = mk2((float)x, (float)y);
+        const float4 ox = sh.ox[k], oy = sh.oy[k], ex = sh.ex[k], ey = sh.ey[k];
+        // edgeFunction >= 0 (swRasterizeHair.wgsl.ts:128-130)
+        const bool inside = fsub(fmul(fsub(p.x, ox.x), ey.x), fmul(fsub(p.y, oy.x), ex.x)) >= 0.0f &&
+                            fsub(fmul(fsub(p.x, ox.y), ey.y), fmul(fsub(p.y, oy.y), ex.y)) >= 0.0f &&
+                            fsub(fmul(fsub(p.x, ox.z), ey.z), fmul(fsub(p.y, oy.z), ex.z)) >= 0.0f &&
+                            fsub(fmul(fsub(p.x, ox.w), ey.w), fmul(fsub(p.y, oy.w), ex.w)) >= 0.0f;
+        if (!inside) continue;
+        const float zb = loadTex2DClamp(depth, W, H, (int)x, (int)H - (int)y);
+        const float4 q0 = sh.q0[k], q1 = sh.q1[k], q2 = sh.q2[k], dp = sh.dp[k];
+        QuadConst qc;
+        qc.sm = mk2(q0.x, q0.y);
+        qc.ab = mk2(q0.z, q0.w);
+        qc.d2 = q1.x; qc.lse = q1.y; qc.wS = q1.z; qc.wE = q1.w;
+        qc.ab2 = mk2(ex.w, ey.w);
+        qc.d22 = q2.x;
+        const f2 wq = interpolateHairQuadPre(qc, {q2.y, q2.z, q2.w}, mk2(ox.w, oy.w), p);
+        const float hd = interpolateHairF32(wq, ld4(dp));
+        if (hd > zb) continue;  // depth test, :193-195
+        const uint2 tl = sh.tile[k];
+        const uint32_t slot = sh.slotBase[k] + ((y >> tsShift) - tl.y) * rect.w + ((x >> tsShift) - tl.x);
+        if (!HFB_EXPECT(slot < TR_SLOTS)) continue;
+        const float2 br = sh.bin[k];
+        if (!(hd >= br.x && hd <= br.y))  // else the record's bin comes from its depth range (E)
+          atomicMin(&accBin[slot], viewDepthBin(U, B, dv0, dv1, p, hd));
+        if (!isnan(hd)) {  // fminf / fmaxf ignore a NaN depth
+          atomicMin(&accMin[slot], orderedBits(hd));
+          atomicMax(&accMax[slot], orderedBits(hd));
         }
       }
     }
-    if (lane == 0) sh.regionCount[warp] = cnt;
-    __syncthreads();
-    // ---- A2: depth, depth test and bin of every passing pixel ----
-    uint32_t rc[TR_SEGS / 32], nPass = 0;
-#pragma unroll
-    for (uint32_t r = 0; r < TR_SEGS / 32; r++) {
-      rc[r] = sh.regionCount[r];
-      nPass += rc[r];
-    }
-    for (uint32_t i = tid; i < nPass; i += TR_SEGS) {
-      uint32_t r = 0, o = i;  // entry i of the regions laid end to end
-#pragma unroll
-      for (uint32_t q = 0; q + 1u < TR_SEGS / 32; q++)
-        if (r == q && o >= rc[q]) { o -= rc[q]; r++; }
-      const uint32_t e = sh.pass[r * REGION + o];
-      const uint32_t k = e & 0x7fu, rx = (e >> 7) & 0xfffu, ry = e >> 19;
-      const uint32_t x = sh.cx0[k] + rx, y = sh.cy0[k] + ry;
-      const f2 p = mk2((float)x, (float)y);
-      QuadConst qc;
-      qc.sm = mk2(sh.qsx[k], sh.qsy[k]);
-      qc.ab = mk2(sh.qax[k], sh.qay[k]);
-      qc.d2 = sh.qd2[k]; qc.lse = sh.qlse[k]; qc.wS = sh.qws[k]; qc.wE = sh.qwe[k];
-      qc.ab2 = mk2(sh.ex[3][k], sh.ey[3][k]);
-      qc.d22 = sh.qd22[k];
-      const f2 wq = interpolateHairQuadPre(qc, {sh.yd2[k], sh.ylse[k], sh.yd22[k]}, mk2(sh.ox[3][k], sh.oy[3][k]), p);
-      const float hd = interpolateHairF32(wq, mk4(sh.dp[0][k], sh.dp[1][k], sh.dp[2][k], sh.dp[3][k]));
-      const float zb = loadTex2DClamp(depth, W, H, (int)x, (int)H - (int)y);
-      if (hd > zb) continue;  // depth test, :193-195
-      const uint32_t slot =
-          sh.slotBase[k] + ((y >> tsShift) - sh.tminy[k]) * sh.tsx[k] + ((x >> tsShift) - sh.tminx[k]);
-      if (!HFB_EXPECT(slot < TR_SLOTS)) continue;
-      if (!(hd >= sh.blo[k] && hd <= sh.bhi[k]))  // else the record's bin comes from its depth range (E)
-        atomicMin(&sh.accBin[slot], viewDepthBin(U, B, dv0, dv1, p, hd));
-      if (!isnan(hd)) {  // fminf / fmaxf ignore a NaN depth
-        atomicMin(&sh.accMin[slot], orderedBits(hd));
-        atomicMax(&sh.accMax[slot], orderedBits(hd));
+    __syncwarp();
+    // ---- E: one record per (segment, tile) that took a pixel ----
+    const uint32_t slotEnd = mine ? slotIncl - base : lane < first ? 0u : nSlots;
+    for (uint32_t i0 = 0; i0 < nSlots; i0 += 32u) {
+      const uint32_t i = i0 + lane;
+      const uint32_t so = warpOwner(slotEnd, i) & 31u;
+      const uint32_t sKey = __shfl_sync(0xffffffffu, key, so);
+      if (i >= nSlots || accMin[i] == 0xffffffffu) continue;  // no pixel with a depth
+      const float dmin = orderedFloat(accMin[i]);
+      if (dmin > 1.0f) continue;
+      const uint32_t k = w0 + so, l = i - sh.slotBase[k], tsx = sh.rect[k].w;
+      const uint32_t ty = sh.tile[k].y + l / tsx, tx = sh.tile[k].x + l % tsx;
+      const float dmax = orderedFloat(accMax[i]);
+      uint32_t bin = accBin[i];
+      if (sh.bin[k].x <= sh.bin[k].y) {  // the smallest bin is at one end of the depths (binRange)
+        const f2 p0 = mk2(0.0f, 0.0f);
+        bin = min(bin, min(viewDepthBin(U, B, dv0, dv1, p0, dmin), viewDepthBin(U, B, dv0, dv1, p0, dmax)));
       }
+      storeTileRecord(tiles, segBuf, segCount, binCount, counters, maxDrawn, tilesX, B, tx, ty, bin, dmin, dmax, sKey,
+                      tilesX * divCeil(H, TS));
     }
-  }  // the loop's barrier ends A2 before the next round and before E
-
-  // ---- E: one record per (segment, tile) that took a pixel ----
-  for (uint32_t i = tid; i < slotTotal && i < TR_SLOTS; i += TR_SEGS) {
-    if (sh.accMin[i] == 0xffffffffu) continue;  // no pixel with a depth
-    const float dmin = orderedFloat(sh.accMin[i]);
-    if (dmin > 1.0f) continue;
-    uint32_t lo = 0, hi = TR_SEGS;  // segment of the slot: last k with slotBase[k] <= i
-    while (hi - lo > 1u) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (sh.slotBase[mid] <= i) lo = mid; else hi = mid;
-    }
-    const uint32_t k = lo, l = i - sh.slotBase[k];
-    const uint32_t ty = sh.tminy[k] + l / sh.tsx[k], tx = sh.tminx[k] + l % sh.tsx[k];
-    const uint32_t g = blk * TR_SEGS + k;
-    const uint32_t strand = g / segsPerStrand, seg = g - strand * segsPerStrand;
-    const float dmax = orderedFloat(sh.accMax[i]);
-    uint32_t bin = sh.accBin[i];
-    if (sh.blo[k] <= sh.bhi[k]) {  // the smallest bin is at one end of the depths (binRange)
-      const f2 p0 = mk2(0.0f, 0.0f);
-      bin = min(bin, min(viewDepthBin(U, B, dv0, dv1, p0, dmin), viewDepthBin(U, B, dv0, dv1, p0, dmax)));
-    }
-    storeTileRecord(tiles, segBuf, segCount, binCount, counters, maxDrawn, tilesX, B, tx, ty, bin, dmin, dmax,
-                    (strand << 8) | seg, tilesX * divCeil(H, TS));
+    __syncwarp();  // the accumulators are reused by the next round
+    first = end;
   }
   if (serial)
     rasterSegmentSerial(U, s, W, H, TS, B, tilesX, maxDrawn, dv0, dv1, key, ux0, uy0, ux1, uy1, depth, tiles,
                         segBuf, segCount, binCount, counters);
-  __syncthreads();  // the block's staging is reused by its next segments
 }
 
 __global__ void __launch_bounds__(TR_SEGS, 6)
@@ -604,9 +561,9 @@ tilesRasterKernel(const HfbUniforms U, uint32_t P, uint32_t nStrands, uint32_t T
                   const float4* __restrict__ tan, const float* __restrict__ depth, uint4* __restrict__ tiles,
                   uint32_t* __restrict__ segBuf, uint32_t* __restrict__ segCount,
                   uint32_t* __restrict__ binCount, DeviceCounters* __restrict__ counters, float4* __restrict__ proj) {
-  __shared__ TrShared<TR_SLOTS, TR_CHUNK> sh;
-  tilesRasterBody<TR_SLOTS, TR_CHUNK>(U, P, nStrands, TS, B, threshold, bsphere, pos, tan, depth, tiles, segBuf,
-                                      segCount, binCount, counters, sh, blockIdx.x, proj);
+  __shared__ TrShared sh;
+  tilesRasterBody(U, P, nStrands, TS, B, threshold, bsphere, pos, tan, depth, tiles, segBuf, segCount, binCount,
+                  counters, sh, blockIdx.x, proj);
 }
 
 // ---------------------------------------------------------------------------
@@ -2390,12 +2347,12 @@ cudaError_t launchFineT(HfbCtx* c, const HfbUniforms& u, const HfbHairData& h, c
     const TilesScratch ts = tilesScratchLayout(I.scratch, cfg, I.W, I.H, I.maxDrawn); \
     (void)ts;
 
-__global__ void __launch_bounds__(TR_SEGS, 7) tilesRasterBatch(BatchView b, HfbConfig cfgParam,
+__global__ void __launch_bounds__(TR_SEGS, 6) tilesRasterBatch(BatchView b, HfbConfig cfgParam,
                                                              DeviceCounters* __restrict__ counters) {
   const HfbConfig cfg = cfgParam;
-  __shared__ TrShared<TR_SLOTS_BATCH, TR_CHUNK_BATCH> sh;
+  __shared__ TrShared sh;
   BATCH_LOOP(BK_RASTER)
-    tilesRasterBody<TR_SLOTS_BATCH, TR_CHUNK_BATCH>(I.U, I.P, min(I.strandsToRender, I.S), cfg.tileSize, cfg.tileDepthBins,
+    tilesRasterBody(I.U, I.P, min(I.strandsToRender, I.S), cfg.tileSize, cfg.tileDepthBins,
                     cfg.invalidTilesPerSegmentThreshold, I.bsphere, I.posNew, I.tan, I.depth, I.tiles, I.segBuf,
                     I.segCount, ts.binCount, counters, sh, local, I.proj);
   }

@@ -4,7 +4,7 @@ tiles' decisions have their edges, against the CPU oracle."""
 import numpy as np
 import pytest
 
-from helpers import small_instance
+from helpers import frame_of, small_instance
 
 pytestmark = pytest.mark.gpu
 
@@ -12,7 +12,7 @@ torch = pytest.importorskip("torch")
 if not torch.cuda.is_available():
     pytest.skip("needs a CUDA GPU", allow_module_level=True)
 
-from test_gpu_parity import _fine_vs_oracle, oracle  # noqa: E402,F401
+from test_gpu_parity import _compare_tiles, _fine_vs_oracle, _raster_gpu, oracle  # noqa: E402,F401
 
 
 @pytest.mark.parametrize("tile,slices", [(8, 4), (8, 8), (16, 4), (16, 8), (32, 4), (32, 8)])
@@ -41,3 +41,17 @@ def test_fine_pass_split_tiles_near_a_full_pool(oracle, tile, avg):  # noqa: F81
     assert cnt["fineSplitTiles"] > 0, "no tile was split: the test does not test"
     err = np.abs(g - o)
     assert err.max() <= 1.0 / 255.0, f"max pixel error {err.max():.4g} (> 1/255)"
+
+
+@pytest.mark.parametrize("tile", [8, 16, 32])
+@pytest.mark.parametrize("points,fiber,size", [(2, 5e-4, (640, 480)), (9, 2e-2, (301, 217)), (16, 2e-5, (640, 480)),
+                                               (16, 5e-4, (2900, 1700))])
+def test_tiles_pass_segments_of_every_size_bit_exact(oracle, tile, points, fiber, size):  # noqa: F811
+    """Segments of tens of tiles each (a warp's accumulators hold a few of its
+    segments at a time), of one tile, thick and thinner than a pixel; a number
+    of segments that ends inside a warp."""
+    inst = small_instance(strands=333, points=points, width=size[0], height=size[1], tile_size=tile,
+                          fiber_radius=fiber, avg_segments_per_tile=2048)
+    fr = frame_of(inst)
+    ctx, hair, rb, d = _raster_gpu(inst, fr)
+    _compare_tiles(oracle, inst, fr, rb)
