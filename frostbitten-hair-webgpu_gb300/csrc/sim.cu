@@ -42,7 +42,12 @@ __device__ __forceinline__ float divBy3(float x) {
   const float a = fabsf(x);
   return a > 0x1p-123f && a < INFINITY ? mulRcp(x, RCP_3_HI, RCP_3_LO) : x / 3.0f;
 }
-__device__ __forceinline__ f3 div3sBy3(f3 v) { return {divBy3(v.x), divBy3(v.y), divBy3(v.z)}; }
+__device__ __forceinline__ f3 div3sBy3(f3 v) {
+  const float lo = fminf(fminf(fabsf(v.x), fabsf(v.y)), fabsf(v.z)), hi = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fabsf(v.z));
+  if (lo > 0x1p-123f && hi < INFINITY)  // one test for the three
+    return {mulRcp(v.x, RCP_3_HI, RCP_3_LO), mulRcp(v.y, RCP_3_HI, RCP_3_LO), mulRcp(v.z, RCP_3_HI, RCP_3_LO)};
+  return {divBy3(v.x), divBy3(v.y), divBy3(v.z)};
+}
 
 __device__ __forceinline__ uint32_t gridIdx(uint32_t G, uint32_t x, uint32_t y, uint32_t z) {
   return clampu(z, 0u, G - 1u) * G * G + clampu(y, 0u, G - 1u) * G + clampu(x, 0u, G - 1u);
@@ -164,21 +169,26 @@ __global__ void __launch_bounds__(256) gridPreSimKernel(const HfbSimUniforms u, 
 // forces, global shape, sphere and SDF collisions) and the coalesced loads
 // and stores.  The padding makes both access patterns conflict-free.
 //
-// The chains are latency-bound (each step waits on the last: an IEEE square
-// root and division per step), so what sets the pass's speed is how many
-// chains an SM walks at once, and shared memory is what bounds that.  Only
-// the points live there (16 B each): the triangle-bending constants and
-// initial tangents the local chain reads are written, in the Verlet phase,
-// over the block's own points of the PREV buffer -- each thread reads its
-// point's previous position first, and nothing else reads those addresses
-// until the final positions overwrite them -- and the segment lengths are
-// read from their buffer, four at a time where a strand's row is 16-byte
-// aligned; the chains load both ahead of the steps that use them.  A block of
-// 128 threads holds 2,048 points (64 strands of 32, 128 of 16), six blocks
-// per SM: 384 strands of 32 points in flight per SM, three chain warps per
-// scheduler.
+// The chains are latency-bound (each step waits on the last through a root and a
+// quotient: overRoot), so what sets their speed is how many an SM walks at once,
+// which shared memory bounds, and what a step waits for besides: the staged points
+// (16 B each) are all that lives there, and where the weights are the usual ones
+// (`plain`, below) a step reads nothing else but the segment lengths, four at a time
+// where a strand's row is 16-byte aligned, a group ahead.  With other weights the
+// bending constants go over the block's own points of the PREV buffer (each thread
+// has read its point's previous position by then, and nothing else reads those
+// addresses until the final positions overwrite them) and the chain loads them two
+// steps ahead.  Against constants in PREV for every block, whose loads came from L2
+// and held each bending step for about 340 cycles: 3.15 -> 2.71 ms (64 instances);
+// with 256 threads, for the point phases, in the single-instance kernel: 309 -> 222 us
+// (40,000 x 16, three passes), 175 -> 137 us (1,501 x 65); 512 threads 250 and 141 us.
+// Per block of the 64-instance frame (clock counters, before): Verlet 32 %, length
+// chain 10 %, global shape 10 %, bending chain 19 %, collisions 29 %.
+//
+// A block of 128 threads of the batched kernel holds 2,048 points (64 strands of 32,
+// 128 of 16), six blocks per SM: 384 strands of 32 points in flight per SM.
 // ---------------------------------------------------------------------------
-constexpr uint32_t SIM_THREADS = 128;        // threads per block of the single-instance kernel
+constexpr uint32_t SIM_THREADS = 256;        // threads per block of the single-instance kernel
 constexpr uint32_t SIM_BATCH_THREADS = 128;  // and of the batched one (6 blocks per SM)
 
 
@@ -198,19 +208,37 @@ __device__ __forceinline__ float4 verletPoint(const HfbSimUniforms& u, uint32_t 
   GridCo co = gridCell(G, gmin, gmax, pn);
   f3 grad = mk3(0.f, 0.f, 0.f), vel = mk3(0.f, 0.f, 0.f);
   float windStr = 0.0f, dens = 0.0f;
-  for (uint32_t z = co.mn[2]; z <= co.mx[2]; z++)
-    for (uint32_t y = co.mn[1]; y <= co.mx[1]; y++)
-      for (uint32_t x = co.mn[0]; x <= co.mx[0]; x++) {
-        f3 w = cellWeights(x, y, z, co.p);
-        float wl = len3(w);
-        uint32_t idx = gridIdx(G, x, y, z);
-        float4 a = __ldg(HFB_G(&gw[idx]));
-        grad = add3(grad, mul3(w, mk3(a.x, a.y, a.z)));
-        windStr = fadd(windStr, fmul(wl, a.w));
-        int4 b = __ldg(HFB_G(&dv[idx]));
-        vel = add3(vel, mul3(w, mk3(gridDecode(b.x), gridDecode(b.y), gridDecode(b.z))));
-        dens = fadd(dens, fmul(wl, gridDecode(b.w)));
-      }
+  // one corner: node idx, its weights per axis and their length
+  auto corner = [&](uint32_t idx, f3 w, float wl) {
+    const float4 a = __ldg(HFB_G(&gw[idx]));
+    const int4 b = __ldg(HFB_G(&dv[idx]));
+    grad = add3(grad, mul3(w, mk3(a.x, a.y, a.z)));
+    windStr = fadd(windStr, fmul(wl, a.w));
+    vel = add3(vel, mul3(w, mk3(gridDecode(b.x), gridDecode(b.y), gridDecode(b.z))));
+    dens = fadd(dens, fmul(wl, gridDecode(b.w)));
+  };
+  if (co.mx[0] > co.mn[0] && co.mx[1] > co.mn[1] && co.mx[2] > co.mn[2]) {
+    // inside a cell (no coordinate a whole number): eight corners, whose weights per axis
+    // are two numbers in (0, 1) (cellWeights without its clamps) and whose squares are
+    // summed once per pair of axes
+    const f3 w0 = {fsub(1.0f, fabsf(fsub(co.p.x, (float)co.mn[0]))), fsub(1.0f, fabsf(fsub(co.p.y, (float)co.mn[1]))),
+                   fsub(1.0f, fabsf(fsub(co.p.z, (float)co.mn[2])))};
+    const f3 w1 = {fsub(1.0f, fabsf(fsub(co.p.x, (float)co.mx[0]))), fsub(1.0f, fabsf(fsub(co.p.y, (float)co.mx[1]))),
+                   fsub(1.0f, fabsf(fsub(co.p.z, (float)co.mx[2])))};
+    const uint32_t i0 = (co.mn[2] * G + co.mn[1]) * G + co.mn[0];
+#pragma unroll
+    for (uint32_t k = 0; k < 8u; k++) {
+      const f3 w = {(k & 1u) ? w1.x : w0.x, (k & 2u) ? w1.y : w0.y, (k & 4u) ? w1.z : w0.z};
+      corner(i0 + (k & 1u) + ((k & 2u) ? G : 0u) + ((k & 4u) ? G * G : 0u), w, len3(w));
+    }
+  } else {
+    for (uint32_t z = co.mn[2]; z <= co.mx[2]; z++)
+      for (uint32_t y = co.mn[1]; y <= co.mx[1]; y++)
+        for (uint32_t x = co.mn[0]; x <= co.mx[0]; x++) {
+          const f3 w = cellWeights(x, y, z, co.p);
+          corner(gridIdx(G, x, y, z), w, len3(w));
+        }
+  }
   float timer = fadd(fmul((float)u.frameIdx, 0.73f), fmul(u.windPhaseOffset, (float)strand));
   float windJitter = fractf(fmul(timer, u.windStrengthFrequency));
   float jitterDelta = mixf(fmul(-0.5f, u.windStrengthJitter), fmul(0.5f, u.windStrengthJitter), windJitter);
@@ -263,15 +291,37 @@ __device__ __forceinline__ void sdfPush(float4& pos, const f3 q, float d, const 
   }
 }
 
+// x / sqrt(d) for a chain step: root and quotient from one reciprocal square root
+// (rootRecip), whose dependent chain is two thirds of an IEEE root and division's.
+__device__ __forceinline__ float overRoot(float x, float d) {
+  Recip l;
+  const bool ok = rootRecip(d, l);
+  const float q = divBy(x, l);
+  if (ok && x >= DIV_TINY && x <= 0x1p25f) return q;
+  return x / sqrtf(d);
+}
+
+// lengthStep between two movable points of weight 1: the products by the weights are
+// the numbers themselves, and .w, which carries something else, stays as it is.
+__device__ __forceinline__ void lengthStepMovable(float4* w, uint32_t j, float4& a, float expected, float kLen) {
+  float4 b = w[j + 1u];
+  const f3 tng = mk3(fsub(b.x, a.x), fsub(b.y, a.y), fsub(b.z, a.z));
+  const float df = fmul(fmul(fsub(1.0f, overRoot(expected, dot3(tng, tng))), kLen), 0.5f);
+  const f3 delta = mul3s(tng, df);
+  a.x = fadd(a.x, delta.x); a.y = fadd(a.y, delta.y); a.z = fadd(a.z, delta.z);
+  b.x = fsub(b.x, delta.x); b.y = fsub(b.y, delta.y); b.z = fsub(b.z, delta.z);
+  w[j] = a;
+  a = b;
+}
+
 // One step of the length chain (applyConstraint_length, constraints.wgsl.ts:5-28):
 // segment j between a (point j, carried in registers) and point j + 1 of the
 // staged strand w; writes point j and carries point j + 1 on in a.
-__device__ __forceinline__ void lengthStep(float4* w, uint32_t j, float4& a, float expected, float kLen) {
+__device__ __forceinline__ void lengthStep(float4* w, uint32_t j, float4& a, float w0, float w1, float expected,
+                                           float kLen) {
   float4 b = w[j + 1u];
-  const float w0 = a.w, w1 = b.w;
   f3 tng = mk3(fsub(b.x, a.x), fsub(b.y, a.y), fsub(b.z, a.z));
-  float actual = len3(tng);
-  float corr = fsub(1.0f, expected / actual);
+  float corr = fsub(1.0f, overRoot(expected, dot3(tng, tng)));
   // two movable points (the common case) make the divisor exactly 2: a halving, exact as a product
   const float num = fmul(corr, kLen), den = fadd(fadd(w0, w1), FLOAT_EPSILON);
   float df = den == 2.0f ? fmul(num, 0.5f) : num / den;
@@ -280,6 +330,24 @@ __device__ __forceinline__ void lengthStep(float4* w, uint32_t j, float4& a, flo
   b.x = fsub(b.x, fmul(w1, delta.x)); b.y = fsub(b.y, fmul(w1, delta.y)); b.z = fsub(b.z, fmul(w1, delta.z));
   w[j] = a;
   a = b;
+}
+
+// h0 of applyConstraint_localShape: the rest distance of a triplet's middle point from its centroid
+__device__ __forceinline__ float restHeight(float4 i0, float4 i1, float4 i2) {
+  const f3 c = div3sBy3(add3(add3(mk3(i0.x, i0.y, i0.z), mk3(i1.x, i1.y, i1.z)), mk3(i2.x, i2.y, i2.z)));
+  return len3(sub3(c, mk3(i1.x, i1.y, i1.z)));
+}
+
+// One triplet of the bending chain: p0, p1, p2 move along the middle point's offset from
+// the centroid by k0, k1, k2 times it (rest distance h0).
+__device__ __forceinline__ void bendStep(float4& p0, float4& p1, float4& p2, float h0, float k0, float k1, float k2) {
+  const f3 c = div3sBy3(add3(add3(mk3(p0.x, p0.y, p0.z), mk3(p1.x, p1.y, p1.z)), mk3(p2.x, p2.y, p2.z)));
+  const f3 hv = sub3(mk3(p1.x, p1.y, p1.z), c);
+  const f3 delta = mul3s(hv, fsub(1.0f, overRoot(h0, dot3(hv, hv))));
+  const f3 d0 = mul3s(delta, k0), d1 = mul3s(delta, k1), d2 = mul3s(delta, k2);
+  p0.x = fadd(p0.x, d0.x); p0.y = fadd(p0.y, d0.y); p0.z = fadd(p0.z, d0.z);
+  p1.x = fadd(p1.x, d1.x); p1.y = fadd(p1.y, d1.y); p1.z = fadd(p1.z, d1.z);
+  p2.x = fadd(p2.x, d2.x); p2.y = fadd(p2.y, d2.y); p2.z = fadd(p2.z, d2.z);
 }
 
 template <uint32_t NT>
@@ -304,26 +372,22 @@ __device__ __forceinline__ void simIntegrateBody(const HfbSimUniforms& u, uint32
   float4* const lcg = prev + (size_t)s0 * P;
 
   // --- Verlet + forces and the chain constants, point-parallel ---
+  // Where every strand of the block has a fixed root (weight 0) and movable points of
+  // weight 1 (`plain`: what assets have), the weights need no storage: .w of a staged point
+  // carries the only bending constant that differs from triplet to triplet, h0.
+  bool plain = true;
 #pragma unroll 2
   for (uint32_t i = tid; i < nPts; i += NT) {
     const uint32_t ls = i / P, pt = i - ls * P;
     const size_t gi = (size_t)s0 * P + i;
     const f4 posNow = ld4(__ldg(HFB_G(&now[gi])));
-    wk[ls * R + pt] = pt == 0u ? make_float4(posNow.x, posNow.y, posNow.z, posNow.w)
-                               : verletPoint(u, G, gmin, gmax, s0 + ls, posNow, ld4(*HFB_G(&prev[gi])), dv, gw);
+    float4 p = pt == 0u ? make_float4(posNow.x, posNow.y, posNow.z, posNow.w)
+                        : verletPoint(u, G, gmin, gmax, s0 + ls, posNow, ld4(*HFB_G(&prev[gi])), dv, gw);
     const float4 i0 = __ldg(HFB_G(&initial[gi]));
-    float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (pt + 3u < P) {  // applyConstraint_localShape constants (constraints.wgsl.ts:54-99)
-      const float4 i1 = __ldg(HFB_G(&initial[gi + 1u])), i2 = __ldg(HFB_G(&initial[gi + 2u]));
-      f3 cI = div3sBy3(add3(add3(mk3(i0.x, i0.y, i0.z), mk3(i1.x, i1.y, i1.z)), mk3(i2.x, i2.y, i2.z)));
-      const float h0 = len3(sub3(cI, mk3(i1.x, i1.y, i1.z)));
-      const float wT = fadd(fadd(i0.w, fmul(2.0f, i1.w)), i2.w);
-      c = make_float4(h0, fmul(i0.w / wT, 2.0f), fmul(i1.w / wT, -4.0f), fmul(i2.w / wT, 2.0f));
-    } else if (pt >= jTan && pt >= 1u) {  // applyConstraint_matchInitialTangent (:100-120)
-      const float4 im = __ldg(HFB_G(&initial[gi - 1u]));
-      c = make_float4(fsub(i0.x, im.x), fsub(i0.y, im.y), fsub(i0.z, im.z), 0.0f);
-    }
-    *HFB_G(&prev[gi]) = c;  // over the previous position this thread has just read
+    const float weight = pt == 0u ? 0.0f : 1.0f;
+    plain = plain && posNow.w == weight && i0.w == weight;
+    if (pt + 3u < P) p.w = restHeight(i0, __ldg(HFB_G(&initial[gi + 1u])), __ldg(HFB_G(&initial[gi + 2u])));
+    wk[ls * R + pt] = p;
   }
   for (uint32_t j = tid; j < P; j += NT) {  // applyConstraint_global's attenuation (constraints.wgsl.ts:31-49)
     const float x = (float)j / (float)(P - 1u);
@@ -332,7 +396,26 @@ __device__ __forceinline__ void simIntegrateBody(const HfbSimUniforms& u, uint32
   // i / P for the block's points (i < NB * P <= 2048, P <= 256): floor(i * ceil(2^32 / P) / 2^32)
   // is exact there, the error i * (ceil(2^32 / P) * P - 2^32) < 2048 * 256 being far below 2^32
   const uint32_t divP = (uint32_t)((0x100000000ull + P - 1u) / P);
-  __syncthreads();  // also makes the constants in PREV visible to the block's chain threads
+  plain = __syncthreads_and(plain) != 0;
+  if (!plain) {  // other weights: .w is the point's, and the chain constants go over the block's points of PREV
+    for (uint32_t i = tid; i < nPts; i += NT) {
+      const uint32_t ls = i / P, pt = i - ls * P;
+      const size_t gi = (size_t)s0 * P + i;
+      wk[ls * R + pt].w = __ldg(HFB_G(&now[gi])).w;
+      const float4 i0 = __ldg(HFB_G(&initial[gi]));
+      float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (pt + 3u < P) {  // applyConstraint_localShape constants (constraints.wgsl.ts:54-99)
+        const float4 i1 = __ldg(HFB_G(&initial[gi + 1u])), i2 = __ldg(HFB_G(&initial[gi + 2u]));
+        const float wT = fadd(fadd(i0.w, fmul(2.0f, i1.w)), i2.w);
+        c = make_float4(restHeight(i0, i1, i2), fmul(i0.w / wT, 2.0f), fmul(i1.w / wT, -4.0f), fmul(i2.w / wT, 2.0f));
+      } else if (pt >= jTan && pt >= 1u) {  // applyConstraint_matchInitialTangent (:100-120)
+        const float4 im = __ldg(HFB_G(&initial[gi - 1u]));
+        c = make_float4(fsub(i0.x, im.x), fsub(i0.y, im.y), fsub(i0.z, im.z), 0.0f);
+      }
+      *HFB_G(&prev[gi]) = c;
+    }
+    __syncthreads();  // also makes the constants in PREV visible to the block's chain threads
+  }
 
   const uint32_t iters = u.constraintIterations;
   const f3 smin = mk3(u.sdf.boundsMin.x, u.sdf.boundsMin.y, u.sdf.boundsMin.z);
@@ -362,17 +445,25 @@ __device__ __forceinline__ void simIntegrateBody(const HfbSimUniforms& u, uint32
         for (uint32_t g = 0; g < NG; g++) {
           const float4 nxt = g + 1u < NG ? __ldg(HFB_G(&L4[g + 1u])) : cur;
           const uint32_t j = g << 2;
-          lengthStep(w, j, a, cur.x, kLen);
-          lengthStep(w, j + 1u, a, cur.y, kLen);
-          lengthStep(w, j + 2u, a, cur.z, kLen);
-          if (g + 1u < NG) lengthStep(w, j + 3u, a, cur.w, kLen);  // step P - 1 does not exist
+          if (plain) {
+            if (g) lengthStepMovable(w, j, a, cur.x, kLen); else lengthStep(w, 0u, a, 0.0f, 1.0f, cur.x, kLen);
+            lengthStepMovable(w, j + 1u, a, cur.y, kLen);
+            lengthStepMovable(w, j + 2u, a, cur.z, kLen);
+            if (g + 1u < NG) lengthStepMovable(w, j + 3u, a, cur.w, kLen);  // step P - 1 does not exist
+          } else {
+            const uint32_t je = g + 1u < NG ? 4u : 3u;
+#pragma unroll 1
+            for (uint32_t e = 0; e < je; e++)
+              lengthStep(w, j + e, a, a.w, w[j + e + 1u].w, e == 0u ? cur.x : e == 1u ? cur.y : e == 2u ? cur.z : cur.w, kLen);
+          }
           cur = nxt;
         }
       } else {
         float expected = __ldg(HFB_G(&L[0])), nextExpected = __ldg(HFB_G(&L[1]));  // P >= 2
         for (uint32_t j = 0; j + 1u < P; j++) {
           const float nextExpected2 = j + 2u < P ? __ldg(HFB_G(&L[j + 2u])) : 0.0f;  // two steps ahead
-          lengthStep(w, j, a, expected, kLen);
+          const float wa = plain ? (j ? 1.0f : 0.0f) : a.w, wb = plain ? 1.0f : w[j + 1u].w;
+          lengthStep(w, j, a, wa, wb, expected, kLen);
           expected = nextExpected;
           nextExpected = nextExpected2;
         }
@@ -389,7 +480,8 @@ __device__ __forceinline__ void simIntegrateBody(const HfbSimUniforms& u, uint32
       const float k = fmul(kGlob, att[j]);
       float4 p = wk[ls * R + j];
       f3 dvv = mk3(fsub(pi.x, p.x), fsub(pi.y, p.y), fsub(pi.z, p.z));
-      f3 d = mul3s(mul3s(dvv, p.w), k);
+      if (!plain) dvv = mul3s(dvv, p.w);
+      f3 d = mul3s(dvv, k);
       p.x = fadd(p.x, d.x); p.y = fadd(p.y, d.y); p.z = fadd(p.z, d.z);
       wk[ls * R + j] = p;
     }
@@ -397,6 +489,40 @@ __device__ __forceinline__ void simIntegrateBody(const HfbSimUniforms& u, uint32
     // local shape (triangle bending, Gauss-Seidel), :209-232, constraints.wgsl.ts:54-120
     for (uint32_t ls = tid; ls < nStr; ls += NT) {
       float4* w = wk + ls * R;
+      if (plain) {
+        // the last three points' rest positions, for their tangents: loaded before the chain that
+        // precedes them (4 <= P: checked by the entry points)
+        const float4* E = initial + (size_t)(s0 + ls + 1u) * P - 4u;
+        const float4 e0 = __ldg(HFB_G(&E[0])), e1 = __ldg(HFB_G(&E[1])), e2 = __ldg(HFB_G(&E[2])),
+                     e3 = __ldg(HFB_G(&E[3]));
+        float4 p0 = w[0], p1 = w[1], p2 = w[2];
+        // the weights 0, 1, 1 of the triplet at the root; 1, 1, 1 of the others
+        bendStep(p0, p1, p2, p0.w, fmul(kLoc, fmul(0.0f / 3.0f, 2.0f)), fmul(kLoc, fmul(1.0f / 3.0f, -4.0f)),
+                 fmul(kLoc, fmul(1.0f / 3.0f, 2.0f)));
+        w[0] = p0;
+        float4 m = p0;  // the point before p1
+        p0 = p1;
+        p1 = p2;
+        const float kEnd = fmul(kLoc, 0.5f), kMid = fmul(kLoc, -1.0f);
+        for (uint32_t jj = 1; jj + 3u < P; jj++) {
+          p2 = w[jj + 2u];
+          bendStep(p0, p1, p2, p0.w, kEnd, kMid, kEnd);
+          w[jj] = m = p0;
+          p0 = p1;
+          p1 = p2;
+        }
+        // matchInitialTangent of the points P - 3 (p0), P - 2 (p1) and P - 1, each from the one before
+        auto tangentStep = [&](float4 p, const float4& ia, const float4& ib, uint32_t j) {
+          const f3 proj = add3(mk3(m.x, m.y, m.z), mk3(fsub(ib.x, ia.x), fsub(ib.y, ia.y), fsub(ib.z, ia.z)));
+          const f3 d = mul3s(sub3(proj, mk3(p.x, p.y, p.z)), kLoc);
+          p.x = fadd(p.x, d.x); p.y = fadd(p.y, d.y); p.z = fadd(p.z, d.z);
+          w[j] = m = p;
+        };
+        tangentStep(p0, e0, e1, P - 3u);
+        tangentStep(p1, e1, e2, P - 2u);
+        tangentStep(w[P - 1u], e2, e3, P - 1u);
+        continue;
+      }
       const float4* C = lcg + (size_t)ls * P;
       uint32_t jj = 0;
       if (P >= 3u) {
@@ -406,15 +532,7 @@ __device__ __forceinline__ void simIntegrateBody(const HfbSimUniforms& u, uint32
         for (; jj + 3u < P; jj++) {
           const float4 ccNext2 = *HFB_G(&C[jj + 2u]);  // jj + 2 < P
           float4 p2 = w[jj + 2u];
-          f3 c = div3sBy3(add3(add3(mk3(p0.x, p0.y, p0.z), mk3(p1.x, p1.y, p1.z)), mk3(p2.x, p2.y, p2.z)));
-          f3 hv = sub3(mk3(p1.x, p1.y, p1.z), c);
-          float h = len3(hv);
-          f3 delta = mul3s(hv, fsub(1.0f, cc.x / h));
-          f3 d0 = mul3s(delta, fmul(kLoc, cc.y)), d1 = mul3s(delta, fmul(kLoc, cc.z)),
-             d2 = mul3s(delta, fmul(kLoc, cc.w));
-          p0.x = fadd(p0.x, d0.x); p0.y = fadd(p0.y, d0.y); p0.z = fadd(p0.z, d0.z);
-          p1.x = fadd(p1.x, d1.x); p1.y = fadd(p1.y, d1.y); p1.z = fadd(p1.z, d1.z);
-          p2.x = fadd(p2.x, d2.x); p2.y = fadd(p2.y, d2.y); p2.z = fadd(p2.z, d2.z);
+          bendStep(p0, p1, p2, cc.x, fmul(kLoc, cc.y), fmul(kLoc, cc.z), fmul(kLoc, cc.w));
           w[jj] = p0;
           p0 = p1;
           p1 = p2;
@@ -454,12 +572,14 @@ __device__ __forceinline__ void simIntegrateBody(const HfbSimUniforms& u, uint32
   // --- write back into the PREV buffer, coalesced (:268-272), over the chain constants ---
   for (uint32_t i = tid; i < nPts; i += NT) {
     const uint32_t ls = i / P, pt = i - ls * P;
-    *HFB_G(&prev[(size_t)s0 * P + i]) = wk[ls * R + pt];
+    float4 p = wk[ls * R + pt];
+    if (plain) p.w = pt == 0u ? 0.0f : 1.0f;
+    *HFB_G(&prev[(size_t)s0 * P + i]) = p;
   }
   // the staging is rewritten by the CTA's next strands only after batchNext's barrier
 }
 
-__global__ void __launch_bounds__(SIM_THREADS, 6)
+__global__ void __launch_bounds__(SIM_THREADS, 3)
 simIntegrateKernel(const HfbSimUniforms u, uint32_t S, uint32_t P, uint32_t G,
                    float4* __restrict__ prev, const float4* __restrict__ now,
                    const float4* __restrict__ initial, const float* __restrict__ segLen,
