@@ -129,7 +129,8 @@ struct HdOut {
 };
 
 template <bool WIN>
-__device__ __forceinline__ void triPixel(const Tri& t, float area, const HdOut& o, int x, int y, uint32_t prim) {
+__device__ __forceinline__ void triPixel(const Tri& t, float area, float rcpArea, const HdOut& o, int x, int y,
+                                         uint32_t prim) {
   const float px = fadd((float)x, 0.5f), py = fadd((float)y, 0.5f);
   float w0 = edgeFn(t.v[1].x, t.v[1].y, t.v[2].x, t.v[2].y, px, py);
   float w1 = edgeFn(t.v[2].x, t.v[2].y, t.v[0].x, t.v[0].y, px, py);
@@ -137,7 +138,9 @@ __device__ __forceinline__ void triPixel(const Tri& t, float area, const HdOut& 
   if (area < 0.0f) { w0 = -w0; w1 = -w1; w2 = -w2; }
   if (!(w0 >= 0.0f && w1 >= 0.0f && w2 >= 0.0f)) return;
   const float a = fabsf(area);
-  const float z = fadd(fadd(fmul(w0, t.v[0].z), fmul(w1, t.v[1].z)), fmul(w2, t.v[2].z)) / a;
+  const float num = fadd(fadd(fmul(w0, t.v[0].z), fmul(w1, t.v[1].z)), fmul(w2, t.v[2].z));
+  float z = divBy(num, {a, rcpArea});  // the quotient's bits, but for tiny numerators and areas out of range
+  if (!(num >= DIV_TINY && z < 4.0f)) z = num / a;
   if (!(z >= 0.0f && z <= 1.0f)) return;
   const size_t p = (size_t)y * o.W + x;
   const unsigned zb = __float_as_uint(fadd(z, 0.0f));  // -0 -> +0
@@ -228,10 +231,11 @@ template <bool WIN>
 __device__ __forceinline__ void drawRows(const Tri& t, float area, const HdOut& o, int x0, int x1, int y0, int y1,
                                          int first, int step, uint32_t prim) {
   const bool safe = spanSafe(t), neg = area < 0.0f;
+  const float rcp = recipOf(fabsf(area)).y;
   for (int y = y0 + first; y <= y1; y += step) {
     int L = x0, R = x1;
     if (safe && !rowSpan(t, neg, y, L, R)) continue;
-    for (int x = L; x <= R; x++) triPixel<WIN>(t, area, o, x, y, prim);
+    for (int x = L; x <= R; x++) triPixel<WIN>(t, area, rcp, o, x, y, prim);
   }
 }
 
@@ -244,28 +248,40 @@ __device__ __forceinline__ Tri segTri(const ScreenV (&q)[4], uint32_t tr) {
   return t;
 }
 
-// A segment's two triangles for the warp's shared pixel loop: their pixel
-// boxes (an empty box for a triangle not drawn here), areas, and the union
-// of the boxes that the loop walks.
-struct HdUnit {
-  int bx0[2], bx1[2], by0[2], by1[2];
-  float area[2];
-  int x0, y0;
-  uint32_t bw, divBw;  // union box width and ceil(2^32 / width) (0 for width 1: 2^32 does not fit)
-};
+// The span lines of triangle t's rows; pixel centres lie at + 0.5.
+__device__ __forceinline__ SpanLines triSpans(const Tri& t, bool neg, int x0, int y0, int rows) {
+  // triPixel's edges a -> b accept (p - a) x (b - a) of one sign; spanLines' accept
+  // (p.x - o.x) d.y >= (p.y - o.y) d.x, so d is a - b, turned round with the winding
+  f2 o[3], d[3];
+#pragma unroll
+  for (int e = 0; e < 3; e++) {
+    const ScreenV& a = t.v[e == 0 ? 1 : e == 1 ? 2 : 0];
+    const ScreenV& b = t.v[e == 0 ? 2 : e == 1 ? 0 : 1];
+    o[e] = mk2(a.x - 0.5f, a.y - 0.5f);
+    d[e] = neg ? mk2(fsub(b.x, a.x), fsub(b.y, a.y)) : mk2(fsub(a.x, b.x), fsub(a.y, b.y));
+  }
+  return spanLines(o, d, (float)x0, (float)y0, (float)rows);
+}
 
+// What the warp's shared loops read: each point's two screen vertices, and of each
+// segment's two triangles their pixel boxes (empty for a triangle not drawn here), the
+// lines that bound their rows' spans (in pixels from the corner of the boxes' union),
+// areas and reciprocals.  One array per quantity, so that neighbouring lanes' entries lie
+// in neighbouring banks.
 struct HdShared {
-  float4 sv[HD_THREADS][2];            // each point's two screen vertices (x, y, z, drawable)
-  HdUnit unit[HD_THREADS];             // each thread's segment
-  uint32_t start[HD_THREADS / 32][32]; // per warp: first pixel of each lane's union box
+  float4 va[HD_THREADS], vb[HD_THREADS];           // x, y, z, drawable
+  float4 lo[2][HD_THREADS], hi[2][HD_THREADS];     // SpanLines
+  float2 area[2][HD_THREADS];                      // signed area; recipOf its magnitude
+  int4 box[2][HD_THREADS];                         // x0, y0, x1, y1
+  int2 corner[HD_THREADS];
 };
 
 // The quad of the segment whose first point has block index k.
 __device__ __forceinline__ void blockQuad(const HdShared& sh, uint32_t k, ScreenV (&q)[4]) {
-  q[0] = unpackV(sh.sv[k][0]);
-  q[1] = unpackV(sh.sv[k][1]);
-  q[2] = unpackV(sh.sv[k + 1][0]);
-  q[3] = unpackV(sh.sv[k + 1][1]);
+  q[0] = unpackV(sh.va[k]);
+  q[1] = unpackV(sh.vb[k]);
+  q[2] = unpackV(sh.va[k + 1]);
+  q[3] = unpackV(sh.vb[k + 1]);
 }
 
 // One block of segment starts [blk * HD_SEGS, (blk + 1) * HD_SEGS): each
@@ -274,12 +290,17 @@ __device__ __forceinline__ void blockQuad(const HdShared& sh, uint32_t k, Screen
 // next (when that point is not its strand's last): the warps need no
 // barrier between them.  A lane boxes its segment's two triangles.  A box
 // of more than HD_BIG_AREA pixels goes onto the big list (entries
-// point << 1 | triangle; capacity `bigCap`); the pixels of the union of a
-// segment's other boxes are shared out over the warp's lanes (an exclusive
-// scan of the union sizes), each pixel tested against both triangles
-// within their own boxes, so a lane with a long thin segment does not hold
-// up the other 31.  A big triangle that finds the list full is drawn by its
-// own thread.  Called by every thread of the block.
+// point << 1 | triangle; capacity `bigCap`); the rows of the other boxes are
+// shared out over the warp's lanes (warpOwner), each row narrowed to the two
+// triangles' spans (spanOf), and the spans' pixels are shared out the same way,
+// one triangle's exact test per lane, so a lane with a long thin segment does
+// not hold up the other 31.  A big triangle that finds the list full is drawn
+// by its own thread.  Called by every thread of the block.
+// Bound by issue (DRAM at 1.5 %): a thin segment covers a tenth of its boxes.
+// Against testing every pixel of the boxes' union for both triangles: 53 -> 30 us
+// (10,000 x 32 at 1920x1080), 1.79 -> 0.91 ms (200,000 x 32 at 4K), 1.51 -> 1.04 ms
+// (64 instances); with a struct per segment (128 bytes, so every lane in the same
+// banks) 67 us, 1.49 and 2.28 ms.
 // prim: the primitive index of triangle tr of the segment from point pt,
 // (strand * (P - 1) + segment) * 2 + tr, the order the reference draws them.
 __device__ __forceinline__ uint32_t primOf(uint32_t pt, uint32_t P, uint32_t tr) {
@@ -298,79 +319,102 @@ __device__ __forceinline__ void hairDepthBlock(const HdView& V, uint32_t P, uint
   if (pt < nPts) {
     ScreenV a, b;
     pointPair(V, pos, tan, pt, a, b);
-    sh.sv[tid][0] = packV(a);
-    sh.sv[tid][1] = packV(b);
+    sh.va[tid] = packV(a);
+    sh.vb[tid] = packV(b);
   }
   __syncwarp();
   const uint32_t W = f2u(V.W), H = f2u(V.H);
-  uint32_t mine = 0;
+  uint32_t rows = 0;
   bool own[2] = {false, false};  // big, list full: drawn by this thread
   if (lane < HD_WARP_SEGS && pt + 1u < nPts && pt % P != P - 1u) {
     ScreenV q[4];
     blockQuad(sh, tid, q);
-    HdUnit un;
-    int ux0 = 0x7fffffff, uy0 = 0x7fffffff, ux1 = -1, uy1 = -1;
+    int ux0 = 0x7fffffff, uy0 = 0x7fffffff, uy1 = -1;
+    float areas[2];
+    bool drawn[2];
 #pragma unroll
     for (uint32_t tr = 0; tr < 2u; tr++) {
-      un.bx0[tr] = 1; un.bx1[tr] = 0; un.by0[tr] = 1; un.by1[tr] = 0;  // empty
-      un.area[tr] = 0.0f;
+      drawn[tr] = false;
+      int4 box = make_int4(1, 1, 0, 0);  // empty
       const Tri t = segTri(q, tr);
       float area;
       int x0, x1, y0, y1;
-      if (!triBox(t, W, H, area, x0, x1, y0, y1)) continue;
-      const uint32_t bw = (uint32_t)(x1 - x0 + 1), bh = (uint32_t)(y1 - y0 + 1);
-      if ((uint64_t)bw * bh > HD_BIG_AREA) {
-        const uint32_t slot = bigCap > 0u && pt < 0x80000000u ? atomicAdd(HFB_G(&big[0]), 1u) : bigCap;
-        if (slot < bigCap)
-          *HFB_G(&big[1u + slot]) = (pt << 1) | tr;
-        else
-          own[tr] = true;
-        continue;
+      if (triBox(t, W, H, area, x0, x1, y0, y1)) {
+        const uint32_t bw = (uint32_t)(x1 - x0 + 1), bh = (uint32_t)(y1 - y0 + 1);
+        if ((uint64_t)bw * bh > HD_BIG_AREA) {
+          const uint32_t slot = bigCap > 0u && pt < 0x80000000u ? atomicAdd(HFB_G(&big[0]), 1u) : bigCap;
+          if (slot < bigCap)
+            *HFB_G(&big[1u + slot]) = (pt << 1) | tr;
+          else
+            own[tr] = true;
+        } else {
+          drawn[tr] = true;
+          areas[tr] = area;
+          box = make_int4(x0, y0, x1, y1);
+          sh.area[tr][tid] = make_float2(area, recipOf(fabsf(area)).y);
+          ux0 = min(ux0, x0); uy0 = min(uy0, y0); uy1 = max(uy1, y1);
+        }
       }
-      un.bx0[tr] = x0; un.bx1[tr] = x1; un.by0[tr] = y0; un.by1[tr] = y1;
-      un.area[tr] = area;
-      ux0 = min(ux0, x0); ux1 = max(ux1, x1); uy0 = min(uy0, y0); uy1 = max(uy1, y1);
+      sh.box[tr][tid] = box;
     }
-    if (ux1 >= ux0) {  // the union of the boxes drawn here
-      un.x0 = ux0;
-      un.y0 = uy0;
-      un.bw = (uint32_t)(ux1 - ux0 + 1);
-      un.divBw = un.bw > 1u ? (uint32_t)((0x100000000ull + un.bw - 1u) / un.bw) : 0u;
-      mine = un.bw * (uint32_t)(uy1 - uy0 + 1);
-      sh.unit[tid] = un;
-    }
-  }
-  // exclusive scan of the lanes' union boxes
-  uint32_t incl = mine;
+    if (uy1 >= uy0) {  // something is drawn here
+      sh.corner[tid] = make_int2(ux0, uy0);
+      rows = (uint32_t)(uy1 - uy0 + 1);
 #pragma unroll
-  for (uint32_t d = 1; d < 32u; d <<= 1) {
-    const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += o;
+      for (uint32_t tr = 0; tr < 2u; tr++) {
+        if (!drawn[tr]) continue;
+        const SpanLines sl = triSpans(segTri(q, tr), areas[tr] < 0.0f, ux0, uy0, (int)rows);
+        sh.lo[tr][tid] = sl.lo;
+        sh.hi[tr][tid] = sl.hi;
+      }
+    }
   }
-  const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-  sh.start[wp][lane] = incl - mine;
+  const uint32_t rowIncl = warpInclusive(rows, lane);
+  const uint32_t nRows = __shfl_sync(0xffffffffu, rowIncl, 31);
   __syncwarp();
-  for (uint32_t k = lane; k < total; k += 32u) {
-    uint32_t lo = 0, hi = 31;  // the last lane whose pixels start at or before k owns pixel k
-    while (lo < hi) {
-      const uint32_t mid = (lo + hi + 1u) >> 1;
-      if (sh.start[wp][mid] <= k) lo = mid; else hi = mid - 1u;
-    }
-    const uint32_t o = wp * 32u + lo;
-    const HdUnit& un = sh.unit[o];
-    const uint32_t local = k - sh.start[wp][lo];
-    // the union of two boxes of at most HD_BIG_AREA pixels each is at most
-    // 2048 wide and holds fewer than 2^21 pixels, so local * (divBw * bw - 2^32)
-    // < 2^21 * 2^11 and the multiply-high quotient is exact
-    const uint32_t row = un.bw > 1u ? __umulhi(local, un.divBw) : local;
-    const int x = un.x0 + (int)(local - row * un.bw), y = un.y0 + (int)row;
-    ScreenV q[4];
-    blockQuad(sh, o, q);
-    const uint32_t opt = blk * HD_SEGS + wp * HD_WARP_SEGS + lo;
+  for (uint32_t r0 = 0; r0 < nRows; r0 += 32u) {
+    // one row of a segment per lane: both triangles' spans (xa, n pixels each)
+    const uint32_t ri = r0 + lane;
+    const uint32_t ro = warpOwner(rowIncl, ri) & 31u;
+    const uint32_t row = ri - __shfl_sync(0xffffffffu, rowIncl - rows, ro);
+    uint32_t n[2] = {0u, 0u};
+    int xa[2] = {0, 0};
+    if (ri < nRows) {
+      const uint32_t o = wp * 32u + ro;
+      const int2 corner = sh.corner[o];
+      const int y = corner.y + (int)row;
 #pragma unroll
-    for (uint32_t tr = 0; tr < 2u; tr++)
-      if (x >= un.bx0[tr] && x <= un.bx1[tr] && y >= un.by0[tr] && y <= un.by1[tr])
-        triPixel<WIN>(segTri(q, tr), un.area[tr], out, x, y, primOf(opt, P, tr));
+      for (uint32_t tr = 0; tr < 2u; tr++) {
+        const int4 box = sh.box[tr][o];
+        if (y < box.y || y > box.w) continue;
+        int xb = box.z - corner.x;
+        xa[tr] = box.x - corner.x;
+        spanOf(sh.lo[tr][o], sh.hi[tr][o], (float)row, xa[tr], xb);
+        n[tr] = xb >= xa[tr] ? (uint32_t)(xb - xa[tr] + 1) : 0u;
+      }
+    }
+    const uint32_t incl = warpInclusive(n[0] + n[1], lane);
+    const uint32_t nPix = __shfl_sync(0xffffffffu, incl, 31);
+    // offsets below 2048 (two boxes of at most HD_BIG_AREA pixels), so the halves hold them
+    const uint32_t tag = ro | (row << 5), spans = (uint32_t)xa[0] | ((uint32_t)xa[1] << 16);
+    const uint32_t ends = (incl - n[0] - n[1]) | (n[0] << 20);
+    for (uint32_t c0 = 0; c0 < nPix; c0 += 32u) {
+      const uint32_t c = c0 + lane;
+      const uint32_t src = warpOwner(incl, c) & 31u;
+      const uint32_t t = __shfl_sync(0xffffffffu, tag, src), sp = __shfl_sync(0xffffffffu, spans, src),
+                     en = __shfl_sync(0xffffffffu, ends, src);
+      if (c >= nPix) continue;
+      const uint32_t k = c - (en & 0xfffffu), n0 = en >> 20;
+      const uint32_t tr = k < n0 ? 0u : 1u;
+      const uint32_t o = t & 31u;
+      const int2 corner = sh.corner[wp * 32u + o];
+      const float2 area = sh.area[tr][wp * 32u + o];
+      const int x = corner.x + (int)(tr ? (sp >> 16) + k - n0 : (sp & 0xffffu) + k), y = corner.y + (int)(t >> 5);
+      ScreenV q[4];
+      blockQuad(sh, wp * 32u + o, q);
+      triPixel<WIN>(segTri(q, tr), area.x, area.y, out, x, y,
+                    primOf(blk * HD_SEGS + wp * HD_WARP_SEGS + o, P, tr));
+    }
   }
   if (own[0] || own[1]) {
     ScreenV q[4];
@@ -513,7 +557,6 @@ __device__ __forceinline__ void loadView(const HfbUniforms& U, HdView& V) {
 }
 
 // ---- batched: persistent over every instance ----
-// 5 blocks per SM (48 registers): 1.33 ms against 1.40 at 4 on the 64-instance frame
 __global__ void __launch_bounds__(HD_THREADS, 5) hairDepthBatch(BatchView b) {
   __shared__ HdShared sh;
   __shared__ HdView V;
@@ -538,10 +581,16 @@ __global__ void __launch_bounds__(HD_THREADS, 5) hairDepthBatch(BatchView b) {
 
 __global__ void __launch_bounds__(HD_THREADS) hairDepthBigBatch(BatchView b) {
   __shared__ HdView V;
+  __shared__ uint32_t count[BATCH_MAX];  // big triangles of each instance (most have none)
   const uint32_t n = b.hdr->n;
-  for (uint32_t i = 0; i < n; i++) {  // every block takes a share of each instance's list
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
     const BatchInst& I = b.insts[i];
-    if (!I.hairDepth) continue;
+    count[i] = I.hairDepth && I.hdCap ? min(*HFB_G(I.hdList), I.hdCap) : 0u;
+  }
+  __syncthreads();
+  for (uint32_t i = 0; i < n; i++) {  // every block takes a share of each instance's list
+    if (count[i] <= blockIdx.x) continue;
+    const BatchInst& I = b.insts[i];
     loadView(I.U, V);
     const HdOut out = {reinterpret_cast<unsigned*>(I.hairDepth), nullptr, I.W};
     hairDepthBigBody<false>(V, I.P, I.posNew, I.tan, out, I.hdList, I.hdCap, blockIdx.x, gridDim.x);

@@ -12,7 +12,8 @@ torch = pytest.importorskip("torch")
 if not torch.cuda.is_available():
     pytest.skip("needs a CUDA GPU", allow_module_level=True)
 
-from test_gpu_parity import _compare_tiles, _fine_vs_oracle, _raster_gpu, oracle  # noqa: E402,F401
+from hairfb.passes import HairObject, HwHairPass, RasterBuffers  # noqa: E402
+from test_gpu_parity import _compare_tiles, _ctx, _fine_vs_oracle, _raster_gpu, oracle  # noqa: E402,F401
 
 
 @pytest.mark.parametrize("tile,slices", [(8, 4), (8, 8), (16, 4), (16, 8), (32, 4), (32, 8)])
@@ -55,3 +56,25 @@ def test_tiles_pass_segments_of_every_size_bit_exact(oracle, tile, points, fiber
     fr = frame_of(inst)
     ctx, hair, rb, d = _raster_gpu(inst, fr)
     _compare_tiles(oracle, inst, fr, rb)
+
+
+@pytest.mark.parametrize("points,fiber,size", [(2, 5e-4, (640, 480)), (9, 2e-2, (301, 217)), (16, 2e-5, (640, 480)),
+                                               (16, 5e-4, (2900, 1700)), (16, 2e-3, (64, 1900))])
+def test_hair_depth_segments_of_every_size_bit_exact(oracle, points, fiber, size):  # noqa: F811
+    """Triangles of one pixel to thousands (drawn by whole blocks), thick and
+    thinner than a pixel; a number of points that ends inside a warp."""
+    inst = small_instance(strands=333, points=points, width=size[0], height=size[1], fiber_radius=fiber)
+    fr = frame_of(inst)
+    ctx = _ctx(inst)
+    hair = HairObject(inst.hair, inst.cfg.shading_points)
+    rb = RasterBuffers(ctx, inst.width, inst.height)
+    d = torch.as_tensor(inst.scene_depth).cuda()
+    out = torch.empty_like(d)
+    HwHairPass(ctx).cmd_draw_hair_depth(fr.uniforms, hair, d, out, rb)
+    ctx.sync()
+    hb = inst.hair
+    o = oracle.hair_depth(fr.uniforms, hb.hair_data, hb.asset.positions, hb.tangents, hb.asset.strands,
+                          inst.scene_depth)
+    g = out.cpu().numpy()
+    assert (g < inst.scene_depth).sum() > 20, "little hair in front: the test does not test"
+    assert np.array_equal(g.view(np.uint32), o.view(np.uint32))
