@@ -15,10 +15,13 @@
 namespace hfb {
 namespace {
 
-__constant__ uint8_t kBayer[64] = {0,  32, 8,  40, 2,  34, 10, 42, 48, 16, 56, 24, 50, 18, 58, 26,
-                                   12, 44, 4,  36, 14, 46, 6,  38, 60, 28, 52, 20, 62, 30, 54, 22,
-                                   3,  35, 11, 43, 1,  33, 9,  41, 51, 19, 59, 27, 49, 17, 57, 25,
-                                   15, 47, 7,  39, 13, 45, 5,  37, 63, 31, 55, 23, 61, 29, 53, 21};
+// dither.wgsl.ts:26-53, each entry over 63
+#define B8(a, b, c, d, e, f, g, h) a / 63.0f, b / 63.0f, c / 63.0f, d / 63.0f, e / 63.0f, f / 63.0f, g / 63.0f, h / 63.0f
+__constant__ float kBayer[64] = {B8(0, 32, 8, 40, 2, 34, 10, 42),  B8(48, 16, 56, 24, 50, 18, 58, 26),
+                                 B8(12, 44, 4, 36, 14, 46, 6, 38),  B8(60, 28, 52, 20, 62, 30, 54, 22),
+                                 B8(3, 35, 11, 43, 1, 33, 9, 41),   B8(51, 19, 59, 27, 49, 17, 57, 25),
+                                 B8(15, 47, 7, 39, 13, 45, 5, 37),  B8(63, 31, 55, 23, 61, 29, 53, 21)};
+#undef B8
 
 __device__ __forceinline__ float aces(float x) {  // doACES_Tonemapping, one channel
   const float num = fmul(x, fadd(fmul(2.51f, x), 0.03f));
@@ -26,70 +29,103 @@ __device__ __forceinline__ float aces(float x) {  // doACES_Tonemapping, one cha
   return sat(num / den);
 }
 
-__device__ __forceinline__ uint8_t unorm8(float c) {  // float -> unorm8, round to nearest
-  return (uint8_t)__float2uint_rn(fmul(sat(c), 255.0f));
+__device__ __forceinline__ uint32_t unorm8(float c) {  // float -> unorm8, round to nearest
+  return __float2uint_rn(fmul(sat(c), 255.0f));
 }
 
-// Pixel i (row-major, row 0 at the top) of one image.
-__device__ __forceinline__ void presentPixel(float gamma, float exposure, float ditherStr, uint32_t W, uint32_t H,
-                                             const float4* __restrict__ result, const float4* __restrict__ scene,
-                                             uchar4* __restrict__ out, uint32_t i) {
-  const uint32_t x = i % W, y = i / W;  // y: row from the top
-  const float4 src = __ldg(HFB_G(&result[(size_t)(H - 1u - y) * W + x]));
-  const float4 dst = scene ? __ldg(HFB_G(&scene[i])) : make_float4(0.f, 0.f, 0.f, 1.f);
-  // blend: src * src.a + dst * (1 - src.a)
-  const float ia = fsub(1.0f, src.w);
-  float c[3] = {fadd(fmul(src.x, src.w), fmul(dst.x, ia)), fadd(fmul(src.y, src.w), fmul(dst.y, ia)),
-                fadd(fmul(src.z, src.w), fmul(dst.z, ia))};
-  const float dither = fmul((float)kBayer[(y % 8u) * 8u + (x % 8u)] / 63.0f, ditherStr) / 256.0f;
-  uint8_t o[3];
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    float v = fadd(c[k], dither);
-    v = fmul(v, exposure);
-    v = aces(v);
-    v = powf(v, 1.0f / gamma);
-    o[k] = unorm8(v);
-  }
-  *HFB_G(&out[i]) = make_uchar4(o[0], o[1], o[2], 255);
+// Tone mapping, gamma and unorm8 of one channel (x: exposed), as the passes define them.
+static __device__ __noinline__ uint32_t toneExact(float x, float power) { return unorm8(powf(aces(x), power)); }
+
+// The same byte from approximate units.  The quotient, logarithm and exponential are good to
+// 2^-22 (the logarithm absolutely within (0.5, 2)), so for powers up to 1 the value times 255 is
+// off by less than 255 * 2^-22 * (0.7 p + 0.7 * 1.25 * 0.53 + 1 + 0.5 p) < 1.7e-4 (r |log2 r| <=
+// 0.53 for r in [0, 1]), and powf and its products by less than 1e-4: farther than 5e-4 from a
+// rounding boundary the byte is decided.  One channel in 1,000 is not, and takes the exact way.
+constexpr float TONE_MARGIN = 5e-4f;
+__device__ __forceinline__ uint32_t tone(float x, float power, bool fast) {
+  const float num = fmul(x, fadd(fmul(2.51f, x), 0.03f));
+  const float den = fadd(fmul(x, fadd(fmul(2.43f, x), 0.59f)), 0.14f);
+  float rcp, lg, r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rcp) : "f"(den));
+  const float v = sat(fmul(num, rcp));
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(lg) : "f"(v));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmul(lg, power)));
+  const float t = fmul(r, 255.0f);
+  const float m = fadd(t, 12582912.0f);  // t rounded to the nearest whole number, in m's low bits
+  // den within the approximate reciprocal's accuracy, v not tiny (a zero is exact either way)
+  const bool ok = fast && fabsf(den) >= 1e-30f && fabsf(den) <= 1e30f && (v >= 1e-30f || num == 0.0f) &&
+                  fabsf(fsub(t, fsub(m, 12582912.0f))) < 0.5f - TONE_MARGIN;
+  if (!ok) return toneExact(x, power);
+  return __float_as_uint(m) & 255u;
 }
 
-__global__ void __launch_bounds__(256)
-presentKernel(float gamma, float exposure, float ditherStr, uint32_t W, uint32_t H, const float4* __restrict__ result,
-              const float4* __restrict__ scene, uchar4* __restrict__ out) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= W * H) return;
-  presentPixel(gamma, exposure, ditherStr, W, H, result, scene, out, i);
-}
-
-// Up to PRESENT_BATCH images in one launch, passed by value (48 B each, inside
-// the 4 KB of kernel parameters every launch may carry): image k covers the
-// launch's pixels [first[k], first[k + 1]).
-constexpr uint32_t PRESENT_BATCH = 64;
+// One image of a launch; it takes the launch's blocks [first, first + blocks).
 struct PresentImage {
-  float gamma, exposure, dither;
+  float power, exposure, dither;  // power: 1 / gamma
   uint32_t W, H, first;
   const float4* result;
   const float4* scene;
   uchar4* out;
 };
+
+// Pixels [blk * PRESENT_PIXELS, (blk + 1) * PRESENT_PIXELS) of an image, row-major, row 0 at
+// the top.  20 B per pixel read (36 with a scene) and 4 written: with ~550 instructions per
+// pixel (powf, divisions, a search for the pixel's image) the pass ran at 1.8 TB/s on 64
+// images; with ~120 it is near the memory's rate.
+constexpr uint32_t PRESENT_THREADS = 256, PRESENT_PIXELS = 1024;
+__device__ __forceinline__ void presentBlock(const PresentImage m, uint32_t blk, float* bayer) {
+  if (threadIdx.x < 64u) bayer[threadIdx.x] = kBayer[threadIdx.x];  // lanes read different entries
+  __syncthreads();
+  const uint32_t n = m.W * m.H, W = m.W;
+  const float power = m.power, exposure = m.exposure, ditherStr = m.dither;
+  const bool fast = power > 0.0f && power <= 1.0f;
+  uint32_t i = blk * PRESENT_PIXELS + threadIdx.x;
+  uint32_t y = i / W, x = i - y * W;  // y: row from the top
+  const uint32_t dy = PRESENT_THREADS / W, dx = PRESENT_THREADS - dy * W;
+#pragma unroll
+  for (uint32_t k = 0; k < PRESENT_PIXELS / PRESENT_THREADS; k++) {
+    if (i < n) {
+      const float4 src = __ldg(HFB_G(&m.result[(size_t)(m.H - 1u - y) * W + x]));
+      const float4 dst = m.scene ? __ldg(HFB_G(&m.scene[i])) : make_float4(0.f, 0.f, 0.f, 1.f);
+      // blend: src * src.a + dst * (1 - src.a)
+      const float ia = fsub(1.0f, src.w);
+      const float dither = fmul(fmul(bayer[(y & 7u) * 8u + (x & 7u)], ditherStr), 1.0f / 256.0f);
+      const float r = fmul(fadd(fadd(fmul(src.x, src.w), fmul(dst.x, ia)), dither), exposure);
+      const float g = fmul(fadd(fadd(fmul(src.y, src.w), fmul(dst.y, ia)), dither), exposure);
+      const float b = fmul(fadd(fadd(fmul(src.z, src.w), fmul(dst.z, ia)), dither), exposure);
+      *HFB_G(&m.out[i]) = make_uchar4((unsigned char)tone(r, power, fast), (unsigned char)tone(g, power, fast),
+                                      (unsigned char)tone(b, power, fast), 255);
+    }
+    i += PRESENT_THREADS;
+    x += dx;
+    y += dy;
+    if (x >= W) { x -= W; y++; }
+  }
+}
+
+__global__ void __launch_bounds__(PRESENT_THREADS) presentKernel(const PresentImage m) {
+  __shared__ float bayer[64];
+  presentBlock(m, blockIdx.x, bayer);
+}
+
+// Up to PRESENT_BATCH images in one launch, passed by value (48 B each, inside
+// the 4 KB of kernel parameters every launch may carry).
+constexpr uint32_t PRESENT_BATCH = 64;
 struct PresentBatch {
-  uint32_t n, total;
+  uint32_t n, blocks;
   PresentImage im[PRESENT_BATCH];
 };
 static_assert(sizeof(PresentBatch) <= 4000, "kernel parameters above 4 KB");
 
-__global__ void __launch_bounds__(256) presentBatchKernel(const PresentBatch pb) {
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < pb.total; g += stride) {
-    uint32_t lo = 0, hi = pb.n - 1u;  // the last image whose first pixel is at or before g
-    while (lo < hi) {
-      const uint32_t mid = (lo + hi + 1u) >> 1;
-      if (pb.im[mid].first <= g) lo = mid; else hi = mid - 1u;
-    }
-    const PresentImage& m = pb.im[lo];
-    presentPixel(m.gamma, m.exposure, m.dither, m.W, m.H, m.result, m.scene, m.out, g - m.first);
+__global__ void __launch_bounds__(PRESENT_THREADS) presentBatchKernel(const PresentBatch pb) {
+  __shared__ float bayer[64];
+  uint32_t lo = 0, hi = pb.n - 1u;  // the last image whose first block is at or before this one
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi + 1u) >> 1;
+    if (pb.im[mid].first <= blockIdx.x) lo = mid; else hi = mid - 1u;
   }
+  const PresentImage m = pb.im[lo];
+  presentBlock(m, blockIdx.x - m.first, bayer);
 }
 
 }  // namespace
@@ -99,8 +135,9 @@ cudaError_t launchPresent(HfbCtx* c, const HfbUniforms& u, uint32_t W, uint32_t 
   HFB_CHECK_BIND(c);
   const uint32_t n = W * H;
   if (n == 0) return cudaSuccess;
-  presentKernel<<<divCeil(n, 256u), 256, 0, c->stream>>>(u.colorMgmt.x, u.colorMgmt.y, u.colorMgmt.z, W, H,
-                                                         (const float4*)result, (const float4*)scene, (uchar4*)rgba);
+  const PresentImage m = {1.0f / u.colorMgmt.x, u.colorMgmt.y, u.colorMgmt.z, W, H, 0u, (const float4*)result,
+                          (const float4*)scene, (uchar4*)rgba};
+  presentKernel<<<divCeil(n, PRESENT_PIXELS), PRESENT_THREADS, 0, c->stream>>>(m);
   HFB_AFTER_LAUNCH(c, "presentKernel");
   c->launches += 1;
   return cudaGetLastError();
@@ -118,23 +155,14 @@ cudaError_t launchPresentBatch(HfbCtx* c, const HfbPresentItem* items, uint32_t 
       const uint32_t W = it.rb->width, H = it.rb->height;
       if ((uint64_t)W * H == 0u) continue;
       if (total + (uint64_t)W * H > 0xffffffffull) return cudaErrorInvalidValue;
-      PresentImage& m = pb.im[pb.n++];
-      m.gamma = it.uniforms->colorMgmt.x;
-      m.exposure = it.uniforms->colorMgmt.y;
-      m.dither = it.uniforms->colorMgmt.z;
-      m.W = W;
-      m.H = H;
-      m.first = (uint32_t)total;
-      m.result = (const float4*)(it.rb->rasterizerResult + 4);
-      m.scene = (const float4*)it.sceneColor;
-      m.out = (uchar4*)it.rgba;
+      pb.im[pb.n++] = {1.0f / it.uniforms->colorMgmt.x, it.uniforms->colorMgmt.y, it.uniforms->colorMgmt.z, W, H,
+                       pb.blocks, (const float4*)(it.rb->rasterizerResult + 4), (const float4*)it.sceneColor,
+                       (uchar4*)it.rgba};
+      pb.blocks += divCeil(W * H, PRESENT_PIXELS);
       total += (uint64_t)W * H;
     }
     if (pb.n == 0) continue;
-    pb.total = (uint32_t)total;
-    const uint32_t blocks = divCeil(pb.total, 256u);
-    const uint32_t cap = c->smCount * 8u;
-    presentBatchKernel<<<blocks < cap ? blocks : cap, 256, 0, c->stream>>>(pb);
+    presentBatchKernel<<<pb.blocks, PRESENT_THREADS, 0, c->stream>>>(pb);
     HFB_AFTER_LAUNCH(c, "presentBatchKernel");
     c->launches += 1;
     cudaError_t e = cudaGetLastError();
