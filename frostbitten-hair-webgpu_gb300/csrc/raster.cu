@@ -976,25 +976,27 @@ tileSortKernel(uint32_t T, uint32_t NB, uint32_t bucketSize, const uint32_t* __r
 // segment that fills the pool keeps its first slots in pixel order, after
 // which the bin stops.
 // ---------------------------------------------------------------------------
-constexpr uint32_t NSHADE = 4;              // shading entries staged per segment
 constexpr uint32_t MAX_RUNS = 66;           // runs of one round: at most one per depth bin (+1)
 constexpr uint32_t EMPTY_BOX = 0x0000ffffu; // x0 = y0 = 255 > x1 = y1 = 0
 constexpr uint32_t RUN_ENDS = 1u << 31;
 constexpr uint32_t FINE_SPLIT_MIN = 256;  // records: tiles below this are never split
 
 template <int TS> struct FineDims;
-// PAIRS: listed pixels of a round (and, in a careful group, box pixels: fineTile); ROWS:
-// box rows (a few per thread); CTAS: CTAs per SM that fineScheduleBody shares a frame's
-// records out over, by slices (4, 8, 16) -- a constant, not the occupancy, so that where
-// a tile is split, and with it the last bits of its pixels, does not depend on the build
+// PAIRS: listed pixels of a round (and, in a careful part, box pixels: fineTile); ROWS:
+// box rows (a few per thread); NSHADE: shading entries staged per segment; CTAS: CTAs
+// per SM that fineScheduleBody shares a frame's records out over, by slices (4, 8, 16) --
+// a constant, not the occupancy, so that where a tile is split, and with it the last bits
+// of its pixels, does not depend on the build.  At 8 px the sizes leave room for 8 CTAs
+// of the batched kernel per SM (28,160 bytes each): 3.10 ms on the 64-instance frame
+// against 3.39 at 7.
 template <> struct FineDims<8> {
-  static constexpr uint32_t STAGE = 64, PAIRS = 768, ROWS = 512, CTAS[3] = {8, 6, 6};
+  static constexpr uint32_t STAGE = 64, PAIRS = 768, ROWS = 512, NSHADE = 3, CTAS[3] = {8, 6, 6};
 };
 template <> struct FineDims<16> {
-  static constexpr uint32_t STAGE = 128, PAIRS = 2048, ROWS = 2048, CTAS[3] = {3, 2, 2};  // 96: 2-3 % slower, 160: 4 % slower
+  static constexpr uint32_t STAGE = 128, PAIRS = 2048, ROWS = 2048, NSHADE = 4, CTAS[3] = {3, 2, 2};  // 96: 2-3 % slower, 160: 4 % slower
 };
 template <> struct FineDims<32> {
-  static constexpr uint32_t STAGE = 256, PAIRS = 4096, ROWS = 4096, CTAS[3] = {1, 1, 1};
+  static constexpr uint32_t STAGE = 256, PAIRS = 4096, ROWS = 4096, NSHADE = 4, CTAS[3] = {1, 1, 1};
 };
 
 // A box row's place in the round's list: the row's listed pixels (bit x), and
@@ -1032,8 +1034,10 @@ template <int TS>
 struct FineSmem {
   static constexpr uint32_t NT = TS * TS, STAGE = FineDims<TS>::STAGE, PAIRS = FineDims<TS>::PAIRS, ROWS = FineDims<TS>::ROWS;
   static_assert(PAIRS >= NT && ROWS >= TS, "any one segment fits in a round");
+  static_assert(STAGE <= NT, "a thread per staged segment");
   static_assert(PAIRS <= 65536 && ROWS % NT == 0, "FineRow's first index is 16 bits; rows per thread");
   static_assert(2 * 6 * STAGE * sizeof(float) <= PAIRS * sizeof(uint2), "stagePoint's scratch fits in frag");
+  static constexpr uint32_t NSHADE = FineDims<TS>::NSHADE;
   float4 shade[STAGE][NSHADE];   // the shading entries each staged segment can sample
   uint2 frag[PAIRS];             // A1: pixel | segment << 16 of a listed pixel; A2: its fragment's colour as 4 x f16
   float4 spanLo[STAGE], spanHi[STAGE];  // SpanLines in tile pixels
@@ -1046,21 +1050,32 @@ struct FineSmem {
   float qsx[STAGE], qsy[STAGE], qax[STAGE], qay[STAGE], qd2[STAGE], qlse[STAGE], qws[STAGE], qwe[STAGE],
       qd22[STAGE];                   // QuadConst
   float yd2[STAGE], ylse[STAGE], yd22[STAGE];  // QuadRecip
-  uint32_t enc[STAGE], listIdx[STAGE];  // strand | segment << 24, place in the list
+  uint32_t enc[STAGE];               // strand | segment << 24
   uint32_t box[STAGE];               // tile-local pixel box x0 | y0 << 8 | x1 << 16 | y1 << 24
   uint32_t shadeBase[STAGE];         // first staged shading index | count << 16 | depth bin << 24
   uint32_t rowBase[STAGE + 1];       // exclusive prefix of the box heights (A1's items)
   uint32_t rowOff[STAGE];            // rowBase minus the box's first row: tile row y is row[rowOff + y]
-  uint32_t cntEdge[STAGE], cntFrag[STAGE];
+  uint32_t cnt[STAGE];               // counted pixels (CAREFUL) or fragments (exact accounting) of each
   uint32_t pixMask[STAGE / 32][NT];  // bit k of pixel p: staged segment k left a fragment at p
   // the tile
   uint4 head[64];                    // HairTileResult per depth bin
-  float td0[64], td1[64];            // its depth range (_getTileDepth), for the slices of its fragments
+  float td0[64], td1[64], tdY[64];   // its depth range (_getTileDepth) and the range's reciprocal (recipOf)
   uint32_t binOff[65];               // tile mode: first entry of each bin in the tile's sequence
   float zbuf[NT];
   uint32_t doneMask[NT / 32];
   // the round
-  uint32_t runBin[MAX_RUNS], runK0[MAX_RUNS], runK1[MAX_RUNS], runOff[MAX_RUNS];
+  uint32_t runBin[MAX_RUNS], runOff[MAX_RUNS];
+  uint16_t runK0[MAX_RUNS], runK1[MAX_RUNS];
+  // tile mode: bit k set where a run with segments starts at staged segment k; the bin of the
+  // j-th such run, and its list index plus k
+  // (walk mode: each staged segment's place in the list)
+  union {
+    struct {
+      uint32_t runStart[STAGE / 32], startBase[64];
+      uint8_t startBin[64];
+    };
+    uint32_t listIdx[STAGE];
+  };
   uint32_t red[32];
   // the work item's instance (written by one thread per item): read where used, so that none of
   // it stays in registers across the tile's rounds
@@ -1109,7 +1124,7 @@ __device__ __forceinline__ uint32_t stageShade(FineSmem<TS>& sh, uint32_t k, uin
   uint32_t a0, a1, b0, b1;
   remapToIndices(SP, fadd((float)sg, 0.0f) / (float)(P - 1u), a0, a1);
   remapToIndices(SP, fadd((float)sg, 1.0f) / (float)(P - 1u), b0, b1);
-  const uint32_t ne = min(b1 - a0 + 1u, NSHADE);
+  const uint32_t ne = min(b1 - a0 + 1u, FineSmem<TS>::NSHADE);
   const size_t sb = (size_t)st * SP;
   for (uint32_t j = 0; j < ne; j++) sh.shade[k][j] = __ldg(HFB_G(&shading[sb + a0 + j]));
   return a0 | (ne << 16);
@@ -1159,8 +1174,7 @@ __device__ __forceinline__ uint32_t stageFromProjection(FineSmem<TS>& sh, uint32
   }
   sh.box[k] = box;
   sh.shadeBase[k] = shadeBase;
-  sh.cntEdge[k] = 0;
-  sh.cntFrag[k] = 0;
+  sh.cnt[k] = 0;
   return rows;
 }
 
@@ -1177,8 +1191,7 @@ __device__ __forceinline__ uint32_t stageSegment(FineSmem<TS>& sh, uint32_t k, u
   }
   sh.box[k] = EMPTY_BOX;
   sh.shadeBase[k] = bin << 24;
-  sh.cntEdge[k] = 0;
-  sh.cntFrag[k] = 0;
+  sh.cnt[k] = 0;
   return 0u;
 }
 
@@ -1186,8 +1199,9 @@ __device__ __forceinline__ uint32_t stageSegment(FineSmem<TS>& sh, uint32_t k, u
 template <int TS>
 __device__ __forceinline__ uint32_t stageCached(FineSmem<TS>& sh, uint32_t k, uint32_t bin,
                                                 const float4* __restrict__ proj, const float4* __restrict__ shading,
-                                                uint32_t S, uint32_t P, uint32_t SP, uint32_t x0, uint32_t y0) {
-  const uint32_t st = sh.enc[k] & 0x00ffffffu, sg = sh.enc[k] >> 24;
+                                                uint32_t enc, uint32_t S, uint32_t P, uint32_t SP, uint32_t x0,
+                                                uint32_t y0) {
+  const uint32_t st = enc & 0x00ffffffu, sg = enc >> 24;
   if (st < S && sg + 1u < P) {
     const float4* q = proj + ((size_t)st * (P - 1u) + sg) * SEG_PROJ_VEC4;
     const float4 a = __ldg(HFB_G(&q[0])), b = __ldg(HFB_G(&q[1])), d = __ldg(HFB_G(&q[2]));
@@ -1201,8 +1215,7 @@ __device__ __forceinline__ uint32_t stageCached(FineSmem<TS>& sh, uint32_t k, ui
   }
   sh.box[k] = EMPTY_BOX;
   sh.shadeBase[k] = bin << 24;
-  sh.cntEdge[k] = 0;
-  sh.cntFrag[k] = 0;
+  sh.cnt[k] = 0;
   return 0u;
 }
 
@@ -1242,8 +1255,7 @@ __device__ __forceinline__ uint32_t stageFromPoints(FineSmem<TS>& sh, uint32_t k
   if (!(st < S && sg + 1u < P)) {
     sh.box[k] = EMPTY_BOX;
     sh.shadeBase[k] = bin << 24;
-    sh.cntEdge[k] = 0;
-    sh.cntFrag[k] = 0;
+    sh.cnt[k] = 0;
     return 0u;
   }
   const float* p0 = reinterpret_cast<const float*>(sh.frag);
@@ -1262,13 +1274,14 @@ __device__ __forceinline__ uint32_t stageFromPoints(FineSmem<TS>& sh, uint32_t k
 // _sampleShading, hairShadingBuffer.ts:28-38), as 4 x f16, and its slice.
 template <int TS>
 __device__ __forceinline__ uint2 fragmentColour(const FineSmem<TS>& sh, uint32_t k, f2 w, float hd, uint32_t P,
-                                                uint32_t SP, uint32_t L, float td0, float td1,
+                                                uint32_t SP, uint32_t L, uint32_t bin,
                                                 uint32_t alphaQuadratic, float alphaMul,
                                                 const float4* __restrict__ shading, uint32_t& slice) {
   float alpha = fsub(1.0f, fabsf(fsub(fmul(w.x, 2.0f), 1.0f)));
   if (alphaQuadratic) alpha = sqrtf(alpha);
   alpha = sat(fmul(alpha, alphaMul));
-  const float tFull = fadd((float)(sh.enc[k] >> 24), w.y) / (float)(P - 1u);
+  // (segment + w.y) / (P - 1): w.y is 0 or at least 2^-75, so divBy's quotient is the division's
+  const float tFull = divBy(fadd((float)(sh.enc[k] >> 24), w.y), {(float)(P - 1u), 1.0f / (float)(P - 1u)});
   uint32_t i0, i1;
   const float fr = remapToIndices(SP, tFull, i0, i1);
   const uint32_t sbase = sh.shadeBase[k];
@@ -1284,7 +1297,11 @@ __device__ __forceinline__ uint2 fragmentColour(const FineSmem<TS>& sh, uint32_t
   }
   f4 c = mix4(ld4(c0), ld4(c1), fr);
   c.w = fmul(c.w, alpha);
-  slice = getDepthBin(L, td0, td1, hd);  // getSliceIdx
+  // getSliceIdx: getDepthBin(L, td0, td1, hd); a quotient too tiny for divBy is in slice 0 either way
+  const float td0 = sh.td0[bin], span = fabsf(fsub(sh.td1[bin], td0)), x = fsub(hd, td0);
+  float t = divBy(x, {span, sh.tdY[bin]});
+  if (!(fabsf(t) < 1e30f)) t = x / span;
+  slice = clampu(f2u(fmul(t, (float)L)), 0u, L - 1u);
   const uint32_t hx = __half_as_ushort(__float2half_rn(c.x)), hy = __half_as_ushort(__float2half_rn(c.y));
   const uint32_t hz = __half_as_ushort(__float2half_rn(c.z)), hw = __half_as_ushort(__float2half_rn(c.w));
   return make_uint2(hx | (hy << 16), hz | (hw << 16));
@@ -1313,31 +1330,49 @@ __device__ __forceinline__ void blendFragment(f4 (&acc)[MAXL], uint32_t sl, uint
 // Tile mode: the runs of the next round, from bin `bin`, entry `off` of its
 // list, up to `cap` segments.  Bins without depth (td1 == 0) are skipped as
 // the reference skips them; a depth bin with an empty list is a run of zero
-// segments (its reduce still runs).  Called by one thread.
+// segments (its reduce still runs).  A bin is in the round when fewer than
+// `cap` entries lie between the cursor and it (binOff), or exactly `cap` and it
+// is empty.  Called by one warp, a lane per bin; sets nRuns, returns the segments.
 template <int TS>
-__device__ __forceinline__ uint32_t buildRuns(FineSmem<TS>& sh, uint32_t B, uint32_t bin, uint32_t off,
-                                              uint32_t cap, uint32_t& used) {
-  uint32_t n = 0;
-  used = 0;
-  while (bin < B && n < MAX_RUNS) {
-    if (sh.head[bin].y == 0u) { bin++; off = 0; continue; }
-    const uint32_t rem = sh.binOff[bin + 1] - sh.binOff[bin] - off;
-    if (rem > 0u && used == cap) break;
-    const uint32_t take = min(rem, cap - used);
-    const bool ends = take == rem;
-    sh.runBin[n] = bin | (ends ? RUN_ENDS : 0u);
-    sh.runK0[n] = used;
-    sh.runK1[n] = used + take;
-    sh.runOff[n] = off;
-    n++;
-    used += take;
-    if (!ends) break;
-    bin++;
-    off = 0;
+__device__ __forceinline__ uint32_t buildRuns(FineSmem<TS>& sh, uint32_t b1, uint32_t bin, uint32_t off, uint32_t cap,
+                                              uint32_t lane) {
+  if (lane < FineSmem<TS>::STAGE / 32u) sh.runStart[lane] = 0;
+  __syncwarp();
+  uint32_t n = 0, nStart = 0, used = 0;
+  const uint32_t p0 = bin < b1 ? sh.binOff[bin] + off : 0u;
+  for (uint32_t c0 = bin & ~31u; c0 < b1; c0 += 32u) {
+    const uint32_t bb = c0 + lane;
+    uint32_t pre = 0, rem = 0, o = 0, hz = 0;
+    bool in = false;
+    if (bb >= bin && bb < b1 && sh.head[bb].y != 0u) {
+      o = bb == bin ? off : 0u;
+      hz = sh.head[bb].z;
+      pre = sh.binOff[bb] + o - p0;
+      rem = sh.binOff[bb + 1u] - sh.binOff[bb] - o;
+      in = pre < cap || (rem == 0u && pre == cap);
+    }
+    const uint32_t take = in ? min(rem, cap - pre) : 0u, lt = (1u << lane) - 1u;
+    const uint32_t m = __ballot_sync(0xffffffffu, in), ms = __ballot_sync(0xffffffffu, take != 0u);
+    if (in) {
+      const uint32_t r = n + (uint32_t)__popc(m & lt);
+      sh.runBin[r] = bb | (take == rem ? RUN_ENDS : 0u);
+      sh.runK0[r] = (uint16_t)pre;
+      sh.runK1[r] = (uint16_t)(pre + take);
+      sh.runOff[r] = o;
+    }
+    if (take) {
+      const uint32_t j = nStart + (uint32_t)__popc(ms & lt);
+      sh.startBin[j] = (uint8_t)bb;
+      sh.startBase[j] = hz - 1u - o + pre;
+      atomicOr(&sh.runStart[pre >> 5], 1u << (pre & 31u));
+    }
+    n += (uint32_t)__popc(m);
+    nStart += (uint32_t)__popc(ms);
+    used = max(used, __reduce_max_sync(0xffffffffu, in ? pre + take : 0u));
   }
-  return n;
+  if (lane == 0) sh.nRuns = n;
+  return used;
 }
-
 
 // Rasterizes depth bins [b0, b1) of tile tileIdx in order, every pixel
 // starting from an empty colour (processTile per bin + reduceHairSlices,
@@ -1386,8 +1421,10 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
   if (tid < a.B) {
     const uint4 h = (*HFB_G(&a.tiles[ty * tilesX * a.B + tx * a.B + tid]));
     sh.head[tid] = h;
-    sh.td0[tid] = (float)(0xffffffffu - h.x) / F_MAX_U32;  // _getTileDepth
-    sh.td1[tid] = (float)h.y / F_MAX_U32;
+    const float d0 = (float)(0xffffffffu - h.x) / F_MAX_U32, d1 = (float)h.y / F_MAX_U32;  // _getTileDepth
+    sh.td0[tid] = d0;
+    sh.td1[tid] = d1;
+    sh.tdY[tid] = recipOf(fabsf(fsub(d1, d0))).y;
   }
   __syncthreads();
 
@@ -1424,7 +1461,8 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
   }
   __syncthreads();
   bool tileMode = sh.tileMode != 0u;
-  if (tileMode) {  // check every link of the contiguous layout
+  // check every link of the contiguous layout, unless the same frame's tiles pass wrote it
+  if (tileMode && a.proj == nullptr) {
     const uint32_t total = sh.total;
     for (uint32_t k = tid; k < total; k += NT) {
       uint32_t lo = 0, hi = a.B;  // bin of k: binOff[lo] <= k < binOff[lo + 1]
@@ -1454,23 +1492,21 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
   uint32_t running = 0, runningUB = 0;            // slots taken (exact / upper bound)
 
   while (true) {
-    // ---------------- stage the round ----------------
+    // ---------------- stage the round: a thread per segment ----------------
+    uint32_t myBin = 0, myEnc = 0xffffffffu;
     if (tileMode) {
-      if (tid == 0) {
-        uint32_t used;
-        sh.nRuns = buildRuns<TS>(sh, b1, bin, off, STAGE, used);
-        sh.nStaged = used;
+      if (warp == 0) {
+        const uint32_t used = buildRuns<TS>(sh, b1, bin, off, STAGE, lane);
+        if (lane == 0) sh.nStaged = used;
       }
       __syncthreads();
-      const uint32_t nStaged = sh.nStaged, nRuns = sh.nRuns;
-      for (uint32_t k = tid; k < nStaged; k += NT) {
-        uint32_t r = 0;
-        while (r + 1u < nRuns && sh.runK0[r + 1u] <= k) r++;
-        const uint32_t b = sh.runBin[r] & 0xffu;
-        const uint32_t idx = sh.head[b].z - 1u - (sh.runOff[r] + k - sh.runK0[r]);
-        const uint32_t enc = HFB_EXPECT(idx < maxDrawn) ? __ldg(HFB_G(&a.segBuf[1u + 2u * idx])) : 0xffffffffu;
-        sh.enc[k] = enc;
-        sh.listIdx[k] = idx;
+      if (tid < sh.nStaged) {
+        uint32_t j = (uint32_t)__popc(sh.runStart[tid >> 5] & (0xffffffffu >> (31u - lane)));
+        for (uint32_t w = 0; w < tid >> 5; w++) j += (uint32_t)__popc(sh.runStart[w]);
+        myBin = sh.startBin[j - 1u];
+        const uint32_t idx = sh.startBase[j - 1u] - tid;
+        myEnc = HFB_EXPECT(idx < maxDrawn) ? __ldg(HFB_G(&a.segBuf[1u + 2u * idx])) : 0xffffffffu;
+        sh.enc[tid] = myEnc;
       }
     } else {
       while (bin < b1 && sh.head[bin].y == 0u) bin++;  // bins without depth are skipped
@@ -1514,7 +1550,7 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
           sh.nRuns = 1;
           sh.runBin[0] = bin | (ends ? RUN_ENDS : 0u);
           sh.runK0[0] = 0;
-          sh.runK1[0] = m;
+          sh.runK1[0] = (uint16_t)m;
           sh.runOff[0] = processed;
         }
       }
@@ -1533,14 +1569,14 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
       const uint32_t nStaged = sh.nStaged;
 #pragma unroll
       for (uint32_t w = 0; w < STAGE / 32; w++) sh.pixMask[w][tid] = 0u;
+      if (!tileMode && tid < nStaged) {
+        myBin = sh.runBin[0] & 0xffu;
+        myEnc = sh.enc[tid];
+      }
       if (a.proj) {
         // the tiles pass projected every segment of the frame already
-        for (uint32_t k = tid; k < nStaged; k += NT) {
-          uint32_t r = 0;
-          while (r + 1u < nRuns && sh.runK0[r + 1u] <= k) r++;
-          sh.rowBase[k] = stageCached<TS>(sh, k, sh.runBin[r] & 0xffu, a.proj, a.shading, a.S, a.P, a.SP, tbp.x0,
-                                           tbp.y0);
-        }
+        if (tid < nStaged)
+          sh.rowBase[tid] = stageCached<TS>(sh, tid, myBin, a.proj, a.shading, myEnc, a.S, a.P, a.SP, tbp.x0, tbp.y0);
       } else if constexpr (2u * STAGE <= NT) {
         // two threads per segment: one projects its first point, one its second
         if (tid < 2u * nStaged) {
@@ -1548,18 +1584,11 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
           stagePoint<TS>(sh, tid - end * nStaged, end, U, a.pos, a.tan, a.shading, a.S, a.P, a.SP, size);
         }
         __syncthreads();
-        for (uint32_t k = tid; k < nStaged; k += NT) {
-          uint32_t r = 0;
-          while (r + 1u < nRuns && sh.runK0[r + 1u] <= k) r++;
-          sh.rowBase[k] = stageFromPoints<TS>(sh, k, sh.runBin[r] & 0xffu, a.S, a.P, tbp.x0, tbp.y0);
-        }
+        if (tid < nStaged) sh.rowBase[tid] = stageFromPoints<TS>(sh, tid, myBin, a.S, a.P, tbp.x0, tbp.y0);
       } else {
-        for (uint32_t k = tid; k < nStaged; k += NT) {
-          uint32_t r = 0;
-          while (r + 1u < nRuns && sh.runK0[r + 1u] <= k) r++;
-          sh.rowBase[k] = stageSegment<TS>(sh, k, sh.runBin[r] & 0xffu, U, a.pos, a.tan, a.shading, a.S, a.P,
-                                            a.SP, size, tbp.x0, tbp.y0);
-        }
+        if (tid < nStaged)
+          sh.rowBase[tid] =
+              stageSegment<TS>(sh, tid, myBin, U, a.pos, a.tan, a.shading, a.S, a.P, a.SP, size, tbp.x0, tbp.y0);
       }
       __syncthreads();
       // exclusive prefix of the box heights (low half) and areas (high half) together, all
@@ -1667,12 +1696,10 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
       for (uint32_t w = 0; w < warp; w++) pos += sh.red[w];
       if (tid == NT - 1u) atomicMin(&sh.passCount, pos + cnt);  // the total: every row's, unless the list fills up
       if (r0 < r1) {
-        uint32_t end = sh.rowBase[kFirst + 1u], off = sh.rowOff[kFirst], myCnt = 0;
+        uint32_t end = sh.rowBase[kFirst + 1u], off = sh.rowOff[kFirst];
         k = kFirst;
         for (uint32_t r = r0; r < r1; r++) {
           if (r >= end) {
-            if (myCnt && part != FINE_CAREFUL) atomicAdd(&sh.cntEdge[k], myCnt);
-            myCnt = 0;
             do { end = sh.rowBase[++k + 1u]; } while (end <= r);
             off = sh.rowOff[k];
           }
@@ -1691,23 +1718,18 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
             if (HFB_EXPECT(pos < PAIRS)) sh.frag[pos].x = tag + qx;
             pos++;
           }
-          myCnt += n;
         }
-        if (myCnt && part != FINE_CAREFUL) atomicAdd(&sh.cntEdge[k], myCnt);
       }
     }
     __syncthreads();
     nSeg = sh.segLimit;
     if (nSeg < sh.nStaged) {  // uniform: drop the segments from nSeg on
-      if (tid == 0) {
-        sh.nSeg = nSeg;
-        if (tileMode) {
-          uint32_t used;
-          sh.nRuns = buildRuns<TS>(sh, b1, bin, off, nSeg, used);
-        } else {
-          sh.runK1[0] = nSeg;
-          sh.runBin[0] &= ~RUN_ENDS;
-        }
+      if (tid == 0) sh.nSeg = nSeg;
+      if (tileMode) {
+        if (warp == 0) buildRuns<TS>(sh, b1, bin, off, nSeg, lane);
+      } else if (tid == 0) {
+        sh.runK1[0] = (uint16_t)nSeg;
+        sh.runBin[0] &= ~RUN_ENDS;
       }
       __syncthreads();
     }
@@ -1728,7 +1750,12 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
         uint32_t wmode = MODE_FAST, keep = nRuns, we0 = 0, weLast = 0;
         for (uint32_t r = 0; r < nRuns; r++) {
           uint32_t e = 0;
-          for (uint32_t k = sh.runK0[r] + lane; k < sh.runK1[r]; k += 32) e += sh.cntEdge[k];
+          if (part == FINE_CAREFUL) {
+            for (uint32_t k = sh.runK0[r] + lane; k < sh.runK1[r]; k += 32) e += sh.cnt[k];
+          } else {
+            for (uint32_t q = sh.rowBase[sh.runK0[r]] + lane; q < sh.rowBase[sh.runK1[r]]; q += 32)
+              e += (uint32_t)__popc(sh.row[q].pixels());
+          }
           e = __reduce_add_sync(0xffffffffu, e);
           const uint32_t base = r == 0u ? runningUB : 0u;
           if (r == 0u) we0 = e;
@@ -1791,7 +1818,7 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
         if (!inside) continue;
         if (part == FINE_CAREFUL) {
           accepted++;
-          atomicAdd(&sh.cntEdge[k], 1u);
+          atomicAdd(&sh.cnt[k], 1u);
         }
         QuadConst qc;
         qc.sm = mk2(sh.qsx[k], sh.qsy[k]);
@@ -1803,14 +1830,12 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
         const float hd = interpolateHairF32(w, mk4(sh.dp[0][k], sh.dp[1][k], sh.dp[2][k], sh.dp[3][k]));
         if (!(hd < sh.zbuf[pix])) continue;  // depth test with GL_LESS (skip when >=)
         const uint32_t kb = sh.shadeBase[k] >> 24;
-        const float td0 = sh.td0[kb], td1 = sh.td1[kb];
         uint32_t slice;
-        const uint2 col = fragmentColour<TS>(sh, k, w, hd, P, SP, L, td0, td1, alphaQuadratic, alphaMul, shading,
-                                             slice);
+        const uint2 col = fragmentColour<TS>(sh, k, w, hd, P, SP, L, kb, alphaQuadratic, alphaMul, shading, slice);
         sh.frag[i] = col;
         sh.slice[i] = (uint8_t)slice;
         atomicOr(&sh.pixMask[k >> 5][pix], 1u << (k & 31u));
-        if (exact) atomicAdd(&sh.cntFrag[k], 1u);
+        if (exact) atomicAdd(&sh.cnt[k], 1u);
       }
       if (accepted) atomicAdd(&sh.edgePasses, accepted);
     }
@@ -1829,7 +1854,7 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
         uint32_t carry = 0, cut = INVALID_PTR, cutSlots = 0;
         for (uint32_t k0 = 0; k0 < nSeg; k0 += 32) {
           const uint32_t k = k0 + lane;
-          const uint32_t c = k < nSeg ? sh.cntFrag[k] : 0u;
+          const uint32_t c = k < nSeg ? sh.cnt[k] : 0u;
           uint32_t incl = c;
 #pragma unroll
           for (int o = 1; o < 32; o <<= 1) {
@@ -1851,7 +1876,7 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
           sh.roundFrags = carry;
           if (cut != INVALID_PTR) {
             sh.nSeg = cut + 1u;
-            sh.runK1[0] = cut + 1u;
+            sh.runK1[0] = (uint16_t)(cut + 1u);
             sh.runBin[0] |= RUN_ENDS;  // the reference breaks after the filling segment
             atomicAdd(HFB_G(&a.counters->finePoolFullBins), 1ull);
           }
