@@ -216,7 +216,7 @@ uint32_t batchBlocks(const HfbConfig& cfg, BatchKind k, const BatchInst& I) {
       return t;
     }
     case BK_GRID_PRE: return divCeil(G3, 256u);
-    case BK_INTEGRATE: return I.S ? divCeil(I.S, simStrandsPerBlock(I.P)) : 0u;
+    case BK_INTEGRATE: return I.S ? divCeil(I.S, I.simNB) : 0u;
     case BK_GRID_POST: return gridPostBlocks(I.S * I.P);
     case BK_RASTER: return divCeil(nSeg, TILES_RASTER_SEGS);
     case BK_SCAN: return divCeil(TB, 2048u);
@@ -487,6 +487,8 @@ cudaError_t frameBatch(HfbCtx* c, HfbInstance* insts, uint32_t n, float* passMs)
   // the frame's projected segments: one region per instance, written by the
   // tiles pass and read by the fine pass
   size_t segs = 0;
+  uint64_t strands = 0;
+  for (uint32_t i = 0; i < n; i++) strands += insts[i].hair.strandsCount;
   for (uint32_t i = 0; i < n; i++) segs += (size_t)insts[i].hair.strandsCount * (insts[i].hair.pointsPerStrand - 1u);
   e = ensureProjCache(c, segs);
   if (e != cudaSuccess) { delete[] group; return e; }
@@ -498,6 +500,7 @@ cudaError_t frameBatch(HfbCtx* c, HfbInstance* insts, uint32_t n, float* passMs)
     BatchInst& I = ((BatchInst*)(h + BATCH_INSTS_OFF))[ng[g]++];
     fillInstance(cfg, insts[i], I);
     I.proj = c->projCache + segOff * SEG_PROJ_VEC4;
+    I.simNB = simStrandsForBatch(strands, I.P, (uint32_t)c->smCount);
     segOff += (size_t)insts[i].hair.strandsCount * (insts[i].hair.pointsPerStrand - 1u);
     const size_t sb = simSmemBytes(insts[i].hair.pointsPerStrand);
     smem = smem > sb ? smem : sb;
