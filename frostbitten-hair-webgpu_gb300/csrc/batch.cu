@@ -11,6 +11,8 @@
 // the context.
 #include <algorithm>
 #include <cstring>
+#include <initializer_list>
+#include <new>
 
 #define HFB_TU 5
 #include "hfb_internal.cuh"
@@ -19,21 +21,69 @@ namespace hfb {
 
 static_assert(BATCH_GROUPS_MAX == sizeof(HfbCtx::batchStreams) / sizeof(cudaStream_t), "group stream table");
 
+namespace {
+
+constexpr uint32_t CLEAR_CHUNK = 65536;  // bytes cleared per virtual block
+
+struct Range {
+  unsigned char* p;
+  size_t bytes;
+};
+struct Ranges {
+  Range r[8];
+  uint32_t n;
+};
+
+// Zeroes the ranges (whole words): a block per chunk of CLEAR_CHUNK bytes.
+__global__ void __launch_bounds__(256) clearRangesKernel(const Ranges a) {
+  uint32_t c = blockIdx.x, k = 0;
+  for (; k < a.n; k++) {
+    const uint32_t ch = (uint32_t)((a.r[k].bytes + CLEAR_CHUNK - 1) / CLEAR_CHUNK);
+    if (c < ch) break;
+    c -= ch;
+  }
+  if (k == a.n) return;
+  const size_t off = (size_t)c * CLEAR_CHUNK;
+  const size_t end = off + CLEAR_CHUNK < a.r[k].bytes ? off + CLEAR_CHUNK : a.r[k].bytes;
+  unsigned char* p = a.r[k].p;
+  const size_t end16 = (reinterpret_cast<uintptr_t>(p) & 15u) ? off : off + ((end - off) & ~size_t(15));
+  for (size_t x = off + threadIdx.x * 16u; x < end16; x += 256u * 16u)
+    *HFB_G(reinterpret_cast<uint4*>(p + x)) = make_uint4(0u, 0u, 0u, 0u);
+  for (size_t x = end16 + threadIdx.x * 4u; x < end; x += 256u * 4u) *HFB_G(reinterpret_cast<uint32_t*>(p + x)) = 0u;
+}
+
 // cmdClearBeforeRender of the tiles, fine and sort passes (hairTilesPass.ts:48-52,
-// hairFinePass.ts:50-55, hairTileSortPass.ts:63-68).
-cudaError_t clearRaster(HfbCtx* c, const HfbRasterBuffers& rb) {
+// hairFinePass.ts:50-55, hairTileSortPass.ts:63-68), in one launch instead of six memsets
+// (about 2 us each on the frame's critical path); with `tilesPass`, the tiles pass's own
+// counters too.
+cudaError_t clearRasterRanges(HfbCtx* c, const HfbRasterBuffers& rb, bool tilesPass) {
+  HFB_CHECK_BIND(c);
   const HfbConfig& cfg = c->cfg;
   const size_t T = (size_t)divCeil(rb.width, cfg.tileSize) * divCeil(rb.height, cfg.tileSize);
-  cudaError_t e = cudaSuccess;
-  auto z = [&](void* p, size_t n) { if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, n, c->stream); };
+  Ranges a{};
+  auto z = [&](void* p, size_t n) { a.r[a.n++] = {(unsigned char*)p, n}; };
   z(rb.tiles, T * cfg.tileDepthBins * 16);
   z(rb.segmentCountPerTile, T * 4);
   z(rb.tileSegments, 4);
   z(rb.rasterizerResult, 16 + (size_t)rb.width * rb.height * 16);
   z(rb.tileList, 4);
   z(rb.sortBuckets, (size_t)cfg.sortBuckets * 8);
-  return e;
+  if (tilesPass) {
+    const TilesScratch ts = tilesScratchLayout(rb.scratch, cfg, rb.width, rb.height, rb.maxDrawnSegments);
+    z(ts.binCount, T * cfg.tileDepthBins * 4);
+    z(ts.largeBins, 4);
+  }
+  uint32_t blocks = 0;
+  for (uint32_t k = 0; k < a.n; k++) blocks += (uint32_t)((a.r[k].bytes + CLEAR_CHUNK - 1) / CLEAR_CHUNK);
+  clearRangesKernel<<<blocks, 256, 0, c->stream>>>(a);
+  HFB_AFTER_LAUNCH(c, "clearRangesKernel");
+  c->launches += 1;
+  return cudaGetLastError();
 }
+
+}  // namespace
+
+cudaError_t clearRaster(HfbCtx* c, const HfbRasterBuffers& rb) { return clearRasterRanges(c, rb, false); }
 
 // One pass of one instance's frame (renderer.ts:171-295).  Integration
 // writes positions[1 - current]; every later pass reads those new
@@ -55,13 +105,14 @@ cudaError_t framePass(HfbCtx* c, HfbInstance* in, FramePass p) {
                                 in->densityVelocity, in->densityGradWind, in->sdf, in->sdfDims);
     case FP_GRID_POST:  // after the swap: "prev" = the old positions, "now" = the new ones
       return launchGridPostSim(c, su, h, now, prev, in->densityVelocity, in->gridOrder);
-    case FP_CLEAR:
-      return clearRaster(c, rb);
+    case FP_CLEAR:  // with the tiles pass's counters
+      return clearRasterRanges(c, rb, true);
     case FP_TILES: {
       // the segments' projections, for this frame's fine pass
       const cudaError_t e = ensureProjCache(c, (size_t)h.strandsCount * (h.pointsPerStrand - 1u));
       if (e != cudaSuccess) return e;
-      return launchTilesPass(c, u, h, prev, in->tangents, in->sceneDepth, in->strandsToRender, rb, c->projCache);
+      return launchTilesPass(c, u, h, prev, in->tangents, in->sceneDepth, in->strandsToRender, rb, c->projCache,
+                             true);
     }
     case FP_SORT:
       return launchTileSort(c, rb);
@@ -79,6 +130,122 @@ cudaError_t framePass(HfbCtx* c, HfbInstance* in, FramePass p) {
     default:
       return cudaErrorInvalidValue;
   }
+}
+
+// ---------------------------------------------------------------------------
+// What a frame runs beside its main chain of passes, on the context's side
+// stream: the raster clears, which wait for nothing of the frame, beside the
+// simulation; and, once the positions are there, the grid splat (read by the next
+// frame) and the hair depth (read by the shading) beside the tiles, sort and fine
+// passes, which alone leave most of a GPU idle on one instance.  The hair depth
+// may not run beside the tiles and fine passes where they read what it writes: a
+// frame whose hairDepth overlaps a sceneDepth keeps everything in turn on the
+// caller's stream.
+// ---------------------------------------------------------------------------
+enum SideEvent : uint32_t { SE_START = 0, SE_CLEAR, SE_SIM, SE_DONE };
+
+void sideCreate(HfbCtx* c) {
+  cudaError_t e = cudaStreamCreateWithFlags(&c->sideStream, cudaStreamNonBlocking);
+  for (int i = 0; i < 4 && e == cudaSuccess; i++) e = cudaEventCreateWithFlags(&c->sideEvents[i], cudaEventDisableTiming);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    sideRelease(c);
+  }
+}
+
+void sideRelease(HfbCtx* c) {
+  for (cudaEvent_t& ev : c->sideEvents) {
+    if (ev) cudaEventDestroy(ev);
+    ev = nullptr;
+  }
+  if (c->sideStream) cudaStreamDestroy(c->sideStream);
+  c->sideStream = nullptr;
+}
+
+// Runs f with the side stream as the context's.
+template <class F>
+static cudaError_t onSide(HfbCtx* c, F f) {
+  const cudaStream_t caller = c->stream;
+  c->stream = c->sideStream;
+  const cudaError_t e = f();
+  c->stream = caller;
+  return e;
+}
+
+// A frame's passes: start(side), sim(main), after(side), raster(main), shade(main), with the
+// side stream forked from the caller's and joined back into it, also after a failed launch.
+template <class Start, class Sim, class After, class Raster, class Shade>
+static cudaError_t forkedFrame(HfbCtx* c, Start start, Sim sim, After after, Raster raster, Shade shade) {
+  const cudaStream_t M = c->stream, S = c->sideStream;
+  const cudaEvent_t* ev = c->sideEvents;
+  cudaError_t e = cudaEventRecord(ev[SE_START], M);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(S, ev[SE_START], 0);
+  if (e != cudaSuccess) return e;
+  e = onSide(c, start);
+  if (e == cudaSuccess) e = cudaEventRecord(ev[SE_CLEAR], S);
+  if (e == cudaSuccess) e = sim();
+  if (e == cudaSuccess) e = cudaEventRecord(ev[SE_SIM], M);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(S, ev[SE_SIM], 0);
+  if (e == cudaSuccess) e = onSide(c, after);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(M, ev[SE_CLEAR], 0);
+  if (e == cudaSuccess) e = raster();
+  cudaError_t ej = cudaEventRecord(ev[SE_DONE], S);
+  if (ej == cudaSuccess) ej = cudaStreamWaitEvent(M, ev[SE_DONE], 0);
+  if (e == cudaSuccess) e = ej;
+  if (e == cudaSuccess) e = shade();
+  return e;
+}
+
+// Whether [a, a + an) and [b, b + bn) share a byte.
+static bool overlap(const void* a, size_t an, const void* b, size_t bn) {
+  const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+  return x < y + bn && y < x + an;
+}
+static size_t depthBytes(const HfbInstance& in) { return (size_t)in.raster.width * in.raster.height * 4; }
+
+// Whether some instance's hairDepth overlaps some instance's sceneDepth.
+static bool depthsOverlap(const HfbInstance* in, uint32_t n) {
+  if (n == 1)
+    return in->hairDepth && overlap(in->hairDepth, depthBytes(*in), in->sceneDepth, depthBytes(*in));
+  struct Span {
+    uintptr_t p, end;
+  };
+  Span* scene = new (std::nothrow) Span[n];  // sorted by start; the furthest end up to each
+  if (!scene) return true;
+  for (uint32_t i = 0; i < n; i++) {
+    const uintptr_t p = (uintptr_t)in[i].sceneDepth;
+    scene[i] = {p, p + depthBytes(in[i])};
+  }
+  std::sort(scene, scene + n, [](const Span& a, const Span& b) { return a.p < b.p; });
+  for (uint32_t i = 1; i < n; i++) scene[i].end = std::max(scene[i].end, scene[i - 1].end);
+  bool found = false;
+  for (uint32_t i = 0; i < n && !found; i++) {
+    if (!in[i].hairDepth) continue;
+    const uintptr_t p = (uintptr_t)in[i].hairDepth, end = p + depthBytes(in[i]);
+    // the sceneDepths that start before this one ends
+    const Span* it = std::lower_bound(scene, scene + n, end, [](const Span& a, uintptr_t v) { return a.p < v; });
+    found = it != scene && (it - 1)->end > p;
+  }
+  delete[] scene;
+  return found;
+}
+
+cudaError_t frameOne(HfbCtx* c, HfbInstance* in) {
+  auto pass = [&](FramePass p) { return framePass(c, in, p); };
+  auto passes = [&](std::initializer_list<FramePass> ps) {
+    cudaError_t e = cudaSuccess;
+    for (FramePass p : ps)
+      if (e == cudaSuccess) e = pass(p);
+    return e;
+  };
+  // grown before the fork: growing waits for the streams
+  const cudaError_t e = ensureProjCache(c, (size_t)in->hair.strandsCount * (in->hair.pointsPerStrand - 1u));
+  if (e != cudaSuccess) return e;
+  if (!c->sideStream || depthsOverlap(in, 1))
+    return passes({FP_GRID_PRE, FP_INTEGRATE, FP_GRID_POST, FP_CLEAR, FP_TILES, FP_SORT, FP_FINE, FP_HAIR_DEPTH, FP_SHADING});
+  return forkedFrame(c, [&] { return passes({FP_CLEAR}); }, [&] { return passes({FP_GRID_PRE, FP_INTEGRATE}); },
+                     [&] { return passes({FP_HAIR_DEPTH, FP_GRID_POST}); },
+                     [&] { return passes({FP_TILES, FP_SORT, FP_FINE}); }, [&] { return passes({FP_SHADING}); });
 }
 
 cudaError_t ensureProjCache(HfbCtx* c, size_t segments) {
@@ -105,13 +272,6 @@ cudaError_t ensureProjCache(HfbCtx* c, size_t segments) {
 }
 
 namespace {
-
-constexpr uint32_t CLEAR_CHUNK = 65536;  // bytes cleared per virtual block
-
-struct Range {
-  unsigned char* p;
-  size_t bytes;
-};
 
 // What a frame clears for one instance before the raster passes: the
 // reference's cmdClearBeforeRender of the tiles, fine and sort passes
@@ -291,6 +451,31 @@ static cudaError_t batchSequence(HfbCtx* c, const BatchView& b, cudaEvent_t* ev 
   return e;
 }
 
+// The same passes, those that need not be in turn on the side stream.
+static cudaError_t batchSequenceForked(HfbCtx* c, const BatchView& b) {
+  return forkedFrame(
+      c,
+      [&] {
+        const cudaError_t e = launchBatchClear(c, b, BK_CLEAR_FRAME);
+        return e == cudaSuccess ? launchBatchDepthCopy(c, b) : e;
+      },
+      [&] {
+        const cudaError_t e = launchBatchSim(c, b, BK_GRID_PRE);
+        return e == cudaSuccess ? launchBatchSim(c, b, BK_INTEGRATE) : e;
+      },
+      [&] {
+        cudaError_t e = launchBatchHairDepth(c, b);
+        if (e == cudaSuccess) e = launchBatchClear(c, b, BK_CLEAR_GRID);
+        return e == cudaSuccess ? launchBatchSim(c, b, BK_GRID_POST) : e;
+      },
+      [&] {
+        cudaError_t e = launchBatchTiles(c, b);
+        if (e == cudaSuccess) e = launchBatchSort(c, b);
+        return e == cudaSuccess ? launchBatchFine(c, b) : e;
+      },
+      [&] { return launchBatchShading(c, b); });
+}
+
 // One instance as the batched kernels read it.
 static void fillInstance(const HfbConfig& cfg, const HfbInstance& s, BatchInst& I) {
   memset(&I, 0, sizeof(I));
@@ -357,8 +542,8 @@ static cudaError_t ensureGroupStreams(HfbCtx* c) {
 
 // The launch sequence of NG groups: one group on c->stream, or each group
 // on its own worker stream, forked from c->stream and joined back into it.
-static cudaError_t groupsSequence(HfbCtx* c, uint32_t NG) {
-  if (NG == 1) return batchSequence(c, batchView(c->batchDev));
+static cudaError_t groupsSequence(HfbCtx* c, uint32_t NG, bool side) {
+  if (NG == 1) return side ? batchSequenceForked(c, batchView(c->batchDev)) : batchSequence(c, batchView(c->batchDev));
   const cudaStream_t caller = c->stream;
   cudaError_t e = cudaEventRecord(c->batchFork, caller);
   for (uint32_t g = 0; g < NG && e == cudaSuccess; g++) e = cudaStreamWaitEvent(c->batchStreams[g], c->batchFork, 0);
@@ -393,6 +578,13 @@ static cudaError_t ensurePipe(HfbCtx* c) {
     if (e == cudaSuccess && !c->pipeCaller[i]) e = cudaEventCreateWithFlags(&c->pipeCaller[i], cudaEventDisableTiming);
   }
   return e;
+}
+
+static void batchGraphsRelease(HfbCtx* c) {
+  for (cudaGraphExec_t& g : c->batchGraph) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
 }
 
 static void pipeGraphsRelease(HfbCtx* c) {
@@ -487,8 +679,11 @@ cudaError_t frameBatch(HfbCtx* c, HfbInstance* insts, uint32_t n, float* passMs)
   // the frame's projected segments: one region per instance, written by the
   // tiles pass and read by the fine pass
   size_t segs = 0;
-  uint64_t strands = 0;
-  for (uint32_t i = 0; i < n; i++) strands += insts[i].hair.strandsCount;
+  uint64_t strands = 0, fullBlocks = 0;
+  for (uint32_t i = 0; i < n; i++) {
+    strands += insts[i].hair.strandsCount;
+    fullBlocks += divCeil(insts[i].hair.strandsCount, simStrandsPerBlock(insts[i].hair.pointsPerStrand));
+  }
   for (uint32_t i = 0; i < n; i++) segs += (size_t)insts[i].hair.strandsCount * (insts[i].hair.pointsPerStrand - 1u);
   e = ensureProjCache(c, segs);
   if (e != cudaSuccess) { delete[] group; return e; }
@@ -515,8 +710,7 @@ cudaError_t frameBatch(HfbCtx* c, HfbInstance* insts, uint32_t n, float* passMs)
     for (int i = 0; i < 2 && e == cudaSuccess; i++)
       if (c->pipeStream[i]) e = cudaStreamSynchronize(c->pipeStream[i]);
     if (e != cudaSuccess) return e;
-    if (c->batchGraph) cudaGraphExecDestroy(c->batchGraph);
-    c->batchGraph = nullptr;
+    batchGraphsRelease(c);
     pipeGraphsRelease(c);
   }
   for (uint32_t g = 0; g < NG && e == cudaSuccess; g++) {
@@ -583,45 +777,49 @@ cudaError_t frameBatch(HfbCtx* c, HfbInstance* insts, uint32_t n, float* passMs)
     return cudaGetLastError();
   }
 #ifdef HFB_DEVICE_CHECKS
-  c->batchGraphLaunches = ~0ull;  // the checked build waits after every launch: no capture
+  c->batchNoGraph = true;  // the checked build waits after every launch: no capture
 #endif
-  if (c->batchGraph && c->batchGraphGroups != NG) {  // made for another number of groups
+  const bool side = NG == 1u && c->sideStream && fullBlocks <= (uint64_t)SIDE_MAX_BLOCKS * c->smCount &&
+                    !depthsOverlap(insts, n);
+  cudaGraphExec_t& graph = c->batchGraph[side ? 1 : 0];
+  uint64_t& graphLaunches = c->batchGraphLaunches[side ? 1 : 0];
+  if (!side && graph && c->batchGraphGroups != NG) {  // made for another number of groups
     e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return e;
-    cudaGraphExecDestroy(c->batchGraph);
-    c->batchGraph = nullptr;
+    cudaGraphExecDestroy(graph);
+    graph = nullptr;
   }
-  if (c->batchCalls++ == 0 || c->batchGraphLaunches == ~0ull) {
+  if (c->batchCalls++ == 0 || c->batchNoGraph) {
     // the first batch (which also sets the kernels' attributes), or no graph: plain launches
-    e = groupsSequence(c, NG);
+    e = groupsSequence(c, NG, side);
   } else {
-    if (!c->batchGraph) {
+    if (!graph) {
       cudaGraph_t gr = nullptr;
       e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
       if (e != cudaSuccess) return e;
       const uint64_t l0 = c->launches;
-      cudaError_t el = groupsSequence(c, NG);
+      cudaError_t el = groupsSequence(c, NG, side);
       const uint64_t captured = c->launches - l0;
       c->launches = l0;
       e = cudaStreamEndCapture(c->stream, &gr);
       if (el != cudaSuccess) e = el;
-      if (e == cudaSuccess) e = cudaGraphInstantiate(&c->batchGraph, gr, 0);
+      if (e == cudaSuccess) e = cudaGraphInstantiate(&graph, gr, 0);
       if (gr) cudaGraphDestroy(gr);
       if (e != cudaSuccess) {
         // a stream that cannot be captured (e.g. the legacy default stream): plain launches
         cudaGetLastError();
-        c->batchGraph = nullptr;
-        c->batchGraphLaunches = ~0ull;
-        e = groupsSequence(c, NG);
+        graph = nullptr;
+        c->batchNoGraph = true;
+        e = groupsSequence(c, NG, side);
         if (e != cudaSuccess) return e;
         for (uint32_t i = 0; i < n; i++) insts[i].current ^= 1u;
         return cudaGetLastError();
       }
-      c->batchGraphLaunches = captured;
-      c->batchGraphGroups = NG;
+      graphLaunches = captured;
+      if (!side) c->batchGraphGroups = NG;
     }
-    e = cudaGraphLaunch(c->batchGraph, c->stream);
-    c->launches += c->batchGraphLaunches;
+    e = cudaGraphLaunch(graph, c->stream);
+    c->launches += graphLaunches;
   }
   if (e != cudaSuccess) return e;
   for (uint32_t i = 0; i < n; i++) insts[i].current ^= 1u;
@@ -646,13 +844,12 @@ void frameBatchRelease(HfbCtx* c) {
   }
   if (c->batchFork) cudaEventDestroy(c->batchFork);
   c->batchFork = nullptr;
-  if (c->batchGraph) cudaGraphExecDestroy(c->batchGraph);
+  batchGraphsRelease(c);
   for (int k = 0; k < 2; k++) {
     if (c->batchCopied[k]) cudaEventDestroy(c->batchCopied[k]);
     if (c->batchHost[k]) cudaFreeHost(c->batchHost[k]);
   }
   if (c->batchDev) cudaFree(c->batchDev);
-  c->batchGraph = nullptr;
   c->batchDev = nullptr;
   if (c->projCache) cudaFree(c->projCache);
   c->projCache = nullptr;

@@ -110,6 +110,7 @@ int hfb_ctx_create(const HfbConfig* cfg, int device, HfbCtx** out) {
   cudaMemsetAsync(c->dCounters, 0, sizeof(hfb::DeviceCounters), c->stream);
   cudaStreamSynchronize(c->stream);
   hfb::noallocPrepare(c);
+  hfb::sideCreate(c);
   *out = c;
   return HFB_OK;
 }
@@ -118,6 +119,7 @@ int hfb_ctx_destroy(HfbCtx* c) {
   HFB_CHECK_CTX(c);
   cudaStreamSynchronize(c->stream);
   hfb::frameBatchRelease(c);
+  hfb::sideRelease(c);
   if (c->checkDev) cudaFree(c->checkDev);
   if (c->dCounters) cudaFree(c->dCounters);
   if (c->ownStream) cudaStreamDestroy(c->ownStream);
@@ -541,8 +543,7 @@ int hfb_frame(HfbCtx* c, HfbInstance* in) {
   HFB_CHECK_CTX(c);
   std::string err = checkInstance(c, in);
   HFB_REQUIRE(c, err.empty(), err);
-  cudaError_t e = cudaSuccess;
-  for (uint32_t p = 0; p < hfb::FP_COUNT && e == cudaSuccess; p++) e = hfb::framePass(c, in, (hfb::FramePass)p);
+  cudaError_t e = hfb::frameOne(c, in);
   if (e != cudaSuccess) return cudaFail(c, e, "frame");
   in->current ^= 1u;
   return HFB_OK;

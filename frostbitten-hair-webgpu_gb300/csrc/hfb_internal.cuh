@@ -30,14 +30,15 @@ struct HfbCtx {
   cudaEvent_t batchCopied[2] = {nullptr, nullptr};
   uint32_t batchFlip = 0;
   uint32_t batchGrid[32] = {};
-  cudaGraphExec_t batchGraph = nullptr;
-  uint64_t batchGraphLaunches = 0;  // kernels in the graph
+  cudaGraphExec_t batchGraph[2] = {};     // [1]: with the side stream
+  uint64_t batchGraphLaunches[2] = {};    // kernels in each graph
+  bool batchNoGraph = false;              // the stream cannot be captured: plain launches
   uint32_t batchCalls = 0;
   size_t simBatchSmem = 0;  // shared memory of the batched integration launch
   // groups of a batched frame: each group's passes on its own worker stream,
   // its persistent launches sized to 1 / groups of the GPU
   uint32_t batchGroups = 1;       // requested (hfb_ctx_set_batch_groups)
-  uint32_t batchGraphGroups = 0;  // groups the captured graph was made with
+  uint32_t batchGraphGroups = 0;  // groups batchGraph[0] was made with
   uint32_t batchGridDiv = 1;      // divisor of the persistent grids while a group launches
   cudaStream_t batchStreams[4] = {};
   cudaEvent_t batchFork = nullptr;
@@ -59,6 +60,10 @@ struct HfbCtx {
   // failed; noallocError then says why)
   void* noallocScratch = nullptr;
   std::string noallocError;
+  // whole frames: a second stream for what does not wait for the passes on the caller's
+  // (made with the context; NULL: everything on the caller's stream)
+  cudaStream_t sideStream = nullptr;
+  cudaEvent_t sideEvents[4] = {};  // frame start, clears done, simulated, side work done
   // the projected segments of a whole frame (hfb_frame, hfb_frame_batch):
   // written by the tiles pass, read by the fine pass; grown on demand
   float4* projCache = nullptr;
@@ -118,6 +123,13 @@ __host__ __device__ inline uint32_t simStrandsPerBlockFor(uint32_t S, uint32_t P
 // batch does not give every SM its SIM_BATCH_BLOCKS of them, down to 8 strands, so that
 // they take one wave: a tick of 6 sessions (35,000 strands of 32) 382 -> 308 us.
 constexpr uint32_t SIM_BATCH_BLOCKS = 6;
+// Integration blocks (full ones) per SM up to which a batch runs its side passes on the
+// side stream: measured on batches of the 64-instance mix and of sessions, 3 sessions 690
+// -> 618 us, 6 1,348 -> 1,250, 16 instances (10 blocks per SM) 2,914 -> 2,887, 24 (19)
+// 5,015 -> 4,974; from there on the persistent kernels fill the GPU by themselves and get
+// in one another's way (48 sessions, 27 per SM: 8,412 -> 8,556; 64 instances, 50: 12.39 ->
+// 12.74 ms).
+constexpr uint32_t SIDE_MAX_BLOCKS = 16;
 inline uint32_t simStrandsForBatch(uint64_t S, uint32_t P, uint32_t smCount) {
   const uint32_t full = simStrandsPerBlock(P);
   const uint64_t want = (S + SIM_BATCH_BLOCKS * smCount - 1u) / (SIM_BATCH_BLOCKS * smCount) + 1u;  // + 1: partial blocks
@@ -139,14 +151,14 @@ cudaError_t launchGridPostSim(HfbCtx* c, const HfbSimUniforms& u, const HfbHairD
 cudaError_t launchShading(HfbCtx* c, const HfbUniforms& u, const HfbHairData& h, const float* pos,
                           const float* tan, const float* depth, const float* ao, uint32_t aoW,
                           uint32_t aoH, const float* sm, uint32_t smSize, float* shading);
-// proj (NULL = none): per segment, SEG_PROJ_VEC4 float4 of its projection
+// cleared: the pass's own counters are zero already.  proj (NULL = none): per segment, SEG_PROJ_VEC4 float4 of its projection
 // (projectSegment) that the tiles pass writes and the fine pass of the same
 // frame reads instead of projecting again (whole frames only, where the
 // library runs both passes on the same positions and uniforms).
 constexpr uint32_t SEG_PROJ_VEC4 = 3;  // v00, v01 | v10, v11 | depthsProj
 cudaError_t launchTilesPass(HfbCtx* c, const HfbUniforms& u, const HfbHairData& h, const float* pos,
                             const float* tan, const float* depth, uint32_t strandsToRender,
-                            HfbRasterBuffers& rb, float4* proj = nullptr);
+                            HfbRasterBuffers& rb, float4* proj = nullptr, bool cleared = false);
 cudaError_t launchTileSort(HfbCtx* c, HfbRasterBuffers& rb);
 cudaError_t launchFinePass(HfbCtx* c, const HfbUniforms& u, const HfbHairData& h, const float* pos,
                            const float* tan, const float* shading, const float* depth,
@@ -208,7 +220,11 @@ enum FramePass : uint32_t {
   FP_COUNT
 };
 cudaError_t framePass(HfbCtx* c, HfbInstance* in, FramePass p);
+// One frame of one checked instance, on c->stream and the context's side stream.
+cudaError_t frameOne(HfbCtx* c, HfbInstance* in);
 cudaError_t clearRaster(HfbCtx* c, const HfbRasterBuffers& rb);
+void sideCreate(HfbCtx* c);
+void sideRelease(HfbCtx* c);
 
 // Looks up the device address of hfb_tiles_pass_noalloc's fixed array with
 // the context's device current (noalloc.cu), which also loads that code

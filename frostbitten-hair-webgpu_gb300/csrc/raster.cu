@@ -2454,16 +2454,19 @@ cudaError_t launchFineBatchT(HfbCtx* c, const BatchView& b) {
 
 cudaError_t launchTilesPass(HfbCtx* c, const HfbUniforms& u, const HfbHairData& h, const float* pos,
                             const float* tan, const float* depth, uint32_t strandsToRender, HfbRasterBuffers& rb,
-                            float4* proj) {
+                            float4* proj, bool cleared) {
   HFB_CHECK_BIND(c);
   const HfbConfig& cfg = c->cfg;
   const uint32_t W = rb.width, H = rb.height, TS = cfg.tileSize, B = cfg.tileDepthBins;
   const uint32_t T = divCeil(W, TS) * divCeil(H, TS);
   const uint32_t TB = T * B;
   TilesScratch s = tilesScratchLayout(rb.scratch, cfg, W, H, rb.maxDrawnSegments);
-  cudaError_t e = cudaMemsetAsync(s.binCount, 0, (size_t)TB * 4, c->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(s.largeBins, 0, 4, c->stream);
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
+  if (!cleared) {
+    e = cudaMemsetAsync(s.binCount, 0, (size_t)TB * 4, c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(s.largeBins, 0, 4, c->stream);
+    if (e != cudaSuccess) return e;
+  }
   const uint32_t nStrands = min(strandsToRender, h.strandsCount);
   const uint32_t nSeg = nStrands * (h.pointsPerStrand - 1u);
   DeviceCounters* dc = (DeviceCounters*)c->dCounters;
