@@ -36,6 +36,7 @@ namespace {
 constexpr uint32_t INVALID_PTR = 0xffffffffu;
 constexpr float F_MAX_U32 = 4294967296.0f;  // f32(MAX_U32)
 constexpr uint32_t SMALL_BIN = 32;
+constexpr uint32_t WARP_BIN = 256;  // keys of one warp; 8 WARP_BIN >= MEDIUM_BIN words per block
 constexpr uint32_t MEDIUM_BIN = 1024;
 constexpr uint32_t LARGE_SMEM_KEYS = 16384;
 constexpr int SCAN_PER_BLOCK = 2048;
@@ -564,12 +565,23 @@ __device__ __forceinline__ void binScatterBody(const uint32_t* __restrict__ segB
   const uint32_t total = (*HFB_G(&segBuf[0]));
   const uint32_t n = min(total, maxDrawn);
   if (blk == 0 && threadIdx.x == 0) atomicAdd(HFB_G(&counters->tileRecords), (unsigned long long)total);
-  for (uint32_t r = blk * blockDim.x + threadIdx.x; r < n; r += nblk * blockDim.x) {
-    uint32_t ti = (*HFB_G(&segBuf[1u + 2u * r]));
-    uint32_t key = (*HFB_G(&segBuf[2u + 2u * r]));
-    if (!HFB_EXPECT(ti < TB)) continue;
-    uint32_t pos = (*HFB_G(&blockSums[ti / SCAN_PER_BLOCK])) + atomicAdd(HFB_G(&binOffset[ti]), 1u);
-    if (HFB_EXPECT(pos < maxDrawn)) (*HFB_G(&keys[pos])) = key;
+  // The records of a warp come from a few neighbouring segments, so many fall into
+  // the same bin, whose counter takes one atomic after the other: one lane adds for
+  // all the lanes of its bin.  359,604 records: 18.5 -> 11 us, 7.6 million: 159 -> 105 us;
+  // four records per lane in flight gave nothing.
+  const uint32_t step = nblk * blockDim.x, lane = threadIdx.x & 31u;
+  for (uint64_t r0 = blk * blockDim.x + (threadIdx.x - lane); r0 < n; r0 += step) {
+    const uint64_t r = r0 + lane;
+    uint32_t ti = r < n ? (*HFB_G(&segBuf[1u + 2u * (uint32_t)r])) : 0xffffffffu;
+    const uint32_t key = r < n ? (*HFB_G(&segBuf[2u + 2u * (uint32_t)r])) : 0u;
+    if (r < n && !HFB_EXPECT(ti < TB)) ti = 0xffffffffu;
+    const uint32_t peers = __match_any_sync(0xffffffffu, ti);
+    const uint32_t leader = __ffs(peers) - 1u;
+    uint32_t pos = 0;
+    if (lane == leader && ti < TB)
+      pos = (*HFB_G(&blockSums[ti / SCAN_PER_BLOCK])) + atomicAdd(HFB_G(&binOffset[ti]), (uint32_t)__popc(peers));
+    pos = __shfl_sync(0xffffffffu, pos, leader) + __popc(peers & ((1u << lane) - 1u));
+    if (ti < TB && HFB_EXPECT(pos < maxDrawn)) (*HFB_G(&keys[pos])) = key;
   }
 }
 
@@ -657,25 +669,29 @@ __device__ __forceinline__ void bitonicSort(uint32_t* s, uint32_t N) {
   }
 }
 
-// Sorts and links the larger bin ti (more than 8 records) with the whole warp.
-__device__ __forceinline__ void finalizeBinWarp(uint32_t ti, uint32_t n, uint32_t start, uint32_t lane,
-                                                uint32_t* __restrict__ keys, uint32_t* __restrict__ segBuf,
-                                                uint4* __restrict__ tiles, uint32_t* __restrict__ largeBins,
-                                                uint32_t* s) {
-  if (n <= SMALL_BIN) {
-    uint32_t v = lane < n ? (*HFB_G(&keys[start + lane])) : 0xffffffffu;
-    // bitonic sort across the warp, ascending
+// Bitonic sort of one key per lane across the warp, ascending.
+__device__ __forceinline__ uint32_t sortWarp32(uint32_t v, uint32_t lane) {
 #pragma unroll
-    for (uint32_t k = 2; k <= 32; k <<= 1) {
+  for (uint32_t k = 2; k <= 32; k <<= 1) {
 #pragma unroll
-      for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-        uint32_t o = __shfl_xor_sync(0xffffffffu, v, j);
-        bool asc = (lane & k) == 0, low = (lane & j) == 0;
-        v = (asc == low) ? min(v, o) : max(v, o);
-      }
+    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+      const uint32_t o = __shfl_xor_sync(0xffffffffu, v, j);
+      const bool asc = (lane & k) == 0, low = (lane & j) == 0;
+      v = (asc == low) ? min(v, o) : max(v, o);
     }
+  }
+  return v;
+}
+
+// Sorts and links bin ti of at most WARP_BIN records with the whole warp (s: WARP_BIN
+// words of the warp's own).
+__device__ __forceinline__ void finalizeBinWarp(uint32_t ti, uint32_t n, uint32_t start, uint32_t lane,
+                                                const uint32_t* __restrict__ keys, uint32_t* __restrict__ segBuf,
+                                                uint4* __restrict__ tiles, uint32_t* s) {
+  if (n <= SMALL_BIN) {
+    const uint32_t v = sortWarp32(lane < n ? (*HFB_G(&keys[start + lane])) : 0xffffffffu, lane);
     if (lane < n) writeList(segBuf, tiles, ti, start, lane, n, v);
-  } else if (n <= MEDIUM_BIN) {
+  } else {
     uint32_t N = 64;
     while (N < n) N <<= 1;
     for (uint32_t i = lane; i < N; i += 32) s[i] = i < n ? (*HFB_G(&keys[start + i])) : 0xffffffffu;
@@ -683,31 +699,144 @@ __device__ __forceinline__ void finalizeBinWarp(uint32_t ti, uint32_t n, uint32_
     bitonicSort<false>(s, N);
     for (uint32_t i = lane; i < n; i += 32) writeList(segBuf, tiles, ti, start, i, n, s[i]);
     __syncwarp();
-  } else if (lane == 0) {
-    uint32_t slot = atomicAdd(HFB_G(&largeBins[0]), 1u);
-    (*HFB_G(&largeBins[1u + slot])) = ti;
   }
 }
 
-// One warp per bin, the warps of the grid striding over the bins (the
-// single-instance launch: a fixed grid, where spreading the larger bins over
-// every warp keeps the tail short).
+// Sorts and links bin ti of more than WARP_BIN records with the whole block (s: 8 WARP_BIN
+// words), or leaves it to largeBins.  A single warp takes ~16 us for 1,024 records, which
+// was the pass's tail.  All threads of the block call it.
+__device__ __forceinline__ void finalizeBinBlock(uint32_t ti, uint32_t n, uint32_t start,
+                                                 const uint32_t* __restrict__ keys, uint32_t* __restrict__ segBuf,
+                                                 uint4* __restrict__ tiles, uint32_t* __restrict__ largeBins,
+                                                 uint32_t* s) {
+  if (n > MEDIUM_BIN) {
+    if (threadIdx.x == 0) {
+      const uint32_t slot = atomicAdd(HFB_G(&largeBins[0]), 1u);
+      (*HFB_G(&largeBins[1u + slot])) = ti;
+    }
+    return;
+  }
+  uint32_t N = 64;
+  while (N < n) N <<= 1;
+  for (uint32_t i = threadIdx.x; i < N; i += blockDim.x) s[i] = i < n ? (*HFB_G(&keys[start + i])) : 0xffffffffu;
+  __syncthreads();
+  bitonicSort<true>(s, N);
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) writeList(segBuf, tiles, ti, start, i, n, s[i]);
+  __syncthreads();
+}
+
+// Sorts a bin of at most 8 records across the 8 lanes of a group (gl: the lane
+// in its group; 0xffffffff past the bin's end), ascending.  mask: the lanes
+// that call it, whole groups.
+__device__ __forceinline__ uint32_t sortGroup8(uint32_t v, uint32_t gl, uint32_t mask) {
+#pragma unroll
+  for (uint32_t k = 2; k <= 8; k <<= 1) {
+#pragma unroll
+    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+      const uint32_t o = __shfl_xor_sync(mask, v, j);
+      const bool asc = (gl & k) == 0, low = (gl & j) == 0;
+      v = (asc == low) ? min(v, o) : max(v, o);
+    }
+  }
+  return v;
+}
+
+// The warps of the grid stride over the bins (the single-instance launch: a
+// fixed grid, where spreading the larger bins over every warp keeps the tail
+// short).  Most bins are empty and a bin is a chain of dependent loads, so a
+// warp reads 32 of its bins' counts and ends at once, one per lane; it then
+// takes the bins of at most 8 records four at a time, 8 lanes each, and the
+// others up to WARP_BIN one at a time, the next bins' keys on their way while these are
+// sorted; the larger ones wait in a queue for the whole block.  Against a warp that
+// walks its bins one by one up to 1,024 records: 1,036,800 bins, 338,890 records of at
+// most 80 per bin, 77 -> 18 us; 130,560 bins, 359,604 records of at most 759, 43 -> 21 us.
 __device__ __forceinline__ void binFinalizeWarpBody(uint32_t TB, const uint32_t* __restrict__ binCount,
                                                     const uint32_t* __restrict__ binOffset,
                                                     const uint32_t* __restrict__ blockSums,
                                                     uint32_t* __restrict__ keys, uint32_t* __restrict__ segBuf,
                                                     uint4* __restrict__ tiles, uint32_t* __restrict__ largeBins,
-                                                    uint32_t (*smem)[MEDIUM_BIN], uint32_t blk, uint32_t nblk) {
+                                                    uint32_t* smem, uint32_t* queue, uint32_t blk, uint32_t nblk) {
+  constexpr uint32_t ALL = 0xffffffffu;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const uint32_t gw = (blk * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t grp = lane >> 3, gl = lane & 7u;
   const uint32_t nw = (nblk * blockDim.x) >> 5;
   const uint32_t drawn = (*HFB_G(&segBuf[0]));
-  for (uint32_t ti = gw; ti < TB; ti += nw) {
-    const uint32_t n = (*HFB_G(&binCount[ti]));
-    if (n == 0) continue;
-    const uint32_t end = (*HFB_G(&blockSums[ti / SCAN_PER_BLOCK])) + (*HFB_G(&binOffset[ti]));  // bin end
-    if (!HFB_EXPECT(n <= end && end <= drawn)) continue;
-    finalizeBinWarp(ti, n, end - n, lane, keys, segBuf, tiles, largeBins, smem[warp]);
+  __shared__ uint32_t nQueue;
+  if (threadIdx.x == 0) nQueue = 0;
+  __syncthreads();
+  for (uint64_t base = (uint64_t)blk * (blockDim.x >> 5); base < TB; base += 32ull * nw) {  // uniform in the block
+    const uint64_t at = base + warp + (uint64_t)lane * nw;
+    const uint32_t ti = at < TB ? (uint32_t)at : 0u;
+    const uint32_t n = at < TB ? (*HFB_G(&binCount[ti])) : 0u;
+    const uint32_t end = n ? (*HFB_G(&blockSums[ti / SCAN_PER_BLOCK])) + (*HFB_G(&binOffset[ti])) : 0u;  // bin end
+    const bool ok = n != 0u && HFB_EXPECT(n <= end && end <= drawn);
+    const uint32_t start = end - n;
+    uint32_t few = __ballot_sync(ALL, ok && n <= 8u);
+    uint32_t mid = __ballot_sync(ALL, ok && n > 8u && n <= SMALL_BIN);
+    uint32_t big = __ballot_sync(ALL, ok && n > SMALL_BIN && n <= WARP_BIN);
+    if (ok && n > WARP_BIN) {
+      const uint32_t q = atomicAdd(&nQueue, 1u);  // below blockDim.x: one per lane of the block
+      queue[3u * q] = ti;
+      queue[3u * q + 1u] = n;
+      queue[3u * q + 2u] = start;
+    }
+    // the next four bins of at most 8 records: this lane's bin, count, start and key
+    uint32_t bT = 0, bN = 0, bS = 0, bV = ALL;
+    auto nextFew = [&]() {
+      uint32_t src = 0, have = 0;
+#pragma unroll
+      for (uint32_t g = 0; g < 4u; g++) {
+        if (grp == g && few) { src = __ffs(few) - 1u; have = 1u; }
+        few &= few - 1u;
+      }
+      bT = __shfl_sync(ALL, ti, src);
+      bN = __shfl_sync(ALL, n, src) * have;
+      bS = __shfl_sync(ALL, start, src);
+      bV = gl < bN ? (*HFB_G(&keys[bS + gl])) : ALL;
+    };
+    // the next bin of 9 .. 32 records
+    auto nextMid = [&]() {
+      const uint32_t src = (__ffs(mid) - 1u) & 31u;
+      bT = __shfl_sync(ALL, ti, src);
+      bN = mid ? __shfl_sync(ALL, n, src) : 0u;
+      bS = __shfl_sync(ALL, start, src);
+      bV = lane < bN ? (*HFB_G(&keys[bS + lane])) : ALL;
+      mid &= mid - 1u;
+    };
+    if (few) {
+      nextFew();
+      while (true) {
+        const bool more = few != 0u;
+        const uint32_t T0 = bT, N0 = bN, S0 = bS, V0 = bV;
+        if (more) nextFew();
+        const uint32_t v = sortGroup8(V0, gl, ALL);
+        if (gl < N0) writeList(segBuf, tiles, T0, S0, gl, N0, v);
+        if (!more) break;
+      }
+    }
+    if (mid) {
+      nextMid();
+      while (true) {
+        const bool more = mid != 0u;
+        const uint32_t T0 = bT, N0 = bN, S0 = bS, V0 = bV;
+        if (more) nextMid();
+        const uint32_t v = sortWarp32(V0, lane);
+        if (lane < N0) writeList(segBuf, tiles, T0, S0, lane, N0, v);
+        if (!more) break;
+      }
+    }
+    for (; big; big &= big - 1u) {
+      const uint32_t src = __ffs(big) - 1u;
+      finalizeBinWarp(__shfl_sync(ALL, ti, src), __shfl_sync(ALL, n, src), __shfl_sync(ALL, start, src), lane, keys,
+                      segBuf, tiles, smem + warp * WARP_BIN);
+    }
+    __syncthreads();
+    const uint32_t nq = nQueue;
+    for (uint32_t q = 0; q < nq; q++)
+      finalizeBinBlock(queue[3u * q], queue[3u * q + 1u], queue[3u * q + 2u], keys, segBuf, tiles, largeBins, smem);
+    __syncthreads();
+    if (threadIdx.x == 0) nQueue = 0;
+    __syncthreads();
   }
 }
 
@@ -720,14 +849,13 @@ __device__ __forceinline__ void binFinalizeBody(uint32_t TB, const uint32_t* __r
                                                 const uint32_t* __restrict__ binOffset,
                                                 const uint32_t* __restrict__ blockSums, uint32_t* __restrict__ keys,
                                                 uint32_t* __restrict__ segBuf, uint4* __restrict__ tiles,
-                                                uint32_t* __restrict__ largeBins, uint32_t (*smem)[MEDIUM_BIN],
+                                                uint32_t* __restrict__ largeBins, uint32_t* smem,
                                                 uint32_t blk, uint32_t nblk) {
   __shared__ uint32_t bigTi[32], bigN[32], bigEnd[32], nBig;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nWarps = blockDim.x >> 5;
   const uint32_t grp = lane >> 3, gl = lane & 7u;  // four groups of 8 lanes
   const uint32_t perBlock = nWarps * 4u;
   const uint32_t drawn = (*HFB_G(&segBuf[0]));
-  uint32_t* s = smem[warp];
   for (uint32_t bbase = blk * perBlock; bbase < TB; bbase += nblk * perBlock) {
     if (threadIdx.x == 0) nBig = 0;
     __syncthreads();
@@ -743,16 +871,7 @@ __device__ __forceinline__ void binFinalizeBody(uint32_t TB, const uint32_t* __r
     if (small) {
       const uint32_t start = endg - ng;
       uint32_t v = gl < ng ? (*HFB_G(&keys[start + gl])) : 0xffffffffu;
-      // bitonic sort across the group's 8 lanes, ascending
-#pragma unroll
-      for (uint32_t k = 2; k <= 8; k <<= 1) {
-#pragma unroll
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-          const uint32_t o = __shfl_xor_sync(smallLanes, v, j);
-          const bool asc = (gl & k) == 0, low = (gl & j) == 0;
-          v = (asc == low) ? min(v, o) : max(v, o);
-        }
-      }
+      v = sortGroup8(v, gl, smallLanes);
       if (gl < ng) writeList(segBuf, tiles, tg, start, gl, ng, v);
     } else if (ok && gl == 0u) {
       const uint32_t q = atomicAdd(&nBig, 1u);  // < 32: one per group of the block
@@ -763,7 +882,12 @@ __device__ __forceinline__ void binFinalizeBody(uint32_t TB, const uint32_t* __r
     __syncthreads();
     const uint32_t nb = nBig;
     for (uint32_t q = warp; q < nb; q += nWarps)
-      finalizeBinWarp(bigTi[q], bigN[q], bigEnd[q] - bigN[q], lane, keys, segBuf, tiles, largeBins, s);
+      if (bigN[q] <= WARP_BIN)
+        finalizeBinWarp(bigTi[q], bigN[q], bigEnd[q] - bigN[q], lane, keys, segBuf, tiles, smem + warp * WARP_BIN);
+    __syncthreads();
+    for (uint32_t q = 0; q < nb; q++)  // uniform in the block
+      if (bigN[q] > WARP_BIN)
+        finalizeBinBlock(bigTi[q], bigN[q], bigEnd[q] - bigN[q], keys, segBuf, tiles, largeBins, smem);
     __syncthreads();  // the queue is rewritten by the next 32 bins
   }
 }
@@ -772,8 +896,8 @@ __global__ void __launch_bounds__(256)
 binFinalizeKernel(uint32_t TB, const uint32_t* __restrict__ binCount, const uint32_t* __restrict__ binOffset,
                   const uint32_t* __restrict__ blockSums, uint32_t* __restrict__ keys,
                   uint32_t* __restrict__ segBuf, uint4* __restrict__ tiles, uint32_t* __restrict__ largeBins) {
-  __shared__ uint32_t smem[8][MEDIUM_BIN];
-  binFinalizeWarpBody(TB, binCount, binOffset, blockSums, keys, segBuf, tiles, largeBins, smem, blockIdx.x,
+  __shared__ uint32_t smem[8 * WARP_BIN], queue[3 * 256];
+  binFinalizeWarpBody(TB, binCount, binOffset, blockSums, keys, segBuf, tiles, largeBins, smem, queue, blockIdx.x,
                       gridDim.x);
 }
 
@@ -859,74 +983,79 @@ largeBinsKernel(const uint32_t* __restrict__ largeBins, const uint32_t* __restri
 // ---------------------------------------------------------------------------
 constexpr uint32_t SORT_MAX_BUCKETS = 256;
 
+constexpr uint32_t SORT_AHEAD = 8;  // tiles of one lane of the tile sort in flight
+
 struct SortShared {
-  uint32_t hist[SORT_MAX_BUCKETS], offs[SORT_MAX_BUCKETS], run[SORT_MAX_BUCKETS];
-  uint32_t wcnt[32][SORT_MAX_BUCKETS];
-  uint32_t drawn;
+  uint32_t wcnt[32][SORT_MAX_BUCKETS];  // a warp's tiles per bucket, then its next place in each
+  uint32_t warpSums[32];
 };
 
+// Warp w takes the w-th contiguous range of tiles, so its counts and its places
+// in every bucket are its own: the block meets three times, not four times per
+// 1024 tiles.  The pass is bound by the latency of one CTA: a lane has
+// SORT_AHEAD tiles on the way.  32,400 tiles: 45 -> 17 us, 8,160: 14 -> 8.4 us.
 __device__ __forceinline__ void tileSortBody(uint32_t T, uint32_t NB, uint32_t bucketSize,
                                              const uint32_t* __restrict__ segCount, uint32_t* __restrict__ buckets,
                                              uint32_t* __restrict__ tileList, SortShared& ss) {
-  uint32_t* hist = ss.hist;
-  uint32_t* offs = ss.offs;
-  uint32_t* run = ss.run;
-  uint32_t (*wcnt)[SORT_MAX_BUCKETS] = ss.wcnt;
-  uint32_t& drawn = ss.drawn;
-  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  for (uint32_t b = tid; b < NB; b += blockDim.x) { hist[b] = 0; run[b] = 0; }
-  if (tid == 0) drawn = 0;
-  __syncthreads();
-  // count-tiles: calcTileSortBucket, hairTileSortPass.countTiles.wgsl.ts:37-40
-  uint32_t local = 0;
-  for (uint32_t t = tid; t < T; t += blockDim.x) {
-    uint32_t c = (*HFB_G(&segCount[t]));
-    if (c > 0u) {
-      atomicAdd(&hist[clampu(c / bucketSize, 0u, NB - 1u)], 1u);
-      local++;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nWarps = blockDim.x >> 5;
+  uint32_t* cnt = ss.wcnt[warp];
+  for (uint32_t b = lane; b < NB; b += 32u) cnt[b] = 0;
+  __syncwarp();
+  const uint32_t perWarp = divCeil(divCeil(T, 32u), nWarps) * 32u;
+  const uint32_t t0 = min(warp * perWarp, T), t1 = min(t0 + perWarp, T);
+  // calcTileSortBucket, hairTileSortPass.countTiles.wgsl.ts:37-40; NB for an empty tile
+  auto load = [&](uint32_t tb, uint32_t* bucket) {
+    uint32_t c[SORT_AHEAD];
+#pragma unroll
+    for (uint32_t k = 0; k < SORT_AHEAD; k++) {
+      const uint32_t t = tb + k * 32u + lane;
+      c[k] = t < t1 ? (*HFB_G(&segCount[t])) : 0u;
     }
+#pragma unroll
+    for (uint32_t k = 0; k < SORT_AHEAD; k++) bucket[k] = c[k] ? clampu(c[k] / bucketSize, 0u, NB - 1u) : NB;
+  };
+  uint32_t bk[SORT_AHEAD];
+  for (uint32_t tb = t0; tb < t1; tb += 32u * SORT_AHEAD) {
+    load(tb, bk);
+#pragma unroll
+    for (uint32_t k = 0; k < SORT_AHEAD; k++)
+      if (bk[k] < NB) atomicAdd(&cnt[bk[k]], 1u);
   }
-  atomicAdd(&drawn, local);
   __syncthreads();
-  // calculateOffsetsForEachBucket: reverse exclusive scan, sort.wgsl.ts:68-75
-  if (tid == 0) {
-    uint32_t off = 0;
-    for (uint32_t i = 0; i < NB; i++) {
-      uint32_t idx = NB - 1u - i;
-      offs[idx] = off;
-      off += hist[idx];
+  // calculateOffsetsForEachBucket: reverse exclusive scan, sort.wgsl.ts:68-75; thread i
+  // takes bucket NB - 1 - i
+  const uint32_t b = NB - 1u - tid;  // for tid < NB
+  uint32_t sum = 0;
+  if (tid < NB)
+    for (uint32_t w = 0; w < nWarps; w++) sum += ss.wcnt[w][b];
+  uint32_t drawn;
+  uint32_t place = blockExclusiveScan(sum, ss.warpSums, drawn);
+  if (tid < NB) {
+    (*HFB_G(&buckets[2u * b])) = sum;
+    (*HFB_G(&buckets[2u * b + 1u])) = sum;  // the in-bucket write counter ends at tileCount
+    for (uint32_t w = 0; w < nWarps; w++) {
+      const uint32_t x = ss.wcnt[w][b];
+      ss.wcnt[w][b] = place;
+      place += x;
     }
-  }
-  for (uint32_t b = tid; b < NB; b += blockDim.x) {
-    (*HFB_G(&buckets[2u * b])) = hist[b];
-    (*HFB_G(&buckets[2u * b + 1u])) = hist[b];  // the in-bucket write counter ends at tileCount
   }
   if (tid == 0) (*HFB_G(&tileList[0])) = drawn;
   __syncthreads();
-  // stable scatter, one 1024-tile chunk at a time
-  for (uint32_t c0 = 0; c0 < T; c0 += blockDim.x) {
-    for (uint32_t i = tid; i < 32u * NB; i += blockDim.x) wcnt[i / NB][i % NB] = 0;
-    __syncthreads();
-    uint32_t t = c0 + tid;
-    uint32_t c = t < T ? (*HFB_G(&segCount[t])) : 0u;
-    bool valid = c > 0u;
-    uint32_t b = valid ? clampu(c / bucketSize, 0u, NB - 1u) : SORT_MAX_BUCKETS;
-    uint32_t peers = __match_any_sync(0xffffffffu, b);
-    uint32_t rank = __popc(peers & ((1u << lane) - 1u));
-    if (valid && rank == 0) wcnt[warp][b] = __popc(peers);
-    __syncthreads();
-    for (uint32_t bb = tid; bb < NB; bb += blockDim.x) {
-      uint32_t s = run[bb];
-      for (uint32_t w = 0; w < 32; w++) {
-        uint32_t x = wcnt[w][bb];
-        wcnt[w][bb] = s;
-        s += x;
-      }
-      run[bb] = s;
+  // the scatter, stable: a warp's tiles in order, the warps' ranges in order
+  for (uint32_t tb = t0; tb < t1; tb += 32u * SORT_AHEAD) {
+    load(tb, bk);
+#pragma unroll
+    for (uint32_t k = 0; k < SORT_AHEAD; k++) {
+      const uint32_t mine = bk[k];
+      if (!__any_sync(0xffffffffu, mine < NB)) continue;
+      const uint32_t peers = __match_any_sync(0xffffffffu, mine);
+      const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
+      const uint32_t at = mine < NB ? cnt[mine] + rank : T;
+      if (mine < NB && HFB_EXPECT(at < T)) (*HFB_G(&tileList[1u + at])) = tb + k * 32u + lane;
+      __syncwarp();
+      if (mine < NB && rank == 0u) cnt[mine] = at + __popc(peers);
+      __syncwarp();
     }
-    __syncthreads();
-    if (valid && HFB_EXPECT(offs[b] + wcnt[warp][b] + rank < T)) (*HFB_G(&tileList[1u + offs[b] + wcnt[warp][b] + rank])) = t;
-    __syncthreads();
   }
 }
 
@@ -1985,12 +2114,17 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
   return FINE_OK;
 }
 
+constexpr uint32_t SCHED_AHEAD = 4;  // tile-list entries of one thread of the schedule in flight
+constexpr uint32_t SCHED_HEADS = 8;  // list heads of one tile in flight
+
 // Builds the work list of the fine pass: one item per drawn tile, in the
 // tile list's order (most records first), except that a tile with more
 // records than a CTA's average share is split into groups of whole depth
 // bins, so that no single CTA carries the frame's tail.  Group sizes come
 // from the list-length hints; a tile without valid hints is not split.
-// One CTA.
+// One CTA, bound by the latency of its loads: the heads of a tile are read once,
+// SCHED_HEADS at a time, and 1024 entries without a split need no scan.  A frame of
+// 32,400 tiles: 26 -> 15 us.
 __device__ __forceinline__ void fineScheduleBody(const uint32_t* __restrict__ tileList,
                                                  const uint32_t* __restrict__ segCount,
                                                  const uint4* __restrict__ tiles, uint32_t T, uint32_t B,
@@ -2003,36 +2137,62 @@ __device__ __forceinline__ void fineScheduleBody(const uint32_t* __restrict__ ti
   if (tid == 0) total = 0;
   __syncthreads();
   uint32_t mine = 0;
-  for (uint32_t q = tid; q < drawn; q += blockDim.x) {
-    const uint32_t t = (*HFB_G(&tileList[1u + q]));
-    if (t < T) mine += (*HFB_G(&segCount[t]));
+  for (uint32_t q0 = tid; q0 < drawn; q0 += SCHED_AHEAD * blockDim.x) {
+    uint32_t t[SCHED_AHEAD];
+#pragma unroll
+    for (uint32_t k = 0; k < SCHED_AHEAD; k++) {
+      const uint32_t q = q0 + k * blockDim.x;
+      t[k] = q < drawn ? (*HFB_G(&tileList[1u + q])) : T;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < SCHED_AHEAD; k++)
+      if (t[k] < T) mine += (*HFB_G(&segCount[t[k]]));
   }
-  atomicAdd(&total, mine);
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if ((tid & 31u) == 0u) atomicAdd(&total, mine);
   __syncthreads();
   const uint32_t thr = max(FINE_SPLIT_MIN, total / max(grid, 1u));
   uint32_t carryItems = 0, carrySlots = 0;
+  uint32_t tNext = tid < drawn ? (*HFB_G(&tileList[1u + tid])) : T;
+  uint32_t cNext = tNext < T ? (*HFB_G(&segCount[tNext])) : 0u;
   for (uint32_t q0 = 0; q0 < drawn; q0 += blockDim.x) {
     const uint32_t q = q0 + tid;
-    uint32_t nG = 0, t = T;  // items of this tile-list entry: none past the list's end
-    if (q < drawn) {
-      nG = 1;
-      t = (*HFB_G(&tileList[1u + q]));
-      if (allowSplit && t < T && (*HFB_G(&segCount[t])) > thr) {  // count the groups of the split
-        uint32_t g = 0, acc = 0;
-        bool ok = true;
-        for (uint32_t b = 0; b < B; b++) {
-          const uint4 h = (*HFB_G(&tiles[(size_t)t * B + b]));
+    const uint32_t t = tNext, c = cNext;  // T, 0 past the list's end
+    tNext = q + blockDim.x < drawn ? (*HFB_G(&tileList[1u + q + blockDim.x])) : T;
+    cNext = tNext < T ? (*HFB_G(&segCount[tNext])) : 0u;
+    uint32_t nG = q < drawn ? 1u : 0u;  // items of this tile-list entry: none past the list's end
+    uint64_t starts = 0;                // bins that start a group but the first
+    if (allowSplit && t < T && c > thr) {  // the groups of the split
+      uint32_t g = 0, acc = 0;
+      bool ok = true;
+      for (uint32_t b0 = 0; b0 < B; b0 += SCHED_HEADS) {
+        uint4 h[SCHED_HEADS];
+#pragma unroll
+        for (uint32_t k = 0; k < SCHED_HEADS; k++)
+          h[k] = b0 + k < B ? (*HFB_G(&tiles[(size_t)t * B + b0 + k])) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (uint32_t k = 0; k < SCHED_HEADS; k++) {
           uint32_t nb = 0;
-          if (h.y != 0u && h.z != 0u) {
-            if (h.w != 0u && h.w <= h.z && h.z <= maxDrawn && h.w <= maxProcessed) nb = h.w; else ok = false;
+          if (h[k].y != 0u && h[k].z != 0u) {
+            if (h[k].w != 0u && h[k].w <= h[k].z && h[k].z <= maxDrawn && h[k].w <= maxProcessed) nb = h[k].w;
+            else ok = false;
           }
           if (nb == 0u) continue;
-          if (acc > 0u && acc + nb > thr) { g++; acc = 0; }
+          if (acc > 0u && acc + nb > thr) {
+            g++;
+            acc = 0;
+            starts |= 1ull << (b0 + k);
+          }
           acc += nb;
         }
-        if (acc > 0u) g++;
-        if (ok && g > 1u) nG = g;
       }
+      if (acc > 0u) g++;
+      if (ok && g > 1u) nG = g;
+    }
+    if (!__syncthreads_or(nG > 1u)) {  // the usual case past the list's front: one item per tile
+      if (q < drawn) (*HFB_G(&fs.items[carryItems + tid])) = make_uint4(q, 0u | (B << 8) | (1u << 24), 0u, 0u);
+      carryItems += min(drawn - q0, blockDim.x);
+      continue;
     }
     uint32_t chunkSlots;
     const uint32_t mySlots = nG > 1u ? nG : 0u;
@@ -2041,28 +2201,19 @@ __device__ __forceinline__ void fineScheduleBody(const uint32_t* __restrict__ ti
     if (nG > 1u && !split) nG = 1;
     uint32_t chunkItems;
     const uint32_t itemBase = carryItems + blockExclusiveScan(nG, warpSums, chunkItems);
-    if (q < drawn) {
-      if (split) {
-        const uint32_t slot = slotEnd - nG;
-        (*HFB_G(&fs.arrivals[slot])) = 0;
-        atomicAdd(HFB_G(&counters->fineSplitTiles), 1ull);
-        uint32_t g = 0, acc = 0, start = 0;
-        for (uint32_t b = 0; b < B; b++) {
-          const uint4 h = (*HFB_G(&tiles[(size_t)t * B + b]));
-          const uint32_t nb = (h.y != 0u && h.z != 0u) ? h.w : 0u;
-          if (nb == 0u) continue;
-          if (acc > 0u && acc + nb > thr) {
-            (*HFB_G(&fs.items[itemBase + g])) = make_uint4(q, start | (b << 8) | (g << 16) | (nG << 24), slot, 0u);
-            g++;
-            acc = 0;
-            start = b;
-          }
-          acc += nb;
-        }
-        (*HFB_G(&fs.items[itemBase + g])) = make_uint4(q, start | (B << 8) | (g << 16) | (nG << 24), slot, 0u);
-      } else {
-        (*HFB_G(&fs.items[itemBase])) = make_uint4(q, 0u | (B << 8) | (1u << 24), 0u, 0u);
+    if (split) {
+      const uint32_t slot = slotEnd - nG;
+      (*HFB_G(&fs.arrivals[slot])) = 0;
+      atomicAdd(HFB_G(&counters->fineSplitTiles), 1ull);
+      uint32_t start = 0;
+      for (uint32_t g = 0; g < nG; g++) {
+        const uint32_t end = starts ? (uint32_t)__ffsll((long long)starts) - 1u : B;
+        starts &= starts - 1ull;
+        (*HFB_G(&fs.items[itemBase + g])) = make_uint4(q, start | (end << 8) | (g << 16) | (nG << 24), slot, 0u);
+        start = end;
       }
+    } else if (nG) {
+      (*HFB_G(&fs.items[itemBase])) = make_uint4(q, 0u | (B << 8) | (1u << 24), 0u, 0u);
     }
     carryItems += chunkItems;
     carrySlots += chunkSlots;
@@ -2351,7 +2502,7 @@ __global__ void __launch_bounds__(256) binScatterBatch(BatchView b, HfbConfig cf
 
 __global__ void __launch_bounds__(256) binFinalizeBatch(BatchView b, HfbConfig cfgParam) {
   const HfbConfig cfg = cfgParam;
-  __shared__ uint32_t smem[8][MEDIUM_BIN];
+  __shared__ uint32_t smem[8 * WARP_BIN];
   BATCH_LOOP(BK_FINALIZE)
     binFinalizeBody(I.T * cfg.tileDepthBins, ts.binCount, ts.binOffset, ts.blockSums, ts.keys, I.segBuf, I.tiles,
                     ts.largeBins, smem, local, nLocal);
@@ -2482,10 +2633,10 @@ cudaError_t launchTilesPass(HfbCtx* c, const HfbUniforms& u, const HfbHairData& 
   HFB_AFTER_LAUNCH(c, "binScanBlocks");
   binScanSums<<<1, 1024, 0, c->stream>>>(s.blockSums, nBlocks);
   HFB_AFTER_LAUNCH(c, "binScanSums");
-  binScatterKernel<<<c->smCount * 4, 256, 0, c->stream>>>(rb.tileSegments, rb.maxDrawnSegments, s.binOffset,
+  binScatterKernel<<<c->smCount * 8, 256, 0, c->stream>>>(rb.tileSegments, rb.maxDrawnSegments, s.binOffset,
                                                           s.blockSums, s.keys, dc, TB);
   HFB_AFTER_LAUNCH(c, "binScatterKernel");
-  binFinalizeKernel<<<min(divCeil(TB, 8), (uint32_t)c->smCount * 16), 256, 0, c->stream>>>(
+  binFinalizeKernel<<<min(divCeil(TB, 8), (uint32_t)c->smCount * 7), 256, 0, c->stream>>>(
       TB, s.binCount, s.binOffset, s.blockSums, s.keys, rb.tileSegments, (uint4*)rb.tiles, s.largeBins);
   HFB_AFTER_LAUNCH(c, "binFinalizeKernel");
   if (!c->largeBinsAttrSet) {
@@ -2493,7 +2644,8 @@ cudaError_t launchTilesPass(HfbCtx* c, const HfbUniforms& u, const HfbHairData& 
     if (e != cudaSuccess) return e;
     c->largeBinsAttrSet = true;
   }
-  largeBinsKernel<<<c->smCount, 1024, LARGE_SMEM_KEYS * 4, c->stream>>>(
+  // two CTAs of 64 KB per SM: 758 bins of up to 34,187 records 475 -> 400 us
+  largeBinsKernel<<<c->smCount * 2, 1024, LARGE_SMEM_KEYS * 4, c->stream>>>(
       s.largeBins, s.binCount, s.binOffset, s.blockSums, s.keys, rb.tileSegments, (uint4*)rb.tiles);
   HFB_AFTER_LAUNCH(c, "largeBinsKernel");
   c->launches += nSeg ? 6 : 5;
