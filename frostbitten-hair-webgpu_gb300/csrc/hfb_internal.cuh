@@ -97,7 +97,7 @@ struct TilesScratch {
 struct FineScratch {
   uint32_t* hdr;       // [0] = work items
   uint4* items;        // tile list index, b0 | b1 << 8 | group << 16 | groups << 24, first group slot
-  uint32_t* arrivals;  // per split tile (at its first group slot): groups done | 1 << 31 if one gave up
+  uint32_t* arrivals;  // per split tile (at its first group slot): see FINE_FIRST in raster.cu
   float4* groups;      // per group slot: the TS*TS composites of the group's depth bins
   uint32_t maxItems, maxGroups;
   size_t bytes;

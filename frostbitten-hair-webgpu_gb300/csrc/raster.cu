@@ -1092,7 +1092,7 @@ tileSortKernel(uint32_t T, uint32_t NB, uint32_t bucketSize, const uint32_t* __r
 // box pixel, with rounds cut at PAIRS box pixels: 150 -> 109 us (10,000 x 32 at
 // 1920x1080, 16 px tiles), 222 -> 154 us (11,400 x 16, 8 px tiles, 8 slices), 320 ->
 // 176 us (7,001 x 23 at 1361x767, 32 px), 7.2 -> 4.2 ms (200,000 x 32 at 4K).  Each slice of a pixel keeps the closed form of
-// its front-to-back blend in registers: fragments arrive back to front
+// its front-to-back blend (FineSlices): fragments arrive back to front
 // (descending key) and acc = f + (1 - f.a) * acc, which equals the
 // reference's per-slice linked list reduced front to back
 // (reduceHairSlices.wgsl.ts:9-73) -- no fragment pool in memory.
@@ -1170,6 +1170,7 @@ struct FineSmem {
   float4 shade[STAGE][NSHADE];   // the shading entries each staged segment can sample
   uint2 frag[PAIRS];             // A1: pixel | segment << 16 of a listed pixel; A2: its fragment's colour as 4 x f16
   float4 spanLo[STAGE], spanHi[STAGE];  // SpanLines in tile pixels
+  float4 liveBox;                // box of the tile's pixels that are not done (x0, y0, x1, y1)
   uint8_t slice[PAIRS];          // A2: the fragment's slice
   FineRow<TS> row[ROWS];         // the box rows of the staged segments, segment after segment
   // staged segments, one array per quantity (consecutive segments in consecutive banks)
@@ -1211,6 +1212,7 @@ struct FineSmem {
   FineArgs args;
   uint32_t nRuns, nStaged, nSeg, passCount, segLimit, edgePasses, queueIdx, bad, tileMode, total, walkNext;
   uint32_t mode, cutSeg, cutSlots, roundFrags, e0, eLast, arrive;
+  uint32_t filled;                   // bins that filled their pool
 };
 
 // Block-wide sum (all threads call; every thread gets the total).
@@ -1255,14 +1257,35 @@ __device__ __forceinline__ uint32_t stageShade(FineSmem<TS>& sh, uint32_t k, uin
   remapToIndices(SP, fadd((float)sg, 1.0f) / (float)(P - 1u), b0, b1);
   const uint32_t ne = min(b1 - a0 + 1u, FineSmem<TS>::NSHADE);
   const size_t sb = (size_t)st * SP;
-  for (uint32_t j = 0; j < ne; j++) sh.shade[k][j] = __ldg(HFB_G(&shading[sb + a0 + j]));
+  float4 v[FineSmem<TS>::NSHADE];
+#pragma unroll
+  for (uint32_t j = 0; j < FineSmem<TS>::NSHADE; j++)  // all in flight together
+    v[j] = j < ne ? __ldg(HFB_G(&shading[sb + a0 + j])) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+  for (uint32_t j = 0; j < FineSmem<TS>::NSHADE; j++)
+    if (j < ne) sh.shade[k][j] = v[j];
   return a0 | (ne << 16);
+}
+
+// Bounding box of the tile's pixels that are not done (x0, y0, x1, y1; the whole tile
+// where none is left), by one warp.  Once most of a tile is opaque, the
+// long lists behind it touch the few open pixels only: the rounds of a tile that carries
+// on in order take 10.9 -> 9.5 us (200,000 x 32 at 4K); elsewhere it gives less than the
+// 0.3 % that it costs.
+template <int TS>
+__device__ __forceinline__ float4 liveBoxOf(const FineSmem<TS>& sh, uint32_t lane) {
+  constexpr uint32_t PER = 32u / TS;  // tile rows in a word of the mask
+  constexpr uint32_t ROW = TS == 32 ? 0xffffffffu : (1u << (TS & 31)) - 1u;
+  const uint32_t m = lane < TS ? ~(sh.doneMask[lane / PER] >> ((lane % PER) * TS)) & ROW : 0u;  // lane's row
+  const uint32_t ys = __ballot_sync(0xffffffffu, m != 0u), xs = __reduce_or_sync(0xffffffffu, m);
+  if (ys == 0u) return make_float4(0.0f, 0.0f, (float)(TS - 1), (float)(TS - 1));
+  return make_float4((float)(__ffs(xs) - 1), (float)(__ffs(ys) - 1), (float)(31 - __clz(xs)), (float)(31 - __clz(ys)));
 }
 
 // Staged segment k from its projection s: edge-test constants, depths, the
 // pixel-independent part of interpolateHairQuad, and the tile-local box of
 // the pixels that can pass the edge tests ([floor(min), ceil(max)] of the
-// vertices).  shade: first | count << 16 of its staged shading entries
+// vertices), within the tile's live box (liveBoxOf).  shade: first | count << 16 of its staged shading entries
 // (stageShade).  Returns the box height (0: no pixel).
 template <int TS>
 __device__ __forceinline__ uint32_t stageFromProjection(FineSmem<TS>& sh, uint32_t k, uint32_t bin, const ProjSeg& s,
@@ -1272,9 +1295,10 @@ __device__ __forceinline__ uint32_t stageFromProjection(FineSmem<TS>& sh, uint32
   float mny = floorf(fminf(fminf(s.v00.y, s.v01.y), fminf(s.v10.y, s.v11.y))) - (float)y0;
   float mxx = ceilf(fmaxf(fmaxf(s.v00.x, s.v01.x), fmaxf(s.v10.x, s.v11.x))) - (float)x0;
   float mxy = ceilf(fmaxf(fmaxf(s.v00.y, s.v01.y), fmaxf(s.v10.y, s.v11.y))) - (float)y0;
-  if (mnx <= mxx && mny <= mxy && mxx >= 0.0f && mxy >= 0.0f && mnx <= (float)(TS - 1) && mny <= (float)(TS - 1)) {
-    const uint32_t bx0 = (uint32_t)fmaxf(mnx, 0.0f), by0 = (uint32_t)fmaxf(mny, 0.0f);
-    const uint32_t bx1 = (uint32_t)fminf(mxx, (float)(TS - 1)), by1 = (uint32_t)fminf(mxy, (float)(TS - 1));
+  const float4 lb = sh.liveBox;
+  if (mnx <= mxx && mny <= mxy && mxx >= lb.x && mxy >= lb.y && mnx <= lb.z && mny <= lb.w) {
+    const uint32_t bx0 = (uint32_t)fmaxf(mnx, lb.x), by0 = (uint32_t)fmaxf(mny, lb.y);
+    const uint32_t bx1 = (uint32_t)fminf(mxx, lb.z), by1 = (uint32_t)fminf(mxy, lb.w);
     box = bx0 | (by0 << 8) | (bx1 << 16) | (by1 << 24);
     rows = by1 - by0 + 1u;
     // edge tests in the order insideQuad evaluates them
@@ -1439,22 +1463,84 @@ __device__ __forceinline__ uint2 fragmentColour(const FineSmem<TS>& sh, uint32_t
 __device__ __forceinline__ float halfLo(uint32_t v) { return __half2float(__ushort_as_half((unsigned short)(v & 0xffffu))); }
 __device__ __forceinline__ float halfHi(uint32_t v) { return __half2float(__ushort_as_half((unsigned short)(v >> 16))); }
 
-// acc[slice] = f + (1 - f.a) * acc[slice], the colours with one rounding; alpha, which decides
-// when a pixel is done, with the two of the reference's product and sum
-template <int MAXL>
-__device__ __forceinline__ void blendFragment(f4 (&acc)[MAXL], uint32_t sl, uint2 h) {
-  const f4 q = mk4(halfLo(h.x), halfHi(h.x), halfLo(h.y), halfHi(h.y));
-  const float kk = fsub(1.0f, q.w);
-#pragma unroll
-  for (int si = 0; si < MAXL; si++) {
-    if ((uint32_t)si == sl) {
-      acc[si].x = __fmaf_rn(kk, acc[si].x, q.x);
-      acc[si].y = __fmaf_rn(kk, acc[si].y, q.y);
-      acc[si].z = __fmaf_rn(kk, acc[si].z, q.z);
-      acc[si].w = fadd(q.w, fmul(kk, acc[si].w));
-    }
+// A pixel's slices of the bin at the cursor.  In shared memory, a float4 of every
+// pixel per slice, where the CTAs that the registers allow leave room for it: a
+// fragment then costs one load and one store, not a predicated blend of every slice,
+// and `touched` names the slices that hold anything: 153 -> 131 us on a frame of 11,400
+// x 32 at 1920x1080 (8 px tiles, 8 slices).  Else in registers: 8 px tiles with 4 slices
+// would lose one of 8 CTAs per SM, 16 px ones one of 3 (4 slices) or of 2 (16 slices),
+// and 32 px tiles have no room.
+template <int TS, int MAXL>
+constexpr bool FINE_SHARED_SLICES = (TS == 8 && MAXL >= 8) || (TS == 16 && MAXL == 8);
+template <int TS, int MAXL>
+constexpr size_t FINE_SMEM = sizeof(FineSmem<TS>) + (FINE_SHARED_SLICES<TS, MAXL> ? MAXL * TS * TS * sizeof(float4) : 0);
+
+// q + kk * acc with kk = 1 - q.a, the colours with one rounding; alpha, which decides when a pixel is
+// done, with the two of the reference's product and sum
+__device__ __forceinline__ void blendOver(f4& acc, const f4 q, float kk) {
+  acc.x = __fmaf_rn(kk, acc.x, q.x);
+  acc.y = __fmaf_rn(kk, acc.y, q.y);
+  acc.z = __fmaf_rn(kk, acc.z, q.z);
+  acc.w = fadd(q.w, fmul(kk, acc.w));
+}
+__device__ __forceinline__ f4 halfColour(uint2 h) { return mk4(halfLo(h.x), halfHi(h.x), halfLo(h.y), halfHi(h.y)); }
+// the slice under what is there, until the pixel is done (reduceHairSlices.wgsl.ts:9-73)
+__device__ __forceinline__ void sliceUnder(f4& fin, const f4 acc) {
+  if (fin.w < 0.999f) {
+    const float kk = fsub(1.0f, fin.w);
+    fin.x = fadd(fin.x, fmul(acc.x, kk));
+    fin.y = fadd(fin.y, fmul(acc.y, kk));
+    fin.z = fadd(fin.z, fmul(acc.z, kk));
+    fin.w = fadd(fin.w, fmul(acc.w, kk));
   }
 }
+
+template <int TS, int MAXL, bool SHARED = FINE_SHARED_SLICES<TS, MAXL>>
+struct FineSlices;
+template <int TS, int MAXL>
+struct FineSlices<TS, MAXL, true> {
+  float4* at;  // this pixel's first slice; the next TS * TS on
+  uint32_t touched = 0;
+  __device__ __forceinline__ explicit FineSlices(FineSmem<TS>& sh)
+      : at(reinterpret_cast<float4*>(&sh + 1) + threadIdx.x) {}
+  __device__ __forceinline__ void blend(uint32_t sl, uint2 h) {
+    if (!HFB_EXPECT(sl < (uint32_t)MAXL)) return;
+    f4 acc = mk4(0.0f, 0.0f, 0.0f, 0.0f);
+    if ((touched >> sl) & 1u) acc = ld4(at[sl * TS * TS]);
+    touched |= 1u << sl;
+    const f4 q = halfColour(h);
+    blendOver(acc, q, fsub(1.0f, q.w));
+    at[sl * TS * TS] = make_float4(acc.x, acc.y, acc.z, acc.w);
+  }
+  __device__ __forceinline__ void reduce(f4& fin, uint32_t L) {
+    for (uint32_t m = touched; m; m &= m - 1u) {  // an empty slice adds nothing
+      const uint32_t si = (uint32_t)__ffs(m) - 1u;
+      if (si < L) sliceUnder(fin, ld4(at[si * TS * TS]));
+    }
+  }
+  __device__ __forceinline__ void clear() { touched = 0; }
+};
+template <int TS, int MAXL>
+struct FineSlices<TS, MAXL, false> {
+  f4 acc[MAXL];
+  __device__ __forceinline__ explicit FineSlices(FineSmem<TS>&) { clear(); }
+  __device__ __forceinline__ void blend(uint32_t sl, uint2 h) {
+    const f4 q = halfColour(h);  // converted once, not once per slice
+    const float kk = fsub(1.0f, q.w);
+#pragma unroll
+    for (int si = 0; si < MAXL; si++)
+      if ((uint32_t)si == sl) blendOver(acc[si], q, kk);
+  }
+  __device__ __forceinline__ void reduce(f4& fin, uint32_t L) {
+#pragma unroll
+    for (int si = 0; si < MAXL; si++)
+      if ((uint32_t)si < L) sliceUnder(fin, acc[si]);
+  }
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int si = 0; si < MAXL; si++) acc[si] = mk4(0.0f, 0.0f, 0.0f, 0.0f);
+  }
+};
 
 // Tile mode: the runs of the next round, from bin `bin`, entry `off` of its
 // list, up to `cap` segments.  Bins without depth (td1 == 0) are skipped as
@@ -1506,7 +1592,8 @@ __device__ __forceinline__ uint32_t buildRuns(FineSmem<TS>& sh, uint32_t b1, uin
 // Rasterizes depth bins [b0, b1) of tile tileIdx in order, every pixel
 // starting from an empty colour (processTile per bin + reduceHairSlices,
 // hairFinePass.wgsl.ts:205-288), and leaves each pixel's colour in fin.
-// With `part` IN_ORDER the bins start the tile.  Otherwise they are a later part
+// With `part` IN_ORDER the bins start the tile, or carry on from the colours at
+// `resume` that the tile's earlier bins left.  Otherwise they are a later part
 // of a split tile: every pixel in view takes part, and the call gives up
 // (FINE_UNSAFE) where a bin could fill its fragment pool, whose cut would depend
 // on which pixels the earlier bins finished.  Where it gives up decides whether
@@ -1514,14 +1601,21 @@ __device__ __forceinline__ uint32_t buildRuns(FineSmem<TS>& sh, uint32_t b1, uin
 // (up to the 0.001 that a finished pixel still lacks), so the decision must not
 // depend on how tight the listed pixels are: CAREFUL takes rounds of at most
 // PAIRS box pixels and counts what the edge tests accept, and its running bound
-// exceeds a bin's own count by less than PAIRS.  QUICK takes full rounds and
-// counts listed pixels; while a bin's count stays PAIRS below the pool, CAREFUL
-// would not give up either; past that it returns FINE_AGAIN, for CAREFUL to decide.
+// exceeds a bin's own count by less than PAIRS.  QUICK takes full rounds and bounds
+// a bin's count from both sides: the accepted pixels of the rounds that are all the
+// bin's, with and without the listed pixels of the others.  Where the lower bound
+// exceeds the pool CAREFUL gives up as well, where the upper one stays PAIRS below
+// it CAREFUL goes on as well; a bin that ends in between is FINE_AGAIN, for CAREFUL
+// to decide.
 enum FinePart : uint32_t { FINE_IN_ORDER = 0, FINE_QUICK, FINE_CAREFUL };
+// Bits of a split tile's word: parts that arrived; bins of the first part that filled their
+// pool; the first part's colours are there; a later part gave up.
+constexpr uint32_t FINE_FILLED_SHIFT = 16, FINE_FILLED = 0x7fu << FINE_FILLED_SHIFT, FINE_FIRST = 1u << 30, FINE_REDO = 1u << 31;
 enum FineEnd : uint32_t { FINE_OK = 0, FINE_UNSAFE, FINE_AGAIN };
 template <int TS, int MAXL>
 __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms& U, const FineArgs& a,
-                                         uint32_t tileIdx, uint32_t b0, uint32_t b1, FinePart part, f4& fin) {
+                                         uint32_t tileIdx, uint32_t b0, uint32_t b1, FinePart part,
+                                         const float4* resume, f4& fin) {
   using SM = FineSmem<TS>;
   constexpr uint32_t NT = SM::NT, STAGE = SM::STAGE, PAIRS = SM::PAIRS, ROWS = SM::ROWS, NW = NT / 32u;
   constexpr uint32_t MODE_FAST = 0, MODE_TIGHTEN = 1, MODE_ABORT = 2;
@@ -1542,11 +1636,21 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
   const bool inView = px < W && py < H;
   sh.zbuf[tid] = inView ? loadTex2DClamp(a.depth, W, H, f2i((float)px), f2i(fsub(size.y, (float)py))) : 0.0f;
   bool done = !inView;
+  fin = mk4(0.f, 0.f, 0.f, 0.f);  // rasterizerResult was cleared before the pass
+  if (resume) {
+    const float4 f = __ldcg(HFB_G(&resume[tid]));
+    fin = mk4(f.x, f.y, f.z, f.w);
+    done = done || fin.w >= 0.999f;
+    if (__syncthreads_and(done)) return FINE_OK;
+  }
+  if (tid == 0) {
+    sh.filled = 0;
+    sh.liveBox = make_float4(0.0f, 0.0f, (float)(TS - 1), (float)(TS - 1));
+  }
   {
     const uint32_t dm = __ballot_sync(0xffffffffu, done);
     if (lane == 0) sh.doneMask[warp] = dm;
   }
-  fin = mk4(0.f, 0.f, 0.f, 0.f);  // rasterizerResult was cleared before the pass
   if (tid < a.B) {
     const uint4 h = (*HFB_G(&a.tiles[ty * tilesX * a.B + tx * a.B + tid]));
     sh.head[tid] = h;
@@ -1611,9 +1715,7 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
   }
 
   // per-pixel state of the current bin
-  f4 acc[MAXL];
-#pragma unroll
-  for (int si = 0; si < MAXL; si++) acc[si] = mk4(0.f, 0.f, 0.f, 0.f);
+  FineSlices<TS, MAXL> slices(sh);
   uint32_t nFrag = 0, pending = 0;
   // uniform state: cursor and the pool accounting of the bin at the cursor
   uint32_t bin = b0, off = 0;                    // tile mode: bin, entry of its list
@@ -1623,6 +1725,10 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
   while (true) {
     // ---------------- stage the round: a thread per segment ----------------
     uint32_t myBin = 0, myEnc = 0xffffffffu;
+    if (resume && warp == 1) {
+      const float4 lb = liveBoxOf<TS>(sh, lane);
+      if (lane == 0) sh.liveBox = lb;
+    }
     if (tileMode) {
       if (warp == 0) {
         const uint32_t used = buildRuns<TS>(sh, b1, bin, off, STAGE, lane);
@@ -1870,9 +1976,10 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
     // fill its pool and nothing needs counting (the common case: every thread
     // sees passCount after the barrier above).  Otherwise one warp sums the
     // listed pixels run by run.  e0 / eLast carry the bounds of the first and
-    // last run (the round's total where it is enough).  A CAREFUL part checks
-    // after A2, which counts what the edge tests accept.
-    const uint32_t cap = part == FINE_QUICK ? (a.CAP > PAIRS ? a.CAP - PAIRS : 0u) : a.CAP;
+    // last run (the round's total where it is enough).  A CAREFUL part, and a QUICK
+    // one inside a bin, check after A2, which counts what the edge tests accept.
+    const uint32_t cap = a.CAP;
+    const uint32_t sure = cap > PAIRS ? cap - PAIRS : 0u;  // CAREFUL goes on where QUICK's bound is at most this
     uint32_t mode = MODE_FAST, e0 = sh.passCount, eLast = e0;
     auto sumRuns = [&]() {  // by run, with the warp 0; all threads call
       if (warp == 0) {
@@ -1888,7 +1995,7 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
           e = __reduce_add_sync(0xffffffffu, e);
           const uint32_t base = r == 0u ? runningUB : 0u;
           if (r == 0u) we0 = e;
-          if (base + e > cap) {
+          if (base + e > (part == FINE_QUICK ? sure : cap)) {
             if (r == 0u) { wmode = MODE_TIGHTEN; keep = 1; } else { keep = r; }
             break;
           }
@@ -1913,7 +2020,8 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
       nRuns = sh.nRuns;
       nSeg = sh.nSeg;
     };
-    if (part != FINE_CAREFUL && runningUB + e0 > cap) {
+    // (QUICK: the bin at the cursor ends, others begin)
+    if (part == FINE_IN_ORDER ? runningUB + e0 > cap : part == FINE_QUICK && nRuns > 1u && runningUB + e0 > sure) {
       sumRuns();
       if (mode == MODE_ABORT) return FINE_AGAIN;
     }
@@ -1945,10 +2053,8 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
         for (int j = 0; j < 4; j++)  // edgeFunction >= 0
           inside = inside && fsub(fmul(fsub(pf.x, sh.ox[j][k]), sh.ey[j][k]), fmul(fsub(pf.y, sh.oy[j][k]), sh.ex[j][k])) >= 0.0f;
         if (!inside) continue;
-        if (part == FINE_CAREFUL) {
-          accepted++;
-          atomicAdd(&sh.cnt[k], 1u);
-        }
+        accepted++;
+        if (part == FINE_CAREFUL) atomicAdd(&sh.cnt[k], 1u);
         QuadConst qc;
         qc.sm = mk2(sh.qsx[k], sh.qsy[k]);
         qc.ab = mk2(sh.qax[k], sh.qay[k]);
@@ -1966,9 +2072,18 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
         atomicOr(&sh.pixMask[k >> 5][pix], 1u << (k & 31u));
         if (exact) atomicAdd(&sh.cnt[k], 1u);
       }
-      if (accepted) atomicAdd(&sh.edgePasses, accepted);
+      if (part == FINE_CAREFUL || (part == FINE_QUICK && nRuns == 1u)) {
+        accepted = __reduce_add_sync(0xffffffffu, accepted);
+        if (lane == 0 && accepted) atomicAdd(&sh.edgePasses, accepted);
+      }
     }
     __syncthreads();
+    if (part == FINE_QUICK && nRuns == 1u) {  // all the cursor's bin: running and runningUB are its bounds
+      e0 = sh.edgePasses;
+      running += e0;
+      if (running > a.CAP) return FINE_UNSAFE;
+      if ((sh.runBin[0] & RUN_ENDS) && runningUB + e0 > sure) return FINE_AGAIN;
+    }
     if (part == FINE_CAREFUL) {
       e0 = eLast = sh.edgePasses;
       if (runningUB + e0 > cap) {
@@ -2007,6 +2122,7 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
             sh.nSeg = cut + 1u;
             sh.runK1[0] = (uint16_t)(cut + 1u);
             sh.runBin[0] |= RUN_ENDS;  // the reference breaks after the filling segment
+            sh.filled++;
             atomicAdd(HFB_G(&a.counters->finePoolFullBins), 1ull);
           }
         }
@@ -2039,7 +2155,7 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
             bits &= bits - 1u;
             const uint32_t at = sh.row[sh.rowOff[j] + ly].at(lx);
             if (HFB_EXPECT(at < PAIRS)) {
-              blendFragment<MAXL>(acc, sh.slice[at], sh.frag[at]);
+              slices.blend(sh.slice[at], sh.frag[at]);
               nFrag++;
               pending++;
             }
@@ -2053,21 +2169,11 @@ __device__ __forceinline__ FineEnd fineTile(FineSmem<TS>& sh, const HfbUniforms&
             const uint32_t cntAll = f2u(fmul(fin.x, (float)dbgMax)) + nFrag;
             fin = mk4(sat((float)cntAll / (float)dbgMax), 0.0f, 0.0f, 1.0f);
           } else {
-#pragma unroll
-            for (int si = 0; si < MAXL; si++) {
-              if ((uint32_t)si < L && fin.w < 0.999f) {
-                const float kk = fsub(1.0f, fin.w);
-                fin.x = fadd(fin.x, fmul(acc[si].x, kk));
-                fin.y = fadd(fin.y, fmul(acc[si].y, kk));
-                fin.z = fadd(fin.z, fmul(acc[si].z, kk));
-                fin.w = fadd(fin.w, fmul(acc[si].w, kk));
-              }
-            }
+            slices.reduce(fin, L);
             done = fin.w >= 0.999f;  // isPixelDone with ALPHA_CUTOFF
           }
         }
-#pragma unroll
-        for (int si = 0; si < MAXL; si++) acc[si] = mk4(0.f, 0.f, 0.f, 0.f);
+        slices.clear();
         nFrag = 0;
         pending = 0;
       }
@@ -2205,11 +2311,12 @@ __device__ __forceinline__ void fineScheduleBody(const uint32_t* __restrict__ ti
       const uint32_t slot = slotEnd - nG;
       (*HFB_G(&fs.arrivals[slot])) = 0;
       atomicAdd(HFB_G(&counters->fineSplitTiles), 1ull);
+      const uint32_t firstEnd = (uint32_t)__ffsll((long long)starts) - 1u;  // split: at least one later group
       uint32_t start = 0;
       for (uint32_t g = 0; g < nG; g++) {
         const uint32_t end = starts ? (uint32_t)__ffsll((long long)starts) - 1u : B;
         starts &= starts - 1ull;
-        (*HFB_G(&fs.items[itemBase + g])) = make_uint4(q, start | (end << 8) | (g << 16) | (nG << 24), slot, 0u);
+        (*HFB_G(&fs.items[itemBase + g])) = make_uint4(q, start | (end << 8) | (g << 16) | (nG << 24), slot, firstEnd);
         start = end;
       }
     } else if (nG) {
@@ -2234,14 +2341,19 @@ fineScheduleKernel(const uint32_t* __restrict__ tileList, const uint32_t* __rest
 }
 
 // One work item of the fine pass: a tile, or one group of depth bins of a
-// split tile (then the last group to finish merges the tile).
+// split tile.  The last group to finish merges the tile; where a later group
+// could fill a pool, the tile is drawn in order instead, from the end of the first
+// group.  The longest tiles in order are what a frame of long lists waits for
+// (200,000 x 32 at 4K: ~160 rounds of 11 us after the first group's ~90): with the
+// whole tile drawn again after the last group had taken its bins a second time with
+// exact counts, 4.2 ms; from the first group's end, with the undecided groups
+// settled from their bounds, 2.6 ms.
 template <int TS, int MAXL>
 __device__ __forceinline__ void fineItem(FineSmem<TS>& sh, const HfbUniforms& U, const FineArgs& a,
                                          const uint32_t* __restrict__ tileList, float* __restrict__ result,
                                          const FineScratch fs, const uint4 item) {
   using SM = FineSmem<TS>;
   constexpr uint32_t NT = SM::NT;
-  constexpr uint32_t UNSAFE = 1u << 31;
   const uint32_t tid = threadIdx.x;
   const uint32_t lx = tid % TS, ly = tid / TS;
   const uint32_t W = f2u(U.viewport.x), H = f2u(U.viewport.y);
@@ -2257,40 +2369,59 @@ __device__ __forceinline__ void fineItem(FineSmem<TS>& sh, const HfbUniforms& U,
     const uint32_t g = (item.y >> 16) & 0xffu, nG = item.y >> 24;
     if (tileIdx >= tileCount || b1 > a.B || b0 >= b1) return;
     bool split = nG > 1u, write = true;
-    if (split && (g >= nG || item.z >= fs.maxGroups || nG > fs.maxGroups - item.z)) {
+    if (split && (g >= nG || item.z >= fs.maxGroups || nG > fs.maxGroups - item.z || item.w == 0u || item.w >= a.B)) {
       // not an item the schedule writes: count it and leave the tile alone
       if (tid == 0) atomicAdd(HFB_G(&a.counters->badWorkItems), 1ull);
       return;
     }
     f4 fin;
     FinePart part = split && g > 0u ? FINE_QUICK : FINE_IN_ORDER;
+    const float4* resume = nullptr;
+    uint32_t* word = split ? &fs.arrivals[item.z] : nullptr;
     while (true) {
-      const FineEnd end = fineTile<TS, MAXL>(sh, U, a, tileIdx, b0, b1, part, fin);
+      const FineEnd end = fineTile<TS, MAXL>(sh, U, a, tileIdx, b0, b1, part, resume, fin);
       if (end == FINE_AGAIN) {  // uniform
         part = FINE_CAREFUL;
         __syncthreads();
         continue;
       }
       if (!split) break;
-      const bool ok = end == FINE_OK;
-      // a group of a split tile: publish its composite; the last to arrive merges
+      // A group of a split tile: publish its composite; the last to arrive merges.  Where
+      // a later group could fill a pool, the tile is drawn in order instead: from the end
+      // of the first group, which is in order already, by whoever finds both that it is
+      // there and that a group gave up.
       (*HFB_G(&fs.groups[(size_t)(item.z + g) * NT + tid])) = make_float4(fin.x, fin.y, fin.z, fin.w);
       __threadfence();
       __syncthreads();
       if (tid == 0) {
-        if (!ok) atomicOr(HFB_G(&fs.arrivals[item.z]), UNSAFE);
-        const uint32_t old = atomicAdd(HFB_G(&fs.arrivals[item.z]), 1u);
-        sh.arrive = (old & 0xffffu) + 1u == nG ? ((old & UNSAFE) ? 2u : 1u) : 0u;
-        if (sh.arrive == 2u) atomicAdd(HFB_G(&a.counters->fineSplitRedone), 1ull);
+        uint32_t todo = 0, old;
+        if (end != FINE_OK) {  // a later group: the count never fills up, so nobody merges
+          old = atomicOr(HFB_G(word), FINE_REDO);
+          if ((old & (FINE_FIRST | FINE_REDO)) == FINE_FIRST) todo = 2u;
+        } else {
+          old = atomicAdd(HFB_G(word), g == 0u ? (FINE_FIRST + 1u) | (sh.filled << FINE_FILLED_SHIFT) : 1u);
+          if (old & FINE_REDO) todo = g == 0u ? 2u : 0u;
+          else if ((old & 0xffffu) + 1u == nG) todo = 1u;
+        }
+        const uint32_t filled = g == 0u ? sh.filled : (old & FINE_FILLED) >> FINE_FILLED_SHIFT;
+        if (todo == 2u) {
+          atomicAdd(HFB_G(&a.counters->fineSplitRedone), 1ull);
+          // the bins before the point where the tile is taken up count once more, as if drawn again
+          if (filled) atomicAdd(HFB_G(&a.counters->finePoolFullBins), (unsigned long long)filled);
+        }
+        sh.arrive = todo;
       }
       __syncthreads();
       const uint32_t m = sh.arrive;
       if (m == 0u) { write = false; break; }
-      if (m == 2u) {  // a later group could fill a pool: the whole tile in order
-        b0 = 0;
+      if (m == 2u) {
+        __threadfence();
+        b0 = item.w;
         b1 = a.B;
+        resume = fs.groups + (size_t)item.z * NT;
         split = false;
         part = FINE_IN_ORDER;
+        __syncthreads();
         continue;
       }
       __threadfence();
@@ -2398,7 +2529,7 @@ cudaError_t launchFineT(HfbCtx* c, const HfbUniforms& u, const HfbHairData& h, c
                         const float4* proj) {
   HFB_CHECK_BIND(c);
   const HfbConfig& cfg = c->cfg;
-  constexpr size_t SMEM = sizeof(FineSmem<TS>);
+  constexpr size_t SMEM = FINE_SMEM<TS, MAXL>;
   int& perSM = c->fineBlocksPerSM[TS == 8 ? 0 : TS == 16 ? 1 : 2][MAXL == 4 ? 0 : MAXL == 8 ? 1 : 2];
   if (perSM == 0) {
     cudaError_t e = cudaFuncSetAttribute(fineKernel<TS, MAXL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
@@ -2570,7 +2701,7 @@ template <int TS, int MAXL>
 cudaError_t launchFineBatchT(HfbCtx* c, const BatchView& b) {
   HFB_CHECK_BIND(c);
   const HfbConfig& cfg = c->cfg;
-  constexpr size_t SMEM = sizeof(FineSmem<TS>);
+  constexpr size_t SMEM = FINE_SMEM<TS, MAXL>;
   uint32_t& grid = c->batchGrid[BK_COUNT];  // the fine kernel's persistent grid
   if (!grid) {
     cudaError_t e = cudaFuncSetAttribute(fineBatch<TS, MAXL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
