@@ -96,7 +96,8 @@ struct TilesScratch {
 // which is dead by then; all offsets 256-byte aligned).
 struct FineScratch {
   uint32_t* hdr;       // [0] = work items
-  uint4* items;        // tile list index, b0 | b1 << 8 | group << 16 | groups << 24, first group slot
+  uint4* items;        // tile list index, b0 | b1 << 8 | group << 16 | groups << 24, first group slot,
+                       // end of the first group's bins
   uint32_t* arrivals;  // per split tile (at its first group slot): see FINE_FIRST in raster.cu
   float4* groups;      // per group slot: the TS*TS composites of the group's depth bins
   uint32_t maxItems, maxGroups;
@@ -112,12 +113,16 @@ __host__ __device__ inline uint32_t simStrandsPerBlock(uint32_t P) {
   const uint32_t n = 2048u / P;
   return n > 128u ? 128u : n < 8u ? 8u : n;
 }
-// The same for one instance launched alone (hfb_sim_integrate, hfb_frame):
-// fewer strands per block (at least 8) while that gives up to two blocks per SM.
+// The same for one instance launched alone (hfb_sim_integrate, hfb_frame): as many
+// strands (at least 4) as make its blocks whole waves of three per SM.  Against full
+// blocks from two per SM on, and at least 8 strands: 40,000 x 16 211 -> 180 us (three
+// passes; 313 blocks of 128 left some SMs three blocks and most two), 1,501 x 65 136 ->
+// 132 us.
 __host__ __device__ inline uint32_t simStrandsPerBlockFor(uint32_t S, uint32_t P, uint32_t smCount) {
   const uint32_t full = simStrandsPerBlock(P);
-  const uint32_t want = (S + 2u * smCount - 1u) / (2u * smCount);  // strands per block for 2 blocks per SM
-  return want >= full ? full : want < 8u ? 8u : want;
+  const uint64_t room = 3ull * smCount, waves = S ? (S + full * room - 1u) / (full * room) : 1u;
+  const uint32_t want = (uint32_t)((S + waves * room - 1u) / (waves * room));
+  return want >= full ? full : want < 4u ? 4u : want;
 }
 // And for an instance of a batch of S strands in all: fewer than full blocks when the
 // batch does not give every SM its SIM_BATCH_BLOCKS of them, down to 8 strands, so that
