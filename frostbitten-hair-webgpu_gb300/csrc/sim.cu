@@ -198,7 +198,8 @@ __global__ void __launch_bounds__(256) gridPreSimKernel(const HfbSimUniforms u, 
 // steps ahead.  Against constants in PREV for every block, whose loads came from L2
 // and held each bending step for about 340 cycles: 3.15 -> 2.71 ms (64 instances);
 // with 256 threads, for the point phases, in the single-instance kernel: 309 -> 222 us
-// (40,000 x 16, three passes), 175 -> 137 us (1,501 x 65); 512 threads 250 and 141 us.
+// (40,000 x 16, three passes), 175 -> 137 us (1,501 x 65); 512 threads 250 and 141 us;
+// with blocks of a whole wave (simStrandsPerBlockFor) 180 and 132 us.
 // Per block of the 64-instance frame (clock counters, before): Verlet 32 %, length
 // chain 10 %, global shape 10 %, bending chain 19 %, collisions 29 %.
 //
@@ -686,8 +687,12 @@ __device__ __forceinline__ void gridPostSimBody(const HfbSimUniforms& u, uint32_
   // the same cell (mostly neighbours on one strand) add their corner values in
   // registers first (wrapping, as the table and the grid do), and the cell's sums
   // go to the table when the cell changes or the points end -- one set of table
-  // adds per run of points
-  uint4 acc[8];
+  // adds per run of points.  A corner's share of the velocity's x depends on its x
+  // alone, so the run's sums are two numbers per axis, and eight of the weights'
+  // lengths; what a point adds to a corner that does not exist is never read
+  // (32 sums, four per corner: 40,000 x 16, three passes, 180 -> 177 us; 64 instances
+  // 12.32 -> 12.24 ms.  Points loaded one ahead, or 2,048 points per block: slower.)
+  unsigned ax[2], ay[2], az[2], aw[8];
   uint32_t c0 = 0, c1 = 0, c2 = 0, cm = GP_NO_CELL;  // the cell being summed; cm: its corner mask
   const uint32_t vb = blk * GP_POINTS + threadIdx.x * GP_PPT;
 #pragma unroll 1
@@ -713,24 +718,28 @@ __device__ __forceinline__ void gridPostSimBody(const HfbSimUniforms& u, uint32_
 #pragma unroll
         for (uint32_t k = 0; k < 8u; k++)
           if ((k & ~cm) == 0u)
-            gridPostAdd(sh, dv, gridIdx(G, c0 + (k & 1u), c1 + ((k >> 1) & 1u), c2 + (k >> 2)), acc[k]);
+            gridPostAdd(sh, dv, gridIdx(G, c0 + (k & 1u), c1 + ((k >> 1) & 1u), c2 + (k >> 2)),
+                        make_uint4(ax[k & 1u], ay[(k >> 1) & 1u], az[k >> 2], aw[k]));
       }
       if (!more) break;
 #pragma unroll
-      for (uint32_t k = 0; k < 8u; k++) acc[k] = make_uint4(0u, 0u, 0u, 0u);
+      for (uint32_t k = 0; k < 2u; k++) ax[k] = ay[k] = az[k] = 0u;
+#pragma unroll
+      for (uint32_t k = 0; k < 8u; k++) aw[k] = 0u;
       c0 = co.mn[0]; c1 = co.mn[1]; c2 = co.mn[2]; cm = m;
     }
+    const f3 w[2] = {cellWeights(co.mn[0], co.mn[1], co.mn[2], co.p),
+                     cellWeights(co.mn[0] + 1u, co.mn[1] + 1u, co.mn[2] + 1u, co.p)};
 #pragma unroll
-    for (uint32_t k = 0; k < 8u; k++) {
-      if ((k & ~m) != 0u) continue;
-      const uint32_t x = co.mn[0] + (k & 1u), y = co.mn[1] + ((k >> 1) & 1u), z = co.mn[2] + (k >> 2);
-      const f3 w = cellWeights(x, y, z, co.p);
-      const f3 cv = mul3(vel, w);
-      acc[k].x += (unsigned)gridEncode(cv.x);
-      acc[k].y += (unsigned)gridEncode(cv.y);
-      acc[k].z += (unsigned)gridEncode(cv.z);
-      acc[k].w += (unsigned)gridEncode(len3(w));
+    for (uint32_t k = 0; k < 2u; k++) {
+      const f3 cv = mul3(vel, w[k]);
+      ax[k] += (unsigned)gridEncode(cv.x);
+      ay[k] += (unsigned)gridEncode(cv.y);
+      az[k] += (unsigned)gridEncode(cv.z);
     }
+#pragma unroll
+    for (uint32_t k = 0; k < 8u; k++)
+      aw[k] += (unsigned)gridEncode(len3(mk3(w[k & 1u].x, w[(k >> 1) & 1u].y, w[k >> 2].z)));
   }
   __syncthreads();
   for (uint32_t e = threadIdx.x; e < GP_HASH; e += blockDim.x) {
