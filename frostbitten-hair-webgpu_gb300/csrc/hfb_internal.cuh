@@ -10,6 +10,7 @@
 
 #include "hfb_check.cuh"
 
+constexpr uint32_t SIDE_EVENTS = 6;
 struct HfbCtx {
   HfbConfig cfg;
   int device = 0;
@@ -63,7 +64,8 @@ struct HfbCtx {
   // whole frames: a second stream for what does not wait for the passes on the caller's
   // (made with the context; NULL: everything on the caller's stream)
   cudaStream_t sideStream = nullptr;
-  cudaEvent_t sideEvents[4] = {};  // frame start, clears done, simulated, side work done
+  cudaEvent_t sideEvents[SIDE_EVENTS] = {};  // frame start, clears done, simulated, rasterized, sorted, side work done
+  cudaEvent_t rasterDone = nullptr;  // recorded by the tiles pass after its raster (set for the call only)
   // the projected segments of a whole frame (hfb_frame, hfb_frame_batch):
   // written by the tiles pass, read by the fine pass; grown on demand
   float4* projCache = nullptr;

@@ -2759,6 +2759,7 @@ cudaError_t launchTilesPass(HfbCtx* c, const HfbUniforms& u, const HfbHairData& 
         (const float4*)tan, depth, (uint4*)rb.tiles, rb.tileSegments, rb.segmentCountPerTile, s.binCount, dc, proj);
     HFB_AFTER_LAUNCH(c, "tilesRasterKernel");
   }
+  if (c->rasterDone && (e = cudaEventRecord(c->rasterDone, c->stream)) != cudaSuccess) return e;
   const uint32_t nBlocks = divCeil(TB, SCAN_PER_BLOCK);
   binScanBlocks<<<nBlocks, 512, 0, c->stream>>>(s.binCount, s.binOffset, s.blockSums, TB);
   HFB_AFTER_LAUNCH(c, "binScanBlocks");
@@ -2858,6 +2859,10 @@ cudaError_t launchBatchTiles(HfbCtx* c, const BatchView& b) {
   }
   tilesRasterBatch<<<batchLaunchGrid(c, g[BK_RASTER]), TR_SEGS, 0, c->stream>>>(b, cfg, dc);
   HFB_AFTER_LAUNCH(c, "tilesRasterBatch");
+  if (c->rasterDone) {
+    const cudaError_t e = cudaEventRecord(c->rasterDone, c->stream);
+    if (e != cudaSuccess) return e;
+  }
   binScanBatch<<<batchLaunchGrid(c, g[BK_SCAN]), 512, 0, c->stream>>>(b, cfg);
   HFB_AFTER_LAUNCH(c, "binScanBatch");
   binScanSumsBatch<<<batchLaunchGrid(c, g[BK_SCAN_SUMS]), 1024, 0, c->stream>>>(b, cfg);
