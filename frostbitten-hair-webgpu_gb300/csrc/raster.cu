@@ -177,7 +177,11 @@ __device__ __forceinline__ uint32_t blockExclusiveScan(uint32_t v, uint32_t* war
 // 2.65 -> 1.58 ms (200,000 x 32 at 4K), 3.14 -> 2.43 ms (64 instances).
 // ---------------------------------------------------------------------------
 constexpr uint32_t TR_SEGS = TILES_RASTER_SEGS;  // segments (and threads) per block
-constexpr uint32_t TR_SLOTS = 256;               // (segment, tile) accumulators per warp
+// (segment, tile) accumulators per warp.  The raster's gathers live from L1, which is what
+// shared memory leaves of the SM's 256 KB: six blocks of 31 KB, not 37 (256 slots), take the
+// 64-instance frame from 12.28 to 12.06 ms; 96 the same, 64 slots 12.13 (more rounds), a
+// seventh block 12.20.
+constexpr uint32_t TR_SLOTS = 128;
 
 struct TrShared {
   float4 ox[TR_SEGS], oy[TR_SEGS], ex[TR_SEGS], ey[TR_SEGS];  // edge tests (insideQuad order)
