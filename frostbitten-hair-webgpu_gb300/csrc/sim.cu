@@ -203,11 +203,14 @@ __global__ void __launch_bounds__(256) gridPreSimKernel(const HfbSimUniforms u, 
 // Per block of the 64-instance frame (clock counters, before): Verlet 32 %, length
 // chain 10 %, global shape 10 %, bending chain 19 %, collisions 29 %.
 //
-// A block of 128 threads of the batched kernel holds 2,048 points (64 strands of 32,
-// 128 of 16), six blocks per SM: 384 strands of 32 points in flight per SM.
+// A block of 128 threads of the batched kernel holds 1,536 points (48 strands of 32, 96
+// of 16), seven blocks per SM: 336 strands of 32 points in flight per SM, and 70 KB of its
+// L1 left for the Verlet phase's grid gathers.  Six blocks of 2,048 points left 50 KB:
+// 12.05 -> 11.88 ms on the 64-instance frame, 1,183 -> 1,160 us on a tick of 6 sessions; six
+// of 1,536 11.96, eight 11.98, seven of 1,280 12.09.
 // ---------------------------------------------------------------------------
 constexpr uint32_t SIM_THREADS = 256;        // threads per block of the single-instance kernel
-constexpr uint32_t SIM_BATCH_THREADS = 128;  // and of the batched one (6 blocks per SM)
+constexpr uint32_t SIM_BATCH_THREADS = 128;  // and of the batched one (SIM_BATCH_BLOCKS per SM)
 
 
 // p + z for z a signed zero whose sign is that of c xor the bit in s: p itself
