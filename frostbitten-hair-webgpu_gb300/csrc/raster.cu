@@ -6,19 +6,19 @@
 // processHairSegment,reduceHairSlices,tileUtils}.wgsl.ts and the buffer
 // layouts of shared/*.ts.
 //
-// Tiles pass = 5 kernels:
-//   1. tilesRaster   one thread per (strand, segment): project, bound, walk
-//                    the covered pixels of every tile of the bounding rect,
-//                    emit one (tile-bin, key) record per touched tile; the
-//                    head min/max depth atomics and the per-tile counts are
-//                    order independent.
-//   2. binScan       exclusive prefix of the per-(tile, bin) record counts.
+// Tiles pass = 6 kernels:
+//   1. tilesRaster   a warp per 32 segments: project, bound, list the pixels of
+//                    the box rows' spans, emit one (tile-bin, key) record per
+//                    touched tile; the head min/max depth atomics and the
+//                    per-tile counts are order independent.
+//   2. binScan       exclusive prefix of the per-(tile, bin) record counts (two
+//                    kernels).
 //   3. binScatter    counting-sort scatter of the record keys into CSR order.
 //   4. binFinalize   sort each (tile, bin)'s keys ascending and write the
-//                    reference's linked list (head -> largest key): a warp
-//                    per bin (single instance); in the batched frame 8 lanes
-//                    per bin of at most 8 records and a warp per larger bin.
-//   5. largeBins     one CTA per bin with more than 1024 records.
+//                    reference's linked list (head -> largest key): 8 lanes per
+//                    bin of at most 8 records, a warp up to WARP_BIN, a block up
+//                    to MEDIUM_BIN.
+//   5. largeBins     one CTA per bin with more than MEDIUM_BIN records.
 // The resulting lists are canonical: they do not depend on atomic order.
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
