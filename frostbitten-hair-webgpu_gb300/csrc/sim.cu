@@ -620,9 +620,9 @@ simIntegrateKernel(const HfbSimUniforms u, uint32_t S, uint32_t P, uint32_t G,
 // _addGridDensityVelocity, densityVelocityGrid.wgsl.ts:93-124.
 //
 // Each point adds to the eight corners of its cell, four wrapping i32 adds
-// each.  A block takes GP_POINTS points, strand after strand in the order
+// each.  A block takes GP_THREADS * PPT points, strand after strand in the order
 // strandOrder gives (neighbouring strands next to each other: their points
-// share grid nodes), a thread GP_PPT consecutive ones: the points of a run
+// share grid nodes), a thread PPT consecutive ones: the points of a run
 // in one cell sum their corner values in registers, each run's sums merge
 // per grid node in a shared-memory hash table, and each node's four sums
 // then go to global memory as one set of atomics.
@@ -631,11 +631,11 @@ simIntegrateKernel(const HfbSimUniforms u, uint32_t S, uint32_t P, uint32_t G,
 // free slot within GP_PROBES goes straight to global memory.
 // ---------------------------------------------------------------------------
 constexpr uint32_t GP_THREADS = 256;
-constexpr uint32_t GP_POINTS = 1024;  // points per block (four per thread)
+constexpr uint32_t GP_PPT = 4;        // consecutive points per thread, at most
+constexpr uint32_t GP_POINTS = GP_PPT * GP_THREADS;  // points per block of the batched kernel
 constexpr uint32_t GP_HASH = 2048;    // slots (power of two)
 constexpr uint32_t GP_PROBES = 32;
 constexpr uint32_t GP_EMPTY = 0xffffffffu;
-constexpr uint32_t GP_PPT = GP_POINTS / GP_THREADS;  // consecutive points per thread
 constexpr uint32_t GP_NO_CELL = 0xffffffffu;
 constexpr uint32_t GP_BATCH_BLOCKS = 3;  // blocks per SM of the batched kernel (the run sums need registers)
 
@@ -677,16 +677,17 @@ __device__ __forceinline__ void gridPostAdd(GridPostShared& sh, unsigned* __rest
   atomicAdd(c + 3, v.w);
 }
 
-// Ordered points [blk * GP_POINTS, (blk + 1) * GP_POINTS) of the S * P: the
+// Ordered points [blk * PPT * GP_THREADS, (blk + 1) * PPT * GP_THREADS) of the S * P: the
 // ordered point v is point v % P of strand order[v / P].  The table is empty
 // on entry and on exit.  All threads of the block call it.
+template <uint32_t PPT>
 __device__ __forceinline__ void gridPostSimBody(const HfbSimUniforms& u, uint32_t S, uint32_t P, uint32_t G,
                                                 const float4* __restrict__ prev, const float4* __restrict__ now,
                                                 unsigned* __restrict__ dv, const uint32_t* __restrict__ order,
                                                 uint32_t blk, GridPostShared& sh) {
   const uint32_t N = S * P;
   const f3 gmin = gridMin(u), gmax = gridMax(u);
-  // a thread's GP_PPT consecutive ordered points: consecutive points that fall in
+  // a thread's PPT consecutive ordered points: consecutive points that fall in
   // the same cell (mostly neighbours on one strand) add their corner values in
   // registers first (wrapping, as the table and the grid do), and the cell's sums
   // go to the table when the cell changes or the points end -- one set of table
@@ -697,11 +698,11 @@ __device__ __forceinline__ void gridPostSimBody(const HfbSimUniforms& u, uint32_
   // 12.32 -> 12.24 ms.  Points loaded one ahead, or 2,048 points per block: slower.)
   unsigned ax[2], ay[2], az[2], aw[8];
   uint32_t c0 = 0, c1 = 0, c2 = 0, cm = GP_NO_CELL;  // the cell being summed; cm: its corner mask
-  const uint32_t vb = blk * GP_POINTS + threadIdx.x * GP_PPT;
+  const uint32_t vb = (blk * GP_THREADS + threadIdx.x) * PPT;
 #pragma unroll 1
-  for (uint32_t r = 0; r <= GP_PPT; r++) {
+  for (uint32_t r = 0; r <= PPT; r++) {
     const uint32_t v = vb + r;
-    const bool more = r < GP_PPT && v < N;
+    const bool more = r < PPT && v < N;
     GridCo co;
     f3 vel;
     uint32_t m = GP_NO_CELL;
@@ -760,13 +761,14 @@ __device__ __forceinline__ void gridPostSimBody(const HfbSimUniforms& u, uint32_
   // the next points' adds come after batchNext's barrier, with the table empty
 }
 
+template <uint32_t PPT>
 __global__ void __launch_bounds__(GP_THREADS)
 gridPostSimKernel(const HfbSimUniforms u, uint32_t S, uint32_t P, uint32_t G, const float4* __restrict__ prev,
                   const float4* __restrict__ now, unsigned* __restrict__ dv, const uint32_t* __restrict__ order) {
   __shared__ GridPostShared sh;
   gridPostClear(sh);
   __syncthreads();
-  gridPostSimBody(u, S, P, G, prev, now, dv, order, blockIdx.x, sh);
+  gridPostSimBody<PPT>(u, S, P, G, prev, now, dv, order, blockIdx.x, sh);
 }
 
 // ---- batched: persistent over the virtual blocks of every instance ----
@@ -813,7 +815,7 @@ __global__ void __launch_bounds__(GP_THREADS, GP_BATCH_BLOCKS) gridPostSimBatch(
     const uint32_t i = batchFind(row, n, v);
     const BatchInst& I = b.insts[i];
     // after the swap: prev = the old current positions, now = the new ones
-    gridPostSimBody(I.SU, I.S, I.P, G, I.posOld, I.posNew, (unsigned*)I.dv, I.gridOrder, v - row[i], sh);
+    gridPostSimBody<GP_PPT>(I.SU, I.S, I.P, G, I.posOld, I.posNew, (unsigned*)I.dv, I.gridOrder, v - row[i], sh);
   }
 }
 
@@ -947,8 +949,17 @@ cudaError_t launchGridPostSim(HfbCtx* c, const HfbSimUniforms& u, const HfbHairD
   if (e != cudaSuccess) return e;
   const uint32_t N = h.strandsCount * h.pointsPerStrand;
   if (N) {
-    gridPostSimKernel<<<gridPostBlocks(N), GP_THREADS, 0, c->stream>>>(
-        u, h.strandsCount, h.pointsPerStrand, G, (const float4*)prev, (const float4*)now, (unsigned*)dv, strandOrder);
+    auto launch = [&](auto kernel, uint32_t ppt) {
+      kernel<<<divCeil(N, ppt * GP_THREADS), GP_THREADS, 0, c->stream>>>(
+          u, h.strandsCount, h.pointsPerStrand, G, (const float4*)prev, (const float4*)now, (unsigned*)dv, strandOrder);
+    };
+    // fewer points per thread where more would leave fewer than two blocks per SM: the
+    // simulation of 1,501 x 65 (96 blocks of 1,024 points) 131 -> 119 us; from 305 blocks of
+    // 1,024 on (10,000 x 32) longer runs are worth more: a frame 337 us, 344 at two points
+    const uint32_t few = 2u * (uint32_t)c->smCount * GP_THREADS;  // points of one per thread
+    if (N >= 4u * few) launch(gridPostSimKernel<4>, 4u);
+    else if (N >= 2u * few) launch(gridPostSimKernel<2>, 2u);
+    else launch(gridPostSimKernel<1>, 1u);
     HFB_AFTER_LAUNCH(c, "gridPostSimKernel");
     c->launches += 1;
   }

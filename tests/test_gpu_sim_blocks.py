@@ -1,6 +1,6 @@
 """The simulation over numbers of strands where its blocks' sizes change (the
 fewest strands per block, a last block of one strand, a second wave of full
-blocks), with points outside the grid and on its nodes; bit for bit, against the
+blocks; one, two and four points per thread of the grid splat), with points outside the grid and on its nodes; bit for bit, against the
 CPU oracle."""
 import numpy as np
 import pytest
@@ -17,7 +17,7 @@ from hairfb.passes import GridPostSimPass, GridPreSimPass, HairObject, HairSimIn
 from test_gpu_parity import _ctx, _sim_inputs, oracle  # noqa: E402,F401
 
 
-@pytest.mark.parametrize("strands,points", [(1, 4), (3, 65), (4, 128), (455, 16), (1825, 17), (2281, 32), (59001, 16)])
+@pytest.mark.parametrize("strands,points", [(1, 4), (3, 65), (4, 128), (455, 16), (1825, 17), (2281, 32), (12001, 16), (59001, 16)])
 def test_one_step_for_any_number_of_strands_bit_exact(oracle, strands, points):  # noqa: F811
     inst = small_instance(strands=strands, points=points, iterations=2)
     hb = inst.hair
