@@ -71,7 +71,7 @@ cudaError_t clearRasterRanges(HfbCtx* c, const HfbRasterBuffers& rb, bool tilesP
   if (tilesPass) {
     const TilesScratch ts = tilesScratchLayout(rb.scratch, cfg, rb.width, rb.height, rb.maxDrawnSegments);
     z(ts.binCount, T * cfg.tileDepthBins * 4);
-    z(ts.largeBins, 4);
+    z(ts.largeBins, 8);  // its count, and the scan's count of blocks
   }
   uint32_t blocks = 0;
   for (uint32_t k = 0; k < a.n; k++) blocks += (uint32_t)((a.r[k].bytes + CLEAR_CHUNK - 1) / CLEAR_CHUNK);

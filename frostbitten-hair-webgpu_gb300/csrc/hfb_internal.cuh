@@ -90,7 +90,8 @@ struct TilesScratch {
   uint32_t* binOffset;   // T*B exclusive prefix of binCount, then cursor
   uint32_t* keys;        // maxDrawn sort keys (strand << 8 | segment), CSR order
   uint32_t* blockSums;   // scan partials
-  uint32_t* largeBins;   // [0] = count, then bin indices with > 1024 records
+  uint32_t* largeBins;   // [0] = count, then bin indices with > 1024 records; until then
+                         // [1] counts binScanKernel's blocks
   size_t bytes;
 };
 

@@ -6,13 +6,13 @@
 // processHairSegment,reduceHairSlices,tileUtils}.wgsl.ts and the buffer
 // layouts of shared/*.ts.
 //
-// Tiles pass = 6 kernels:
+// Tiles pass = 5 kernels:
 //   1. tilesRaster   a warp per 32 segments: project, bound, list the pixels of
 //                    the box rows' spans, emit one (tile-bin, key) record per
 //                    touched tile; the head min/max depth atomics and the
 //                    per-tile counts are order independent.
-//   2. binScan       exclusive prefix of the per-(tile, bin) record counts (two
-//                    kernels).
+//   2. binScan       exclusive prefix of the per-(tile, bin) record counts (the
+//                    batched frame: two kernels).
 //   3. binScatter    counting-sort scatter of the record keys into CSR order.
 //   4. binFinalize   sort each (tile, bin)'s keys ascending and write the
 //                    reference's linked list (head -> largest key): 8 lanes per
@@ -515,7 +515,7 @@ tilesRasterKernel(const HfbUniforms U, uint32_t P, uint32_t nStrands, uint32_t T
 // 2. binScan: exclusive prefix over T*B counts (block-local + block sums)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void binScanBlocksBody(const uint32_t* __restrict__ cnt, uint32_t* __restrict__ off,
-                                                  uint32_t* __restrict__ blockSums, uint32_t n, uint32_t* warpSums,
+                                                  uint32_t* blockSums, uint32_t n, uint32_t* warpSums,
                                                   uint32_t blk) {
   const uint32_t base = blk * SCAN_PER_BLOCK + threadIdx.x * 4u;
   uint32_t v[4], s = 0;
@@ -534,18 +534,12 @@ __device__ __forceinline__ void binScanBlocksBody(const uint32_t* __restrict__ c
   if (threadIdx.x == 0) (*HFB_G(&blockSums[blk])) = total;
 }
 
-__global__ void __launch_bounds__(512) binScanBlocks(const uint32_t* __restrict__ cnt, uint32_t* __restrict__ off,
-                                                     uint32_t* __restrict__ blockSums, uint32_t n) {
-  __shared__ uint32_t warpSums[32];
-  binScanBlocksBody(cnt, off, blockSums, n, warpSums, blockIdx.x);
-}
-
-__device__ __forceinline__ void binScanSumsBody(uint32_t* __restrict__ blockSums, uint32_t nBlocks,
+__device__ __forceinline__ void binScanSumsBody(uint32_t* blockSums, uint32_t nBlocks,
                                                 uint32_t* warpSums) {
   uint32_t carry = 0;
   for (uint32_t b0 = 0; b0 < nBlocks; b0 += blockDim.x) {
     uint32_t i = b0 + threadIdx.x;
-    uint32_t v = i < nBlocks ? (*HFB_G(&blockSums[i])) : 0u;
+    uint32_t v = i < nBlocks ? __ldcg(HFB_G(&blockSums[i])) : 0u;  // other blocks' stores: not from L1
     uint32_t total;
     uint32_t ex = blockExclusiveScan(v, warpSums, total);
     if (i < nBlocks) (*HFB_G(&blockSums[i])) = carry + ex;
@@ -553,9 +547,20 @@ __device__ __forceinline__ void binScanSumsBody(uint32_t* __restrict__ blockSums
   }
 }
 
-__global__ void __launch_bounds__(1024) binScanSums(uint32_t* __restrict__ blockSums, uint32_t nBlocks) {
-  __shared__ uint32_t warpSums[32];
-  binScanSumsBody(blockSums, nBlocks, warpSums);
+// Both in one launch: the block that finishes last scans the sums (arrived, 0 on
+// entry, counts the blocks; nobody waits).  A second launch of one block took 4 us.
+__global__ void __launch_bounds__(512) binScanKernel(const uint32_t* __restrict__ cnt, uint32_t* __restrict__ off,
+                                                     uint32_t* blockSums, uint32_t* __restrict__ arrived, uint32_t n) {
+  __shared__ uint32_t warpSums[32], last;
+  binScanBlocksBody(cnt, off, blockSums, n, warpSums, blockIdx.x);
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(HFB_G(arrived), 1u) == gridDim.x - 1u;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  binScanSumsBody(blockSums, gridDim.x, warpSums);
 }
 
 // ---------------------------------------------------------------------------
@@ -2750,7 +2755,7 @@ cudaError_t launchTilesPass(HfbCtx* c, const HfbUniforms& u, const HfbHairData& 
   cudaError_t e = cudaSuccess;
   if (!cleared) {
     e = cudaMemsetAsync(s.binCount, 0, (size_t)TB * 4, c->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(s.largeBins, 0, 4, c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(s.largeBins, 0, 8, c->stream);
     if (e != cudaSuccess) return e;
   }
   const uint32_t nStrands = min(strandsToRender, h.strandsCount);
@@ -2765,10 +2770,8 @@ cudaError_t launchTilesPass(HfbCtx* c, const HfbUniforms& u, const HfbHairData& 
   }
   if (c->rasterDone && (e = cudaEventRecord(c->rasterDone, c->stream)) != cudaSuccess) return e;
   const uint32_t nBlocks = divCeil(TB, SCAN_PER_BLOCK);
-  binScanBlocks<<<nBlocks, 512, 0, c->stream>>>(s.binCount, s.binOffset, s.blockSums, TB);
-  HFB_AFTER_LAUNCH(c, "binScanBlocks");
-  binScanSums<<<1, 1024, 0, c->stream>>>(s.blockSums, nBlocks);
-  HFB_AFTER_LAUNCH(c, "binScanSums");
+  binScanKernel<<<nBlocks, 512, 0, c->stream>>>(s.binCount, s.binOffset, s.blockSums, &s.largeBins[1], TB);
+  HFB_AFTER_LAUNCH(c, "binScanKernel");
   binScatterKernel<<<c->smCount * 8, 256, 0, c->stream>>>(rb.tileSegments, rb.maxDrawnSegments, s.binOffset,
                                                           s.blockSums, s.keys, dc, TB);
   HFB_AFTER_LAUNCH(c, "binScatterKernel");
@@ -2784,7 +2787,7 @@ cudaError_t launchTilesPass(HfbCtx* c, const HfbUniforms& u, const HfbHairData& 
   largeBinsKernel<<<c->smCount * 2, 1024, LARGE_SMEM_KEYS * 4, c->stream>>>(
       s.largeBins, s.binCount, s.binOffset, s.blockSums, s.keys, rb.tileSegments, (uint4*)rb.tiles);
   HFB_AFTER_LAUNCH(c, "largeBinsKernel");
-  c->launches += nSeg ? 6 : 5;
+  c->launches += nSeg ? 5 : 4;
   return cudaGetLastError();
 }
 
@@ -2796,8 +2799,7 @@ cudaError_t launchTilesPass(HfbCtx* c, const HfbUniforms& u, const HfbHairData& 
 cudaError_t tilesPassLoad(HfbCtx* c) {
   cudaFuncAttributes a;
   cudaError_t e = cudaFuncGetAttributes(&a, tilesRasterKernel);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, binScanBlocks);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, binScanSums);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, binScanKernel);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, binScatterKernel);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, binFinalizeKernel);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, largeBinsKernel);
