@@ -773,8 +773,11 @@ __device__ __forceinline__ void binFinalizeWarpBody(uint32_t TB, const uint32_t*
   __shared__ uint32_t nQueue;
   if (threadIdx.x == 0) nQueue = 0;
   __syncthreads();
-  for (uint64_t base = (uint64_t)blk * (blockDim.x >> 5); base < TB; base += 32ull * nw) {  // uniform in the block
-    const uint64_t at = base + warp + (uint64_t)lane * nw;
+  // a tile's bins, neighbours, go to different blocks: where they are all large, one block
+  // would sort them one after the other (a draw of 7,001 x 23 with 32 px tiles: 343 -> 332
+  // us; 200,000 x 32 at 4K: 6.40 -> 6.31 ms)
+  for (uint64_t base = blk; base < TB; base += 32ull * nw) {  // uniform in the block
+    const uint64_t at = base + (uint64_t)warp * nblk + (uint64_t)lane * nw;
     const uint32_t ti = at < TB ? (uint32_t)at : 0u;
     const uint32_t n = at < TB ? (*HFB_G(&binCount[ti])) : 0u;
     const uint32_t end = n ? (*HFB_G(&blockSums[ti / SCAN_PER_BLOCK])) + (*HFB_G(&binOffset[ti])) : 0u;  // bin end
