@@ -410,8 +410,8 @@ __device__ __forceinline__ void simIntegrateBody(const HfbSimUniforms& u, uint32
     float4 p = pt == 0u ? make_float4(posNow.x, posNow.y, posNow.z, posNow.w)
                         : verletPoint(u, G, gmin, gmax, s0 + ls, posNow, ld4(*HFB_G(&prev[gi])), dv, gw);
     const float4 i0 = __ldg(HFB_G(&initial[gi]));
-    const float weight = pt == 0u ? 0.0f : 1.0f;
-    plain = plain && posNow.w == weight && i0.w == weight;
+    const uint32_t weight = pt == 0u ? 0u : 0x3f800000u;  // by the bits: a root of weight -0 keeps its sign
+    plain = plain && __float_as_uint(posNow.w) == weight && __float_as_uint(i0.w) == weight;
     if (pt + 3u < P) p.w = restHeight(i0, __ldg(HFB_G(&initial[gi + 1u])), __ldg(HFB_G(&initial[gi + 2u])));
     wk[ls * R + pt] = p;
   }

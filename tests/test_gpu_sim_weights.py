@@ -48,3 +48,30 @@ def test_one_step_for_any_weights_bit_exact(oracle, points, weights):  # noqa: F
                                 hb.segment_lengths, odv, ogw, inst.sdf.distances, inst.sdf.dims)
     g = hair.positions.cpu().numpy()
     assert np.array_equal(g.view(np.uint32), onew.view(np.uint32)), f"max abs diff {np.abs(g - onew).max()}"
+
+
+@pytest.mark.parametrize("points", [4, 16, 65])
+def test_a_root_of_weight_minus_zero_keeps_it(oracle, points):  # noqa: F811
+    """A root of weight -0 is fixed too, and its weight comes back as it went in, as the
+    oracle leaves it."""
+    inst = small_instance(strands=301, points=points, iterations=2)
+    pos = inst.hair.asset.positions.reshape(301, points, 4)
+    pos[::3, 0, 3] = -0.0
+    inst.hair = hb = HO.build_hair_buffers(inst.hair.asset)
+    su = _sim_inputs(inst, 3)
+    ctx = _ctx(inst)
+    hair = HairObject(hb, inst.cfg.shading_points)
+    grids = PhysicsGrids(inst.cfg.grid_dims)
+    sdf = SdfCollider(inst.sdf)
+    GridPostSimPass(ctx).cmd_update_grids_after_sim(su, hair, grids)
+    GridPreSimPass(ctx).cmd_update_grids_before_sim(su, grids, sdf)
+    HairSimIntegrationPass(ctx).cmd_simulate_hair_positions(su, hair, grids, sdf)
+    ctx.sync()
+    p0 = hb.asset.positions
+    odv = oracle.grid_post_sim(inst.cfg, su, hb.hair_data, p0, p0)
+    ogw = oracle.grid_pre_sim(inst.cfg, su, odv, inst.sdf.distances, inst.sdf.dims)
+    onew = oracle.sim_integrate(inst.cfg, su, hb.hair_data, p0, p0, p0, hb.segment_lengths, odv, ogw,
+                                inst.sdf.distances, inst.sdf.dims)
+    g = hair.positions.cpu().numpy()
+    assert (g.reshape(301, points, 4)[::3, 0, 3].view(np.uint32) == 0x80000000).all()
+    assert np.array_equal(g.view(np.uint32), onew.view(np.uint32))
