@@ -386,7 +386,8 @@ cudaError_t launchHairNormals(HfbCtx* c, const HfbUniforms& u, const HfbHairData
 // AO texture extent: ceil(viewport * scale), as the reference sizes it (renderer.ts:405-409).
 uint32_t aoExtent(float viewport, float scale);
 cudaError_t launchGtao(HfbCtx* c, const HfbUniforms& u, const float* depth, const float* normals, float scale,
-                       float* ao);
+// general: by the kernel for any scale, also at 0.5
+                       float* ao, bool general = false);
 cudaError_t launchPresent(HfbCtx* c, const HfbUniforms& u, uint32_t W, uint32_t H, const float* result,
                           const float* scene, uint8_t* rgba);
 cudaError_t launchPresentBatch(HfbCtx* c, const HfbPresentItem* items, uint32_t n);

@@ -114,6 +114,7 @@ SIGNATURES = {
     "hfb_gtao": (I, [P, P, P, P, ctypes.c_float, P]),
     "hfb_frame": (I, [P, P]),
     "hfb_frame_batch": (I, [P, P, U32]),
+    "hfb_check_gtao": (I, [P, P, P, P, ctypes.c_float, P]),
     "hfb_frame_batch_profile": (I, [P, P, U32, P]),
     "hfb_ctx_set_batch_groups": (I, [P, U32]),
     "hfb_ctx_set_batch_pipeline": (I, [P, U32]),

@@ -409,6 +409,10 @@ HFB_API int hfb_frame(HfbCtx* ctx, HfbInstance* instance);
  * is a CUDA graph captured once per context, and the fine pass pulls the
  * tiles of all instances from one queue.  The context's config (tile size,
  * depth bins, slices, grid size) applies to every instance.  Results are
+/* The same by the kernel for any scale, without the shared tile that hfb_gtao uses
+ * at scale 0.5: the two are equal bit for bit (a self-check). */
+HFB_API int hfb_check_gtao(HfbCtx* ctx, const HfbUniforms* uniforms, const float* depth, const float* normals,
+                           float scale, float* ao);
  * those of hfb_frame on each instance alone.  The call flips every
  * instance's `current`.  n <= 1024. */
 HFB_API int hfb_frame_batch(HfbCtx* ctx, HfbInstance* instances, uint32_t n);
