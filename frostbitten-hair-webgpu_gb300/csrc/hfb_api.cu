@@ -69,20 +69,6 @@ std::string validateHair(const HfbHairData* h, uint32_t minPoints = 2, uint32_t 
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
-// A self-check's n counts: launch fills them on the device, and they come back to out.
-template <class Launch>
-int runCheck(HfbCtx* c, uint64_t* out, uint32_t n, const char* what, Launch launch) {
-  HFB_REQUIRE(c, out, "out is NULL");
-  unsigned long long* d = nullptr;
-  cudaError_t e = cudaMalloc(&d, n * sizeof(unsigned long long));
-  if (e != cudaSuccess) return cudaFail(c, e, what);
-  e = launch(d);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(out, d, n * sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  cudaFree(d);
-  return e == cudaSuccess ? HFB_OK : cudaFail(c, e, what);
-}
-
 }  // namespace
 
 namespace hfb {
@@ -176,20 +162,18 @@ int hfb_get_counters(HfbCtx* c, HfbCounters* out) {
 
 int hfb_check_constant_division(HfbCtx* c, uint64_t out[3]) {
   HFB_CHECK_CTX(c);
-  return runCheck(c, out, 3, "hfb_check_constant_division",
-                  [&](unsigned long long* d) { return hfb::launchConstDivCheck(c, d); });
-}
-
-int hfb_check_shared_quotients(HfbCtx* c, uint64_t out[4]) {
-  HFB_CHECK_CTX(c);
-  return runCheck(c, out, 4, "hfb_check_shared_quotients",
-                  [&](unsigned long long* d) { return hfb::launchQuotientCheck(c, d); });
-}
-
-int hfb_check_tone(HfbCtx* c, float power, uint64_t out[2]) {
-  HFB_CHECK_CTX(c);
-  return runCheck(c, out, 2, "hfb_check_tone",
-                  [&](unsigned long long* d) { return hfb::launchToneCheck(c, power, d); });
+  HFB_REQUIRE(c, out, "out is NULL");
+  unsigned long long* d = nullptr;
+  cudaError_t e = cudaMalloc(&d, 3 * sizeof(unsigned long long));
+  if (e != cudaSuccess) return cudaFail(c, e, "hfb_check_constant_division");
+  unsigned long long h[3] = {0, 0, 0};
+  e = hfb::launchConstDivCheck(c, d);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  cudaFree(d);
+  if (e != cudaSuccess) return cudaFail(c, e, "hfb_check_constant_division");
+  for (int i = 0; i < 3; i++) out[i] = h[i];
+  return HFB_OK;
 }
 
 int hfb_buffer_alloc(HfbCtx* c, size_t bytes, void** out) {
@@ -496,23 +480,14 @@ int hfb_hair_normals(HfbCtx* c, const HfbUniforms* u, const HfbHairData* h, cons
              "hair_normals");
 }
 
-static int gtaoImpl(HfbCtx* c, const HfbUniforms* u, const float* depth, const float* normals, float scale, float* ao,
-                    bool general) {
+int hfb_gtao(HfbCtx* c, const HfbUniforms* u, const float* depth, const float* normals, float scale, float* ao) {
   HFB_CHECK_CTX(c);
   HFB_REQUIRE(c, u && depth && normals && ao, "NULL argument");
   HFB_REQUIRE(c, scale > 0.0f && scale <= 1.0f, "scale must be in (0, 1]");
   HFB_REQUIRE(c, u->viewport.x >= 1.0f && u->viewport.y >= 1.0f && u->viewport.x <= 65536.0f &&
                      u->viewport.y <= 65536.0f, "the viewport must be in [1, 65536]");
   HFB_REQUIRE(c, u->ao.numDirections <= 64 && u->ao.numSteps <= 64, "numDirections and numSteps must be <= 64");
-  HFB_LAUNCH(c, hfb::launchGtao(c, *u, depth, normals, scale, ao, general), "gtao");
-}
-
-int hfb_gtao(HfbCtx* c, const HfbUniforms* u, const float* depth, const float* normals, float scale, float* ao) {
-  return gtaoImpl(c, u, depth, normals, scale, ao, false);
-}
-
-int hfb_check_gtao(HfbCtx* c, const HfbUniforms* u, const float* depth, const float* normals, float scale, float* ao) {
-  return gtaoImpl(c, u, depth, normals, scale, ao, true);
+  HFB_LAUNCH(c, hfb::launchGtao(c, *u, depth, normals, scale, ao), "gtao");
 }
 
 int hfb_present(HfbCtx* c, const HfbUniforms* u, const HfbRasterBuffers* rb, const float* scene, uint8_t* rgba) {

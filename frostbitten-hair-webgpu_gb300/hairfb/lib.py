@@ -86,8 +86,6 @@ SIGNATURES = {
     "hfb_sync": (I, [P]),
     "hfb_get_counters": (I, [P, P]),
     "hfb_check_constant_division": (I, [P, P]),
-    "hfb_check_shared_quotients": (I, [P, P]),
-    "hfb_check_tone": (I, [P, ctypes.c_float, P]),
     "hfb_buffer_alloc": (I, [P, SZ, P]),
     "hfb_buffer_free": (I, [P, P]),
     "hfb_buffer_upload": (I, [P, P, P, SZ]),
@@ -116,7 +114,6 @@ SIGNATURES = {
     "hfb_gtao": (I, [P, P, P, P, ctypes.c_float, P]),
     "hfb_frame": (I, [P, P]),
     "hfb_frame_batch": (I, [P, P, U32]),
-    "hfb_check_gtao": (I, [P, P, P, P, ctypes.c_float, P]),
     "hfb_frame_batch_profile": (I, [P, P, U32, P]),
     "hfb_ctx_set_batch_groups": (I, [P, U32]),
     "hfb_ctx_set_batch_pipeline": (I, [P, U32]),

@@ -198,21 +198,6 @@ HFB_API int hfb_get_counters(HfbCtx* ctx, HfbCounters* out);
  * int32 v, out[2] x / 1e6 over every finite float with |x| >= 2^-92.
  * Synchronizes. */
 HFB_API int hfb_check_constant_division(HfbCtx* ctx, uint64_t out[3]);
-/* Self-check of the quotients that the kernels form from a divisor's reciprocal
- * or from one approximate reciprocal root (simulation chains, hair depth, tiles
- * and fine passes), against the device's IEEE root and division, bit for bit:
- * for every float d, 16 numerators from a hash of d and 16 at the edges of the
- * forms' ranges.  Mismatch counts, all 0 expected: out[0] sqrt(d), out[1]
- * x / sqrt(d), out[2] x / d for |d| in [2^-25, 2^25] and x = 0 or |x| in
- * [2^-100, 2^102); out[3]: how many of out[1]'s quotients took the short form.
- * Synchronizes. */
-HFB_API int hfb_check_shared_quotients(HfbCtx* ctx, uint64_t out[4]);
-/* Self-check of the present pass's tone mapping: the bytes that its approximate
- * units decide, for every float as the exposed channel and the given power (1 /
- * gamma), against the exact operations: out[0] the bytes that differ (0
- * expected), out[1] how many of the values in [0, 16] were decided.
- * Synchronizes. */
-HFB_API int hfb_check_tone(HfbCtx* ctx, float power, uint64_t out[2]);
 
 /* ---- buffers ------------------------------------------------------------ */
 HFB_API int hfb_buffer_alloc(HfbCtx* ctx, size_t bytes, void** out);
@@ -424,10 +409,6 @@ HFB_API int hfb_frame(HfbCtx* ctx, HfbInstance* instance);
  * is a CUDA graph captured once per context, and the fine pass pulls the
  * tiles of all instances from one queue.  The context's config (tile size,
  * depth bins, slices, grid size) applies to every instance.  Results are
-/* The same by the kernel for any scale, without the shared tile that hfb_gtao uses
- * at scale 0.5: the two are equal bit for bit (a self-check). */
-HFB_API int hfb_check_gtao(HfbCtx* ctx, const HfbUniforms* uniforms, const float* depth, const float* normals,
-                           float scale, float* ao);
  * those of hfb_frame on each instance alone.  The call flips every
  * instance's `current`.  n <= 1024. */
 HFB_API int hfb_frame_batch(HfbCtx* ctx, HfbInstance* instances, uint32_t n);
