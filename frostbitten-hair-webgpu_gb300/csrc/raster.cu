@@ -167,8 +167,11 @@ __device__ __forceinline__ uint32_t blockExclusiveScan(uint32_t v, uint32_t* war
 //      the bin): the result does not depend on the order;
 //   E  one lane per (segment, tile): the record, as processTile stores it
 //      (:220-237).
-// A segment whose tiles do not fit the accumulators alone, or whose rectangle is
-// enormous, is walked by its own lane, tile by tile (rasterSegmentSerial).
+// A segment of more tiles than there are accumulators is walked by the warp, a tile per
+// lane (rasterSegmentTiles).  TR_SLOTS is the default of invalidTilesPerSegmentThreshold:
+// such segments exist above it only, and have kernels of their own (WIDE).  A draw of 20,000 x 3 at 4K with 8 px tiles,
+// a threshold of 1,024 and every 64th strand ten times as long: 906 us; with each such
+// segment walked by its own lane 1,523, with 768 accumulators per block of four warps 1,042.
 //
 // Bound by issue: an fp32 projection with IEEE roots and quotients per segment,
 // then what each row and each covered pixel costs.  Against edge tests of every
@@ -275,47 +278,66 @@ __device__ __forceinline__ void storeTileRecord(uint4* __restrict__ tiles, uint3
   }
 }
 
-// processTile for every tile of one segment's tile range, by one thread.
-__device__ void rasterSegmentSerial(const HfbUniforms& U, const ProjSeg& s, uint32_t W, uint32_t H, uint32_t TS,
-                                    uint32_t B, uint32_t tilesX, uint32_t maxDrawn, float dv0, float dv1,
-                                    uint32_t key, uint32_t ux0, uint32_t uy0, uint32_t ux1, uint32_t uy1,
-                                    const float* __restrict__ depth, uint4* __restrict__ tiles,
-                                    uint32_t* __restrict__ segBuf, uint32_t* __restrict__ segCount,
-                                    uint32_t* __restrict__ binCount, DeviceCounters* __restrict__ counters) {
-  const uint32_t tminx = ux0 / TS, tminy = uy0 / TS, tmaxx = ux1 / TS, tmaxy = uy1 / TS;
+// getRasterizedHairBounds, swRasterizeHair.wgsl.ts:111-124: x0, y0, x1, y1
+__device__ __forceinline__ uint4 segmentBounds(const ProjSeg& s, f2 size) {
+  const float bx1 = fminf(ceilf(fmaxf(fmaxf(s.v00.x, s.v01.x), fmaxf(s.v10.x, s.v11.x))), size.x);
+  const float by1 = fminf(ceilf(fmaxf(fmaxf(s.v00.y, s.v01.y), fmaxf(s.v10.y, s.v11.y))), size.y);
+  const float bx0 = fmaxf(floorf(fminf(fminf(s.v00.x, s.v01.x), fminf(s.v10.x, s.v11.x))), 0.0f);
+  const float by0 = fmaxf(floorf(fminf(fminf(s.v00.y, s.v01.y), fminf(s.v10.y, s.v11.y))), 0.0f);
+  return make_uint4(f2u(bx0), f2u(by0), f2u(bx1), f2u(by1));
+}
+
+// processTile for every tile of segment gid's tile range, by a warp: lane l takes the
+// range's tiles l, l + 32, ... in row-major order.  Projects the segment again: rare, and
+// the ordinary segments' rounds then have nothing of it to keep.
+// Inlined: U may be a kernel parameter, whose address no function may take.
+__device__ __forceinline__ void rasterSegmentTiles(const HfbUniforms& U, uint32_t P, uint32_t gid, uint32_t TS,
+                                                   uint32_t B, float dv0, float dv1, uint32_t lane,
+                                                   const float4* __restrict__ pos, const float4* __restrict__ tan,
+                                                   const float* __restrict__ depth, uint4* __restrict__ tiles,
+                                                   uint32_t* __restrict__ segBuf, uint32_t* __restrict__ segCount,
+                                                   uint32_t* __restrict__ binCount,
+                                                   DeviceCounters* __restrict__ counters) {
+  const f2 size = mk2(U.viewport.x, U.viewport.y);
+  const uint32_t W = f2u(size.x), H = f2u(size.y), tilesX = divCeil(W, TS), maxDrawn = U.maxDrawnHairSegments;
+  const uint32_t strand = gid / (P - 1u), seg = gid - strand * (P - 1u), key = (strand << 8) | seg;
+  const ProjSeg s = projectSegment(U, pos, tan, P, strand, seg, size);
+  const uint4 u = segmentBounds(s, size);
+  const uint32_t tminx = u.x / TS, tminy = u.y / TS, tsx = u.z / TS - tminx + 1u, n = tsx * (u.w / TS - tminy + 1u);
   const RowSpan span = makeRowSpan(s);
-  for (uint32_t ty = tminy; ty <= tmaxy; ty++) {
-    for (uint32_t tx = tminx; tx <= tmaxx; tx++) {
-      TileB tb = tileBoundsPx(W, H, TS, tx, ty);
-      // Only pixel corners inside the segment's bounding rectangle can pass
-      // the four edge tests, so the walk is restricted to tile x rect, and
-      // per row to the candidate span around the covered interval.
-      const uint32_t xa = max(tb.x0, ux0), xb = min(tb.x1, ux1 + 1u);
-      const uint32_t ya = max(tb.y0, uy0), yb = min(tb.y1, uy1 + 1u);
-      float dmin = 999.0f, dmax = -999.0f;
-      uint32_t dbin = B;
-      for (uint32_t y = ya; y < yb; y++) {
-        uint32_t x0r = xa, x1r = xb;
-        span.candidates((float)y, x0r, x1r);
-        for (uint32_t x = x0r; x < x1r; x++) {
-          f2 p = mk2((float)x, (float)y);
-          if (!insideQuad(s, p)) continue;
-          f2 w = interpolateHairQuad(s, p);
-          float hd = interpolateHairF32(w, s.depthsProj);
-          float zb = loadTex2DClamp(depth, W, H, (int)x, (int)H - (int)y);
-          if (hd > zb) continue;  // depth test, :193-195
-          dmin = fminf(dmin, hd);
-          dmax = fmaxf(dmax, hd);
-          dbin = min(dbin, viewDepthBin(U, B, dv0, dv1, p, hd));
-        }
+  for (uint32_t i = lane; i < n; i += 32u) {
+    const uint32_t ty = tminy + i / tsx, tx = tminx + i % tsx;
+    TileB tb = tileBoundsPx(W, H, TS, tx, ty);
+    // Only pixel corners inside the segment's bounding rectangle can pass
+    // the four edge tests, so the walk is restricted to tile x rect, and
+    // per row to the candidate span around the covered interval.
+    const uint32_t xa = max(tb.x0, u.x), xb = min(tb.x1, u.z + 1u);
+    const uint32_t ya = max(tb.y0, u.y), yb = min(tb.y1, u.w + 1u);
+    float dmin = 999.0f, dmax = -999.0f;
+    uint32_t dbin = B;
+    for (uint32_t y = ya; y < yb; y++) {
+      uint32_t x0r = xa, x1r = xb;
+      span.candidates((float)y, x0r, x1r);
+      for (uint32_t x = x0r; x < x1r; x++) {
+        f2 p = mk2((float)x, (float)y);
+        if (!insideQuad(s, p)) continue;
+        f2 w = interpolateHairQuad(s, p);
+        float hd = interpolateHairF32(w, s.depthsProj);
+        float zb = loadTex2DClamp(depth, W, H, (int)x, (int)H - (int)y);
+        if (hd > zb) continue;  // depth test, :193-195
+        dmin = fminf(dmin, hd);
+        dmax = fmaxf(dmax, hd);
+        dbin = min(dbin, viewDepthBin(U, B, dv0, dv1, p, hd));
       }
-      if (dmin > 1.0f) continue;
-      storeTileRecord(tiles, segBuf, segCount, binCount, counters, maxDrawn, tilesX, B, tx, ty, dbin, dmin, dmax,
-                      key, tilesX * divCeil(H, TS));
     }
+    if (dmin > 1.0f) continue;
+    storeTileRecord(tiles, segBuf, segCount, binCount, counters, maxDrawn, tilesX, B, tx, ty, dbin, dmin, dmax, key,
+                    tilesX * divCeil(H, TS));
   }
 }
 
+// WIDE: the threshold lets segments of more than TR_SLOTS tiles through.
+template <bool WIDE>
 __device__ __forceinline__ void tilesRasterBody(const HfbUniforms& U, uint32_t P, uint32_t nStrands, uint32_t TS,
                                                 uint32_t B, uint32_t threshold, float4 bsphere,
                                                 const float4* __restrict__ pos, const float4* __restrict__ tan,
@@ -342,34 +364,28 @@ __device__ __forceinline__ void tilesRasterBody(const HfbUniforms& U, uint32_t P
 
   // ---- project this lane's segment ----
   uint32_t rows = 0, slots = 0, key = 0;
-  bool serial = false;
-  ProjSeg s;
-  uint32_t ux0 = 0, uy0 = 0, ux1 = 0, uy1 = 0;
+  bool wide = false;
   if (gid < nSeg) {
     const uint32_t strand = gid / segsPerStrand, seg = gid - strand * segsPerStrand;
     key = (strand << 8) | seg;
-    s = projectSegment(U, pos, tan, P, strand, seg, size);
+    const ProjSeg s = projectSegment(U, pos, tan, P, strand, seg, size);
     if (projOut) {  // for the fine pass of the same frame
       float4* o = projOut + (size_t)gid * SEG_PROJ_VEC4;
       o[0] = make_float4(s.v00.x, s.v00.y, s.v01.x, s.v01.y);
       o[1] = make_float4(s.v10.x, s.v10.y, s.v11.x, s.v11.y);
       o[2] = make_float4(s.depthsProj.x, s.depthsProj.y, s.depthsProj.z, s.depthsProj.w);
     }
-    // getRasterizedHairBounds, swRasterizeHair.wgsl.ts:111-124
-    const float bx1 = fminf(ceilf(fmaxf(fmaxf(s.v00.x, s.v01.x), fmaxf(s.v10.x, s.v11.x))), size.x);
-    const float by1 = fminf(ceilf(fmaxf(fmaxf(s.v00.y, s.v01.y), fmaxf(s.v10.y, s.v11.y))), size.y);
-    const float bx0 = fmaxf(floorf(fminf(fminf(s.v00.x, s.v01.x), fminf(s.v10.x, s.v11.x))), 0.0f);
-    const float by0 = fmaxf(floorf(fminf(fminf(s.v00.y, s.v01.y), fminf(s.v10.y, s.v11.y))), 0.0f);
-    ux0 = f2u(bx0); uy0 = f2u(by0); ux1 = f2u(bx1); uy1 = f2u(by1);
+    const uint4 ub = segmentBounds(s, size);
+    const uint32_t ux0 = ub.x, uy0 = ub.y, ux1 = ub.z, uy1 = ub.w;
     const uint32_t tminx = ux0 >> tsShift, tminy = uy0 >> tsShift, tmaxx = ux1 >> tsShift, tmaxy = uy1 >> tsShift;
     const uint32_t tsx = (tmaxx - tminx) + 1u, tsy = (tmaxy - tminy) + 1u;
     if (tsx * tsy <= threshold) {  // degenerate segment rejection, :111-117
       const uint32_t cx1 = min(ux1 + 1u, W - 1u), cy1 = min(uy1 + 1u, H - 1u);
       const uint32_t cwid = cx1 > ux0 ? cx1 - ux0 : 0u, chei = cy1 > uy0 ? cy1 - uy0 : 0u;
       if (cwid && chei) {
-        if (cwid > 4096u || chei > 4096u || tsx * tsy > TR_SLOTS) {
-          serial = true;  // its own walk
-        } else {
+        if (WIDE && tsx * tsy > TR_SLOTS) {
+          wide = true;  // walked by the whole warp
+        } else {  // at most TR_SLOTS tiles of 32 px either way: 4,096 rows and columns
           rows = chei;
           slots = tsx * tsy;
         }
@@ -495,11 +511,16 @@ __device__ __forceinline__ void tilesRasterBody(const HfbUniforms& U, uint32_t P
     __syncwarp();  // the accumulators are reused by the next round
     first = end;
   }
-  if (serial)
-    rasterSegmentSerial(U, s, W, H, TS, B, tilesX, maxDrawn, dv0, dv1, key, ux0, uy0, ux1, uy1, depth, tiles,
-                        segBuf, segCount, binCount, counters);
+  if constexpr (WIDE) {
+    for (uint32_t m = __ballot_sync(0xffffffffu, wide); m; m &= m - 1u) {
+      rasterSegmentTiles(U, P, blk * TR_SEGS + w0 + (uint32_t)__ffs(m) - 1u, TS, B, dv0, dv1, lane, pos, tan, depth,
+                         tiles, segBuf, segCount, binCount, counters);
+      __syncwarp();
+    }
+  }
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(TR_SEGS, 6)
 tilesRasterKernel(const HfbUniforms U, uint32_t P, uint32_t nStrands, uint32_t TS, uint32_t B,
                   uint32_t threshold, float4 bsphere, const float4* __restrict__ pos,
@@ -507,9 +528,12 @@ tilesRasterKernel(const HfbUniforms U, uint32_t P, uint32_t nStrands, uint32_t T
                   uint32_t* __restrict__ segBuf, uint32_t* __restrict__ segCount,
                   uint32_t* __restrict__ binCount, DeviceCounters* __restrict__ counters, float4* __restrict__ proj) {
   __shared__ TrShared sh;
-  tilesRasterBody(U, P, nStrands, TS, B, threshold, bsphere, pos, tan, depth, tiles, segBuf, segCount, binCount,
-                  counters, sh, blockIdx.x, proj);
+  tilesRasterBody<WIDE>(U, P, nStrands, TS, B, threshold, bsphere, pos, tan, depth, tiles, segBuf, segCount, binCount,
+                        counters, sh, blockIdx.x, proj);
 }
+
+// Whether some segment can need rasterSegmentTiles.
+bool rasterWide(const HfbConfig& cfg) { return cfg.invalidTilesPerSegmentThreshold > TR_SLOTS; }
 
 // ---------------------------------------------------------------------------
 // 2. binScan: exclusive prefix over T*B counts (block-local + block sums)
@@ -2606,12 +2630,13 @@ cudaError_t launchFineT(HfbCtx* c, const HfbUniforms& u, const HfbHairData& h, c
     const TilesScratch ts = tilesScratchLayout(I.scratch, cfg, I.W, I.H, I.maxDrawn); \
     (void)ts;
 
+template <bool WIDE>
 __global__ void __launch_bounds__(TR_SEGS, 6) tilesRasterBatch(BatchView b, HfbConfig cfgParam,
                                                              DeviceCounters* __restrict__ counters) {
   const HfbConfig cfg = cfgParam;
   __shared__ TrShared sh;
   BATCH_LOOP(BK_RASTER)
-    tilesRasterBody(I.U, I.P, min(I.strandsToRender, I.S), cfg.tileSize, cfg.tileDepthBins,
+    tilesRasterBody<WIDE>(I.U, I.P, min(I.strandsToRender, I.S), cfg.tileSize, cfg.tileDepthBins,
                     cfg.invalidTilesPerSegmentThreshold, I.bsphere, I.posNew, I.tan, I.depth, I.tiles, I.segBuf,
                     I.segCount, ts.binCount, counters, sh, local, I.proj);
   }
@@ -2766,7 +2791,7 @@ cudaError_t launchTilesPass(HfbCtx* c, const HfbUniforms& u, const HfbHairData& 
   DeviceCounters* dc = (DeviceCounters*)c->dCounters;
   if (nSeg) {
     float4 bs = make_float4(h.boundingSphere[0], h.boundingSphere[1], h.boundingSphere[2], h.boundingSphere[3]);
-    tilesRasterKernel<<<divCeil(nSeg, TR_SEGS), TR_SEGS, 0, c->stream>>>(
+    (rasterWide(cfg) ? tilesRasterKernel<true> : tilesRasterKernel<false>)<<<divCeil(nSeg, TR_SEGS), TR_SEGS, 0, c->stream>>>(
         u, h.pointsPerStrand, nStrands, TS, B, cfg.invalidTilesPerSegmentThreshold, bs, (const float4*)pos,
         (const float4*)tan, depth, (uint4*)rb.tiles, rb.tileSegments, rb.segmentCountPerTile, s.binCount, dc, proj);
     HFB_AFTER_LAUNCH(c, "tilesRasterKernel");
@@ -2801,7 +2826,7 @@ cudaError_t launchTilesPass(HfbCtx* c, const HfbUniforms& u, const HfbHairData& 
 // context creation so that its own launches load (allocate) nothing.
 cudaError_t tilesPassLoad(HfbCtx* c) {
   cudaFuncAttributes a;
-  cudaError_t e = cudaFuncGetAttributes(&a, tilesRasterKernel);
+  cudaError_t e = cudaFuncGetAttributes(&a, rasterWide(c->cfg) ? tilesRasterKernel<true> : tilesRasterKernel<false>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, binScanKernel);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, binScatterKernel);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, binFinalizeKernel);
@@ -2853,9 +2878,10 @@ cudaError_t launchBatchTiles(HfbCtx* c, const BatchView& b) {
   const HfbConfig& cfg = c->cfg;
   DeviceCounters* dc = (DeviceCounters*)c->dCounters;
   uint32_t* g = c->batchGrid;
+  const auto raster = rasterWide(cfg) ? tilesRasterBatch<true> : tilesRasterBatch<false>;
   if (!g[BK_RASTER]) {
     int per = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, tilesRasterBatch, TR_SEGS, 0);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, raster, TR_SEGS, 0);
     if (e != cudaSuccess) return e;
     g[BK_RASTER] = (uint32_t)(per > 0 ? per : 1) * c->smCount;
     g[BK_SCAN] = c->smCount * 4u;
@@ -2866,7 +2892,7 @@ cudaError_t launchBatchTiles(HfbCtx* c, const BatchView& b) {
     e = cudaFuncSetAttribute(largeBinsBatch, cudaFuncAttributeMaxDynamicSharedMemorySize, LARGE_SMEM_KEYS * 4);
     if (e != cudaSuccess) return e;
   }
-  tilesRasterBatch<<<batchLaunchGrid(c, g[BK_RASTER]), TR_SEGS, 0, c->stream>>>(b, cfg, dc);
+  raster<<<batchLaunchGrid(c, g[BK_RASTER]), TR_SEGS, 0, c->stream>>>(b, cfg, dc);
   HFB_AFTER_LAUNCH(c, "tilesRasterBatch");
   if (c->rasterDone) {
     const cudaError_t e = cudaEventRecord(c->rasterDone, c->stream);

@@ -12,6 +12,7 @@ torch = pytest.importorskip("torch")
 if not torch.cuda.is_available():
     pytest.skip("needs a CUDA GPU", allow_module_level=True)
 
+from hairfb import hair_object as HO  # noqa: E402
 from hairfb.passes import HairObject, HwHairPass, RasterBuffers  # noqa: E402
 from test_gpu_parity import _compare_tiles, _ctx, _fine_vs_oracle, _raster_gpu, oracle  # noqa: E402,F401
 
@@ -78,3 +79,43 @@ def test_hair_depth_segments_of_every_size_bit_exact(oracle, points, fiber, size
     g = out.cpu().numpy()
     assert (g < inst.scene_depth).sum() > 20, "little hair in front: the test does not test"
     assert np.array_equal(g.view(np.uint32), o.view(np.uint32))
+
+
+def _with_long_strands(strands, points, size, tile, fiber, longer, threshold):
+    """Every other strand `longer` times as long."""
+    inst = small_instance(strands=strands, points=points, width=size[0], height=size[1], tile_size=tile,
+                          fiber_radius=fiber, avg_segments_per_tile=512)
+    p = inst.hair.asset.positions.reshape(strands, points, 4)
+    p[::2, :, :3] = p[::2, :1, :3] + longer * (p[::2, :, :3] - p[::2, :1, :3])
+    inst.hair = HO.build_hair_buffers(inst.hair.asset)
+    inst.cfg.invalid_tiles_per_segment_threshold = threshold
+    return inst
+
+
+@pytest.mark.parametrize("tile,size,fiber,longer", [(8, (2900, 1700), 5e-4, 8), (16, (2901, 1697), 5e-4, 12),
+                                                    (8, (2160, 1440), 2e-2, 6), (32, (9000, 1200), 5e-4, 300)])
+@pytest.mark.parametrize("threshold", [128, 700, 100000])
+def test_tiles_pass_segments_past_the_accumulators_bit_exact(oracle, tile, size, fiber, longer, threshold):  # noqa: F811
+    """Segments of more tiles than a warp has accumulators, which a threshold above the default lets
+    through, some longer than the spans' range, among ordinary ones."""
+    inst = _with_long_strands(90, 3, size, tile, fiber, longer, threshold)
+    fr = frame_of(inst)
+    ctx, hair, rb, d = _raster_gpu(inst, fr)
+    _, osg, _ = _compare_tiles(oracle, inst, fr, rb)
+    if threshold > 128:
+        inst = _with_long_strands(90, 3, size, tile, fiber, longer, 128)
+        _, rb128 = _raster_gpu(inst, frame_of(inst))[1:3]
+        assert osg[0] > rb128.read_tile_segments()[0], "no segment past the default threshold: the test does not test"
+
+
+@pytest.mark.parametrize("tile,slices", [(8, 4), (16, 8), (32, 4)])
+def test_fine_pass_segments_longer_than_the_spans_range(oracle, tile, slices):  # noqa: F811
+    """A viewport and segments above 8,192 px: rows whose edges are out of the spans' range keep the
+    whole box."""
+    inst = _with_long_strands(60, 3, (9000, 1200), tile, 2e-3, 300, 1 << 20)
+    inst.cfg.slices_per_pixel = slices
+    cnt, g, o = _fine_vs_oracle(oracle, inst)
+    err = np.abs(g - o)
+    assert err.max() <= 1.0 / 255.0, f"max pixel error {err.max():.4g} (> 1/255)"
+    assert np.array_equal(g[:, 3] > 0, o[:, 3] > 0), "coverage differs"
+    assert (o[:, 3] > 0).sum() > 5000
