@@ -144,6 +144,12 @@ cudaError_t framePass(HfbCtx* c, HfbInstance* in, FramePass p) {
 // may not run beside the tiles and fine passes where they read what it writes: a
 // frame whose hairDepth overlaps a sceneDepth keeps everything in turn on the
 // caller's stream.
+//
+// A batch of one group does so at every size, although its persistent kernels fill the GPU
+// by themselves: each pass's tail is filled by the others.  In turn against forked, from 0.5 to 121
+// integration blocks per SM: ticks of 2, 6, 24 and 96 sessions 420 -> 314 us, 1,276 -> 1,155,
+// 4,241 -> 4,098, 17,650 -> 17,400; 4, 16, 64 and 128 instances of the 64-instance mix 1,088 ->
+// 977 us, 2,683 -> 2,535, 11,750 -> 11,560, 20,810 -> 20,600; 256 small ones 5,995 -> 5,875.
 // ---------------------------------------------------------------------------
 enum SideEvent : uint32_t { SE_START = 0, SE_CLEAR, SE_SIM, SE_RASTER, SE_SORT, SE_DONE };
 static_assert(SE_DONE + 1 == SIDE_EVENTS, "an event each");
@@ -693,11 +699,8 @@ cudaError_t frameBatch(HfbCtx* c, HfbInstance* insts, uint32_t n, float* passMs)
   // the frame's projected segments: one region per instance, written by the
   // tiles pass and read by the fine pass
   size_t segs = 0;
-  uint64_t strands = 0, fullBlocks = 0;
-  for (uint32_t i = 0; i < n; i++) {
-    strands += insts[i].hair.strandsCount;
-    fullBlocks += divCeil(insts[i].hair.strandsCount, simStrandsPerBlock(insts[i].hair.pointsPerStrand));
-  }
+  uint64_t strands = 0;
+  for (uint32_t i = 0; i < n; i++) strands += insts[i].hair.strandsCount;
   for (uint32_t i = 0; i < n; i++) segs += (size_t)insts[i].hair.strandsCount * (insts[i].hair.pointsPerStrand - 1u);
   e = ensureProjCache(c, segs);
   if (e != cudaSuccess) { delete[] group; return e; }
@@ -793,8 +796,7 @@ cudaError_t frameBatch(HfbCtx* c, HfbInstance* insts, uint32_t n, float* passMs)
 #ifdef HFB_DEVICE_CHECKS
   c->batchNoGraph = true;  // the checked build waits after every launch: no capture
 #endif
-  const bool side = NG == 1u && c->sideStream && fullBlocks <= (uint64_t)SIDE_MAX_BLOCKS * c->smCount &&
-                    !depthsOverlap(insts, n);
+  const bool side = NG == 1u && c->sideStream && !depthsOverlap(insts, n);
   cudaGraphExec_t& graph = c->batchGraph[side ? 1 : 0];
   uint64_t& graphLaunches = c->batchGraphLaunches[side ? 1 : 0];
   if (!side && graph && c->batchGraphGroups != NG) {  // made for another number of groups

@@ -131,13 +131,6 @@ __host__ __device__ inline uint32_t simStrandsPerBlockFor(uint32_t S, uint32_t P
 // batch does not give every SM its SIM_BATCH_BLOCKS of them, down to 8 strands, so that
 // they take one wave: a tick of 6 sessions (35,000 strands of 32) 382 -> 308 us.
 constexpr uint32_t SIM_BATCH_BLOCKS = 7;
-// Integration blocks (full ones) per SM up to which a batch runs its side passes on the
-// side stream: measured on batches of the 64-instance mix and of sessions, 3 sessions 690
-// -> 618 us, 6 1,348 -> 1,250, 16 instances (13 blocks per SM) 2,914 -> 2,887, 24 (25)
-// 5,015 -> 4,974; from there on the persistent kernels fill the GPU by themselves and get
-// in one another's way (48 sessions, 36 per SM: 8,412 -> 8,556; 64 instances, 67: 12.39 ->
-// 12.74 ms).
-constexpr uint32_t SIDE_MAX_BLOCKS = 21;
 inline uint32_t simStrandsForBatch(uint64_t S, uint32_t P, uint32_t smCount) {
   const uint32_t full = simStrandsPerBlock(P);
   const uint64_t want = (S + SIM_BATCH_BLOCKS * smCount - 1u) / (SIM_BATCH_BLOCKS * smCount) + 1u;  // + 1: partial blocks

@@ -90,3 +90,69 @@ def test_batch_with_another_instances_depth():
             for k in (0, 1, 4, 5):  # positions, grids, tile depths, counts
                 assert np.array_equal(a[k], b[k])
     assert np.array_equal(_state(got[0])[0][3], _state(want[0])[0][3])
+
+
+@pytest.mark.parametrize("batch", [1, 3])
+def test_frames_on_changing_streams(batch):
+    """Each frame on another stream than the last, the streams ordered by the caller: the work on the
+    context's own second stream is joined into the stream that the frame was given."""
+    inst = small_instance()
+    ctx = Context(inst.cfg.to_c(), 0)
+    got = [_renderer(k, ctx, False) for k in range(batch)]
+    plain = Context(inst.cfg.to_c(), 0)
+    want = [_renderer(k, plain, False) for k in range(batch)]
+    torch.cuda.synchronize()
+    for r in got + want:
+        r.before_first_frame()
+    torch.cuda.synchronize()
+    many = BatchRenderer(got)
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    for f in range(7):
+        s = streams[f % 3]
+        s.wait_stream(streams[(f - 1) % 3])
+        ctx.set_stream(s)
+        many.frame() if batch > 1 else got[0].frame_native()
+        for r in want:
+            r.frame()
+    torch.cuda.synchronize()
+    for g, w in zip(got, want):
+        (gs, gi), (ws, wi) = _state(g), _state(w)
+        for a, b in zip(gs, ws):
+            assert np.array_equal(a, b)
+        assert np.abs(gi - wi).max() <= 1.0 / 255.0
+
+
+def test_frames_captured_by_the_caller():
+    """Two frames in a graph of the caller's: nothing runs while they are captured, and a launch of the
+    graph gives the two frames."""
+    inst = small_instance()
+    s = torch.cuda.Stream()
+    ctx = Context(inst.cfg.to_c(), 0)
+    ctx.set_stream(s)
+    first, got = _renderer(1, ctx, False), _renderer(1, ctx, False)
+    plain = Context(inst.cfg.to_c(), 0)
+    want = _renderer(1, plain, False)
+    torch.cuda.synchronize()
+    for r in (first, got, want):
+        r.before_first_frame()
+    first.frame_native()  # the context's buffers grow to these frames' sizes
+    torch.cuda.synchronize()
+    before = _state(got)[0]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s, capture_error_mode="thread_local"):
+        got.frame_native()
+        got.frame_native()
+    for a, b in zip(before, _state(got)[0]):
+        assert np.array_equal(a, b)
+    with torch.cuda.stream(s):
+        graph.replay()
+    want.frame()
+    want.frame()
+    (gs, gi), (ws, wi) = _state(got), _state(want)
+    for a, b in zip(gs, ws):
+        assert np.array_equal(a, b)
+    assert np.abs(gi - wi).max() <= 1.0 / 255.0
+    got.frame_native()  # the context's streams are as they were
+    want.frame()
+    for a, b in zip(_state(got)[0], _state(want)[0]):
+        assert np.array_equal(a, b)
