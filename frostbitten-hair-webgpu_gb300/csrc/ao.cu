@@ -1,7 +1,7 @@
 // GTAO: AoPass (aoPass.wgsl.ts main_fs, gtao.wgsl.ts) as CUDA.
 //
-// One thread per AO texel (the AO texture is the viewport times the
-// reference's textureSizeMul, 0.5): the texel's full-resolution position
+// Per AO texel (the AO texture is the viewport times the reference's
+// textureSizeMul, 0.5; at that scale four threads, else one): the texel's full-resolution position
 // ((x + 0.5) / scale), the normal there (rg16float octahedron, decoded as
 // decodeOctahedronNormal does), and gtao(): for each of numDirections
 // directions, numSteps steps each way, every sample reprojected to view
@@ -95,7 +95,7 @@ __device__ __forceinline__ void gtao(const HfbUniforms& U, const AoCtx& a, float
       fmul(AO_PI, fractf(fmul(52.9829189f, fractf(fadd(fmul(px, 0.06711056f), fmul(py, 0.00583715f))))));
   const float jitterMod = fmul(fadd(px, py), 0.25f);
   const float radiusJitter = fmul(fmul(fractf(jitterMod), stepSize), 0.25f);
-  // gtaoFalloff's divisor is the same for every sample (divBy, where its range allows)
+  // gtaoFalloff's divisor is the same for every sample (divBy on the tile, where its range allows)
   const float s2 = P.falloffStart2, fd = fsub(P.falloffEnd2, s2);
   const Recip fr = s2 >= 1e-6f && s2 <= 1e6f ? recipOf(fd) : Recip{fd, __int_as_float(0x7fffffff)};
   auto horizon = [&](f3 s, float h) {
@@ -103,8 +103,13 @@ __device__ __forceinline__ void gtao(const HfbUniforms& U, const AoCtx& a, float
     const float d2 = len3(ws);
     const float c = fmul(dot3(ws, toCam), rsqrtf(d2));
     const float n = fsub(d2, s2);
-    float q = divBy(n, fr);
-    if (!(fabsf(q) < 1e30f)) q = n / fd;
+    float q;
+    if constexpr (TILE) {
+      q = divBy(n, fr);
+      if (!(fabsf(q) < 1e30f)) q = n / fd;
+    } else {  // hidden behind a sample's reprojection: 33 directions at 1080p 1,446 us, by divBy 1,456
+      q = n / fd;
+    }
     return fmaxf(h, fsub(c, fmul(2.0f, sat(q))));
   };
   for (uint32_t i = i0; i < i1; i++) {
@@ -241,13 +246,13 @@ gtaoTileKernel(const HfbUniforms U, const float* __restrict__ depth, const float
 uint32_t aoExtent(float viewport, float scale) { return (uint32_t)ceilf(viewport * scale); }
 
 cudaError_t launchGtao(HfbCtx* c, const HfbUniforms& u, const float* depth, const float* normals, float scale,
-                       float* ao) {
+                       float* ao, bool general) {
   HFB_CHECK_BIND(c);
   const uint32_t aoW = aoExtent(u.viewport.x, scale), aoH = aoExtent(u.viewport.y, scale);
   const uint32_t n = aoW * aoH;
   if (n == 0) return cudaSuccess;
   const uint32_t by = divCeil(aoH, AO_BY);
-  if (scale == 0.5f && by <= 65535u && u.ao.numDirections <= AO_SPLIT * AO_TERMS) {
+  if (!general && scale == 0.5f && by <= 65535u && u.ao.numDirections <= AO_SPLIT * AO_TERMS) {
     gtaoTileKernel<<<dim3(divCeil(aoW, AO_BX), by), AO_THREADS, 0, c->stream>>>(u, depth, (const float2*)normals, aoW,
                                                                                 aoH, ao);
     HFB_AFTER_LAUNCH(c, "gtaoTileKernel");

@@ -480,14 +480,23 @@ int hfb_hair_normals(HfbCtx* c, const HfbUniforms* u, const HfbHairData* h, cons
              "hair_normals");
 }
 
-int hfb_gtao(HfbCtx* c, const HfbUniforms* u, const float* depth, const float* normals, float scale, float* ao) {
+static int gtaoImpl(HfbCtx* c, const HfbUniforms* u, const float* depth, const float* normals, float scale, float* ao,
+                    bool general) {
   HFB_CHECK_CTX(c);
   HFB_REQUIRE(c, u && depth && normals && ao, "NULL argument");
   HFB_REQUIRE(c, scale > 0.0f && scale <= 1.0f, "scale must be in (0, 1]");
   HFB_REQUIRE(c, u->viewport.x >= 1.0f && u->viewport.y >= 1.0f && u->viewport.x <= 65536.0f &&
                      u->viewport.y <= 65536.0f, "the viewport must be in [1, 65536]");
   HFB_REQUIRE(c, u->ao.numDirections <= 64 && u->ao.numSteps <= 64, "numDirections and numSteps must be <= 64");
-  HFB_LAUNCH(c, hfb::launchGtao(c, *u, depth, normals, scale, ao), "gtao");
+  HFB_LAUNCH(c, hfb::launchGtao(c, *u, depth, normals, scale, ao, general), "gtao");
+}
+
+int hfb_gtao(HfbCtx* c, const HfbUniforms* u, const float* depth, const float* normals, float scale, float* ao) {
+  return gtaoImpl(c, u, depth, normals, scale, ao, false);
+}
+
+int hfb_check_gtao(HfbCtx* c, const HfbUniforms* u, const float* depth, const float* normals, float scale, float* ao) {
+  return gtaoImpl(c, u, depth, normals, scale, ao, true);
 }
 
 int hfb_present(HfbCtx* c, const HfbUniforms* u, const HfbRasterBuffers* rb, const float* scene, uint8_t* rgba) {

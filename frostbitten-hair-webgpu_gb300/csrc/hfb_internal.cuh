@@ -385,8 +385,9 @@ cudaError_t launchHairNormals(HfbCtx* c, const HfbUniforms& u, const HfbHairData
                               HfbRasterBuffers& rb);
 // AO texture extent: ceil(viewport * scale), as the reference sizes it (renderer.ts:405-409).
 uint32_t aoExtent(float viewport, float scale);
+// general: by the kernel for any scale, also at 0.5
 cudaError_t launchGtao(HfbCtx* c, const HfbUniforms& u, const float* depth, const float* normals, float scale,
-                       float* ao);
+                       float* ao, bool general = false);
 cudaError_t launchPresent(HfbCtx* c, const HfbUniforms& u, uint32_t W, uint32_t H, const float* result,
                           const float* scene, uint8_t* rgba);
 cudaError_t launchPresentBatch(HfbCtx* c, const HfbPresentItem* items, uint32_t n);

@@ -394,6 +394,10 @@ HFB_API int hfb_hair_normals(HfbCtx* ctx, const HfbUniforms* uniforms, const Hfb
  * The shading reads it (hfb_shading's ao, aoWidth, aoHeight). */
 HFB_API int hfb_gtao(HfbCtx* ctx, const HfbUniforms* uniforms, const float* depth, const float* normals, float scale,
                      float* ao);
+/* The same by the kernel for any scale, without the shared tile that hfb_gtao uses
+ * at scale 0.5: the two are equal bit for bit (a self-check). */
+HFB_API int hfb_check_gtao(HfbCtx* ctx, const HfbUniforms* uniforms, const float* depth, const float* normals,
+                           float scale, float* ao);
 
 HFB_API int hfb_hair_depth(HfbCtx* ctx, const HfbUniforms* uniforms, const HfbHairData* hair, const float* positions,
                            const float* tangents, uint32_t strandsToRender, const float* sceneDepth,
