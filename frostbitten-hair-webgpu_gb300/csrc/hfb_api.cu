@@ -69,6 +69,20 @@ std::string validateHair(const HfbHairData* h, uint32_t minPoints = 2, uint32_t 
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
+// A self-check's n counts: launch fills them on the device, and they come back to out.
+template <class Launch>
+int runCheck(HfbCtx* c, uint64_t* out, uint32_t n, const char* what, Launch launch) {
+  HFB_REQUIRE(c, out, "out is NULL");
+  unsigned long long* d = nullptr;
+  cudaError_t e = cudaMalloc(&d, n * sizeof(unsigned long long));
+  if (e != cudaSuccess) return cudaFail(c, e, what);
+  e = launch(d);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(out, d, n * sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  cudaFree(d);
+  return e == cudaSuccess ? HFB_OK : cudaFail(c, e, what);
+}
+
 }  // namespace
 
 namespace hfb {
@@ -162,18 +176,14 @@ int hfb_get_counters(HfbCtx* c, HfbCounters* out) {
 
 int hfb_check_constant_division(HfbCtx* c, uint64_t out[3]) {
   HFB_CHECK_CTX(c);
-  HFB_REQUIRE(c, out, "out is NULL");
-  unsigned long long* d = nullptr;
-  cudaError_t e = cudaMalloc(&d, 3 * sizeof(unsigned long long));
-  if (e != cudaSuccess) return cudaFail(c, e, "hfb_check_constant_division");
-  unsigned long long h[3] = {0, 0, 0};
-  e = hfb::launchConstDivCheck(c, d);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  cudaFree(d);
-  if (e != cudaSuccess) return cudaFail(c, e, "hfb_check_constant_division");
-  for (int i = 0; i < 3; i++) out[i] = h[i];
-  return HFB_OK;
+  return runCheck(c, out, 3, "hfb_check_constant_division",
+                  [&](unsigned long long* d) { return hfb::launchConstDivCheck(c, d); });
+}
+
+int hfb_check_shared_quotients(HfbCtx* c, uint64_t out[4]) {
+  HFB_CHECK_CTX(c);
+  return runCheck(c, out, 4, "hfb_check_shared_quotients",
+                  [&](unsigned long long* d) { return hfb::launchQuotientCheck(c, d); });
 }
 
 int hfb_buffer_alloc(HfbCtx* c, size_t bytes, void** out) {

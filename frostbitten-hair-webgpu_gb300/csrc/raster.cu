@@ -1469,7 +1469,10 @@ __device__ __forceinline__ uint2 fragmentColour(const FineSmem<TS>& sh, uint32_t
   float alpha = fsub(1.0f, fabsf(fsub(fmul(w.x, 2.0f), 1.0f)));
   if (alphaQuadratic) alpha = sqrtf(alpha);
   alpha = sat(fmul(alpha, alphaMul));
-  // (segment + w.y) / (P - 1): w.y is 0 or at least 2^-75, so divBy's quotient is the division's
+  // (segment + w.y) / (P - 1).  w.y is a quotient of a length, which is 0 or at least 2^-75, by
+  // the segment's: for segments up to 2^25 px it is 0 or at least DIV_TINY, and divBy's quotient is the
+  // division's; below (a numerator that only segment 0 has) it may miss one unit of 2^-149,
+  // which nothing of a colour in 16 bits (steps of 2^-24 at the least) shows
   const float tFull = divBy(fadd((float)(sh.enc[k] >> 24), w.y), {(float)(P - 1u), 1.0f / (float)(P - 1u)});
   uint32_t i0, i1;
   const float fr = remapToIndices(SP, tFull, i0, i1);

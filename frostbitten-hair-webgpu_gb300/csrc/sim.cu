@@ -843,7 +843,63 @@ __global__ void __launch_bounds__(256) constDivCheckKernel(unsigned long long* _
   if (bad6) atomicAdd(&cnt[2], bad6);
 }
 
+// Compares the quotients by a shared divisor (hfb_math.cuh) and the chains' overRoot with the
+// device's IEEE operations, over every float d with numerators from a hash of d's bits and from
+// the edges of what the forms take: cnt[0] rootRecip's root against sqrtf, cnt[1] overRoot
+// against x / sqrtf(d), cnt[2] divBy against x / d for x in its range, cnt[3] the quotients
+// by a root that took the short form (what the first two counts rest on).
+constexpr uint32_t QC_EDGES = 16, QC_RANDOM = 16;
+__global__ void __launch_bounds__(256) quotientCheckKernel(unsigned long long* __restrict__ cnt) {
+  unsigned long long badRoot = 0, badOver = 0, badDiv = 0, shortForm = 0;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  // numerators that differ in their last bits, and at the ends of the ranges
+  const uint32_t edges[QC_EDGES] = {0x3f800000u, 0x3f800001u, 0x3fffffffu, 0x3ffffffeu, 0x0d800000u, 0x0d7fffffu,
+                                    0x0d800001u, 0x4c000000u, 0x4c000001u, 0x4bffffffu, 0x00000000u, 0x00000001u,
+                                    0x007fffffu, 0x7f800000u, 0x7fc00000u, 0xbf800000u};
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (1ull << 32); i += stride) {
+    const float d = __uint_as_float((uint32_t)i);
+    Recip l;
+    const bool ok = rootRecip(d, l);
+    const float root = sqrtf(d);
+    if (ok) badRoot += __float_as_uint(l.d) != __float_as_uint(root);
+    const Recip r = recipOf(d);
+    const bool divides = r.y == r.y;  // d within recipOf's range
+    uint32_t h = (uint32_t)i * 0x9e3779b9u + 0x7f4a7c15u;
+#pragma unroll 1
+    for (uint32_t k = 0; k < QC_EDGES + QC_RANDOM; k++) {
+      h ^= h >> 15; h *= 0x2c1b3c6du; h ^= h >> 12; h *= 0x297a2d39u; h ^= h >> 15;
+      uint32_t xb = h;
+      if (k < QC_EDGES) xb = edges[k];
+      const float x = __uint_as_float(xb);
+      shortForm += ok && x >= DIV_TINY && x <= 0x1p25f;
+      const float q = overRoot(x, d), want = x / root;
+      badOver += __float_as_uint(q) != __float_as_uint(want) && (q == q || want == want);
+      if (divides) {
+        // exponents of x spread over [2^-100, 2^102): the quotients stay finite and normal
+        const float y = k < QC_EDGES ? x : __uint_as_float((xb & 0x807fffffu) | ((27u + (xb >> 23) % 202u) << 23));
+        const float b = fabsf(y), v = divBy(y, r), w = y / d;
+        if (b == 0.0f) badDiv += fabsf(v) != 0.0f;
+        else if (b >= DIV_TINY && b < 0x1p102f) badDiv += __float_as_uint(v) != __float_as_uint(w);
+      }
+    }
+  }
+  if (badRoot) atomicAdd(&cnt[0], badRoot);
+  if (badOver) atomicAdd(&cnt[1], badOver);
+  if (badDiv) atomicAdd(&cnt[2], badDiv);
+  atomicAdd(&cnt[3], shortForm);
+}
+
 }  // namespace
+
+cudaError_t launchQuotientCheck(HfbCtx* c, unsigned long long* cnt) {
+  HFB_CHECK_BIND(c);
+  cudaError_t e = cudaMemsetAsync(cnt, 0, 4 * sizeof(unsigned long long), c->stream);
+  if (e != cudaSuccess) return e;
+  quotientCheckKernel<<<c->smCount * 8u, 256, 0, c->stream>>>(cnt);
+  HFB_AFTER_LAUNCH(c, "quotientCheckKernel");
+  c->launches += 1;
+  return cudaGetLastError();
+}
 
 cudaError_t launchConstDivCheck(HfbCtx* c, unsigned long long* cnt) {
   HFB_CHECK_BIND(c);

@@ -198,6 +198,15 @@ HFB_API int hfb_get_counters(HfbCtx* ctx, HfbCounters* out);
  * int32 v, out[2] x / 1e6 over every finite float with |x| >= 2^-92.
  * Synchronizes. */
 HFB_API int hfb_check_constant_division(HfbCtx* ctx, uint64_t out[3]);
+/* Self-check of the quotients that the kernels form from a divisor's reciprocal
+ * or from one approximate reciprocal root (simulation chains, hair depth, tiles
+ * and fine passes), against the device's IEEE root and division, bit for bit:
+ * for every float d, 16 numerators from a hash of d and 16 at the edges of the
+ * forms' ranges.  Mismatch counts, all 0 expected: out[0] sqrt(d), out[1]
+ * x / sqrt(d), out[2] x / d for |d| in [2^-25, 2^25] and x = 0 or |x| in
+ * [2^-100, 2^102); out[3]: how many of out[1]'s quotients took the short form.
+ * Synchronizes. */
+HFB_API int hfb_check_shared_quotients(HfbCtx* ctx, uint64_t out[4]);
 
 /* ---- buffers ------------------------------------------------------------ */
 HFB_API int hfb_buffer_alloc(HfbCtx* ctx, size_t bytes, void** out);
