@@ -186,6 +186,12 @@ int hfb_check_shared_quotients(HfbCtx* c, uint64_t out[4]) {
                   [&](unsigned long long* d) { return hfb::launchQuotientCheck(c, d); });
 }
 
+int hfb_check_tone(HfbCtx* c, float power, uint64_t out[2]) {
+  HFB_CHECK_CTX(c);
+  return runCheck(c, out, 2, "hfb_check_tone",
+                  [&](unsigned long long* d) { return hfb::launchToneCheck(c, power, d); });
+}
+
 int hfb_buffer_alloc(HfbCtx* c, size_t bytes, void** out) {
   HFB_CHECK_CTX(c);
   HFB_REQUIRE(c, out, "out is NULL");

@@ -370,6 +370,7 @@ cudaError_t launchBatchSim(HfbCtx* c, const BatchView& b, BatchKind k);
 // hfb_check_constant_division: cnt[3] on the device, zeroed here
 cudaError_t launchConstDivCheck(HfbCtx* c, unsigned long long* cnt);
 cudaError_t launchQuotientCheck(HfbCtx* c, unsigned long long* cnt);
+cudaError_t launchToneCheck(HfbCtx* c, float power, unsigned long long* cnt);
 cudaError_t launchBatchShading(HfbCtx* c, const BatchView& b);
 cudaError_t launchBatchTiles(HfbCtx* c, const BatchView& b);
 cudaError_t launchBatchSort(HfbCtx* c, const BatchView& b);

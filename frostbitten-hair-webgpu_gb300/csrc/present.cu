@@ -42,7 +42,8 @@ static __device__ __noinline__ uint32_t toneExact(float x, float power) { return
 // 0.53 for r in [0, 1]), and powf and its products by less than 1e-4: farther than 5e-4 from a
 // rounding boundary the byte is decided.  One channel in 1,000 is not, and takes the exact way.
 constexpr float TONE_MARGIN = 5e-4f;
-__device__ __forceinline__ uint32_t tone(float x, float power, bool fast) {
+// False: not decided.  Compared with toneExact over every float by hfb_check_tone.
+__device__ __forceinline__ bool toneShort(float x, float power, uint32_t& byte) {
   const float num = fmul(x, fadd(fmul(2.51f, x), 0.03f));
   const float den = fadd(fmul(x, fadd(fmul(2.43f, x), 0.59f)), 0.14f);
   float rcp, lg, r;
@@ -53,10 +54,32 @@ __device__ __forceinline__ uint32_t tone(float x, float power, bool fast) {
   const float t = fmul(r, 255.0f);
   const float m = fadd(t, 12582912.0f);  // t rounded to the nearest whole number, in m's low bits
   // den within the approximate reciprocal's accuracy, v not tiny (a zero is exact either way)
-  const bool ok = fast && fabsf(den) >= 1e-30f && fabsf(den) <= 1e30f && (v >= 1e-30f || num == 0.0f) &&
-                  fabsf(fsub(t, fsub(m, 12582912.0f))) < 0.5f - TONE_MARGIN;
-  if (!ok) return toneExact(x, power);
-  return __float_as_uint(m) & 255u;
+  byte = __float_as_uint(m) & 255u;
+  return fabsf(den) >= 1e-30f && fabsf(den) <= 1e30f && (v >= 1e-30f || num == 0.0f) &&
+         fabsf(fsub(t, fsub(m, 12582912.0f))) < 0.5f - TONE_MARGIN;
+}
+__device__ __forceinline__ bool toneFast(float power) { return power > 0.0f && power <= 1.0f; }
+// fast: toneFast(power)
+__device__ __forceinline__ uint32_t tone(float x, float power, bool fast) {
+  uint32_t byte;
+  return fast && toneShort(x, power, byte) ? byte : toneExact(x, power);
+}
+
+// Compares the short form's bytes with toneExact's over every float: cnt[0] the ones that
+// differ, cnt[1] the values in [0, 16] that it decided.
+__global__ void __launch_bounds__(256) toneCheckKernel(float power, unsigned long long* __restrict__ cnt) {
+  unsigned long long bad = 0, decided = 0;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  if (toneFast(power))
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (1ull << 32); i += stride) {
+      const float x = __uint_as_float((uint32_t)i);
+      uint32_t byte;
+      if (!toneShort(x, power, byte)) continue;
+      bad += byte != toneExact(x, power);
+      decided += x >= 0.0f && x <= 16.0f;
+    }
+  if (bad) atomicAdd(&cnt[0], bad);
+  if (decided) atomicAdd(&cnt[1], decided);
 }
 
 // One image of a launch; it takes the launch's blocks [first, first + blocks).
@@ -78,7 +101,7 @@ __device__ __forceinline__ void presentBlock(const PresentImage m, uint32_t blk,
   __syncthreads();
   const uint32_t n = m.W * m.H, W = m.W;
   const float power = m.power, exposure = m.exposure, ditherStr = m.dither;
-  const bool fast = power > 0.0f && power <= 1.0f;
+  const bool fast = toneFast(power);
   uint32_t i = blk * PRESENT_PIXELS + threadIdx.x;
   uint32_t y = i / W, x = i - y * W;  // y: row from the top
   const uint32_t dy = PRESENT_THREADS / W, dx = PRESENT_THREADS - dy * W;
@@ -129,6 +152,16 @@ __global__ void __launch_bounds__(PRESENT_THREADS) presentBatchKernel(const Pres
 }
 
 }  // namespace
+
+cudaError_t launchToneCheck(HfbCtx* c, float power, unsigned long long* cnt) {
+  HFB_CHECK_BIND(c);
+  cudaError_t e = cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned long long), c->stream);
+  if (e != cudaSuccess) return e;
+  toneCheckKernel<<<c->smCount * 8u, 256, 0, c->stream>>>(power, cnt);
+  HFB_AFTER_LAUNCH(c, "toneCheckKernel");
+  c->launches += 1;
+  return cudaGetLastError();
+}
 
 cudaError_t launchPresent(HfbCtx* c, const HfbUniforms& u, uint32_t W, uint32_t H, const float* result,
                           const float* scene, uint8_t* rgba) {

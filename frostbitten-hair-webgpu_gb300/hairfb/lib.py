@@ -87,6 +87,7 @@ SIGNATURES = {
     "hfb_get_counters": (I, [P, P]),
     "hfb_check_constant_division": (I, [P, P]),
     "hfb_check_shared_quotients": (I, [P, P]),
+    "hfb_check_tone": (I, [P, ctypes.c_float, P]),
     "hfb_buffer_alloc": (I, [P, SZ, P]),
     "hfb_buffer_free": (I, [P, P]),
     "hfb_buffer_upload": (I, [P, P, P, SZ]),

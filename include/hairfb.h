@@ -207,6 +207,12 @@ HFB_API int hfb_check_constant_division(HfbCtx* ctx, uint64_t out[3]);
  * [2^-100, 2^102); out[3]: how many of out[1]'s quotients took the short form.
  * Synchronizes. */
 HFB_API int hfb_check_shared_quotients(HfbCtx* ctx, uint64_t out[4]);
+/* Self-check of the present pass's tone mapping: the bytes that its approximate
+ * units decide, for every float as the exposed channel and the given power (1 /
+ * gamma), against the exact operations: out[0] the bytes that differ (0
+ * expected), out[1] how many of the values in [0, 16] were decided.
+ * Synchronizes. */
+HFB_API int hfb_check_tone(HfbCtx* ctx, float power, uint64_t out[2]);
 
 /* ---- buffers ------------------------------------------------------------ */
 HFB_API int hfb_buffer_alloc(HfbCtx* ctx, size_t bytes, void** out);

@@ -46,3 +46,16 @@ def test_tone_of_every_kind_of_value(gamma, size):
     assert clear.mean() > 0.98
     assert np.array_equal(g[:, :3][clear], np.rint(t)[clear].astype(np.uint8))
     assert (g[:, 3] == 255).all()
+
+
+@pytest.mark.parametrize("power", [1.0 / 2.2, 1.0, 0.999, 0.5, 1.0 / 3.5, 0.04, 1e-3, 1e-6, 1e-30, 1e-42])
+def test_short_form_gives_the_exact_bytes(power):
+    """Every float: a byte that the approximate units decide is the exact operations'."""
+    import ctypes
+    ctx = Context(small_instance(strands=4).cfg.to_c(), 0)
+    out = (ctypes.c_uint64 * 2)()
+    ctx.call("hfb_check_tone", power, out)
+    assert out[0] == 0, f"{out[0]} bytes differ"
+    # about 1 in 1,000 is left to the exact way, and what rounds to a tone below 1e-30
+    assert out[1] > 0.6 * np.float32(16.0).view(np.uint32)
+    ctx.close()
