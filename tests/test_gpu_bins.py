@@ -72,3 +72,23 @@ def test_split_tiles_drawn_in_order(oracle, tile, slices, avg, bins):  # noqa: F
         assert np.array_equal(rb.read_result()[4:].reshape(-1, 4), g)
         again = ctx.counters()
         assert all(again[k] == cnt[k] for k in ("fineSplitTiles", "fineSplitRedone", "finePoolFullBins"))
+
+
+CLASSES = ((1, 8), (9, 32), (33, 256), (257, 1024), (1025, 16384), (16385, 1 << 24))
+
+
+@pytest.mark.parametrize("strands,points,size,tile,bins,classes", [
+    (6000, 32, (320, 240), 16, 16, (0, 1, 2, 3)), (60000, 16, (192, 160), 32, 4, (1, 2, 3, 4, 5))])
+def test_lists_of_every_class(oracle, strands, points, size, tile, bins, classes):  # noqa: F811
+    """Bins for each way to sort one -- 8 lanes, a warp's registers, its shared memory, a block's, all of
+    a block's, sorted runs -- and that they are there."""
+    tiles = -(-size[0] // tile) * -(-size[1] // tile)
+    inst = small_instance(strands=strands, points=points, width=size[0], height=size[1], tile_size=tile,
+                          depth_bins=bins, avg_segments_per_tile=-(-4_000_000 // tiles))
+    fr = frame_of(inst)
+    ctx, hair, rb, d = _raster_gpu(inst, fr)
+    heads = rb.read_tiles().reshape(-1, 4)
+    n = heads[heads[:, 2] != 0, 3]  # the lists' lengths
+    for k in classes:
+        assert ((n >= CLASSES[k][0]) & (n <= CLASSES[k][1])).any(), f"no bin of {CLASSES[k]} records"
+    _compare_tiles(oracle, inst, fr, rb)
