@@ -284,6 +284,12 @@ __device__ __forceinline__ void blockQuad(const HdShared& sh, uint32_t k, Screen
   q[3] = unpackV(sh.vb[k + 1]);
 }
 
+// prim: the primitive index of triangle tr of the segment from point pt,
+// (strand * (P - 1) + segment) * 2 + tr, the order the reference draws them.
+__device__ __forceinline__ uint32_t primOf(uint32_t pt, uint32_t P, uint32_t tr) {
+  return ((pt - pt / P) << 1) | tr;
+}
+
 // One block of segment starts [blk * HD_SEGS, (blk + 1) * HD_SEGS): each
 // warp projects the two vertices of 32 consecutive points into shared
 // memory and its first 31 lanes own the segments from their point to the
@@ -301,12 +307,6 @@ __device__ __forceinline__ void blockQuad(const HdShared& sh, uint32_t k, Screen
 // (10,000 x 32 at 1920x1080), 1.79 -> 0.91 ms (200,000 x 32 at 4K), 1.51 -> 1.04 ms
 // (64 instances); with a struct per segment (128 bytes, so every lane in the same
 // banks) 67 us, 1.49 and 2.28 ms.
-// prim: the primitive index of triangle tr of the segment from point pt,
-// (strand * (P - 1) + segment) * 2 + tr, the order the reference draws them.
-__device__ __forceinline__ uint32_t primOf(uint32_t pt, uint32_t P, uint32_t tr) {
-  return ((pt - pt / P) << 1) | tr;
-}
-
 template <bool WIN>
 __device__ __forceinline__ void hairDepthBlock(const HdView& V, uint32_t P, uint32_t nPts,
                                                const float4* __restrict__ pos, const float4* __restrict__ tan,

@@ -218,7 +218,6 @@ enum FramePass : uint32_t {
   FP_FINE,          // HairFinePass
   FP_HAIR_DEPTH,    // HwHairPass's depth (only for instances with hairDepth)
   FP_SHADING,       // HairShadingPass
-  FP_COUNT
 };
 cudaError_t framePass(HfbCtx* c, HfbInstance* in, FramePass p);
 // One frame of one checked instance, on c->stream and the context's side stream.

@@ -1153,7 +1153,10 @@ template <int TS> struct FineDims;
 // a constant, not the occupancy, so that where a tile is split, and with it the last bits
 // of its pixels, does not depend on the build.  At 8 px the sizes leave room for 8 CTAs
 // of the batched kernel per SM (28,160 bytes each): 3.10 ms on the 64-instance frame
-// against 3.39 at 7.
+// against 3.39 at 7.  The single-instance kernel, with 1,184 bytes more for its copy of the
+// uniforms, has 7; 256 ROWS would give it the eighth, and the batched one nothing: draws of
+// 10,000 x 32 at 1920x1080 353 -> 350 us, of 200,000 x 32 at 4K 6.41 -> 6.75 ms, frames of 11,400 x 16
+// 340 -> 348 us, 16 instances in one batch 2.54 -> 2.59 ms.
 template <> struct FineDims<8> {
   static constexpr uint32_t STAGE = 64, PAIRS = 768, ROWS = 512, NSHADE = 3, CTAS[3] = {8, 6, 6};
 };
@@ -1506,16 +1509,19 @@ __device__ __forceinline__ float halfHi(uint32_t v) { return __half2float(__usho
 // pixel per slice, where the CTAs that the registers allow leave room for it: a
 // fragment then costs one load and one store, not a predicated blend of every slice,
 // and `touched` names the slices that hold anything: 153 -> 131 us on a frame of 11,400
-// x 32 at 1920x1080 (8 px tiles, 8 slices).  Else in registers: 8 px tiles with 4 slices
-// would lose one of 8 CTAs per SM, 16 px ones one of 3 (4 slices) or of 2 (16 slices),
-// and 32 px tiles have no room.
+// x 16 at 1920x1080 (8 px tiles, 32 bins, 8 slices).  16 slices at 8 px cost one of 6 CTAs per
+// SM and are faster all the same: draws of 10,000 x 32 at 1920x1080 433 -> 385 us, of 200,000 x
+// 32 at 4K 7.04 -> 6.46 ms, 16 instances in one batch 2.83 -> 2.69 ms.  Else in registers: 8 px
+// tiles with 4 slices would lose one of 8 CTAs per SM, 16 px ones one of 3 (4 slices) or of 2
+// (16 slices), and 32 px tiles have no room.
 template <int TS, int MAXL>
 constexpr bool FINE_SHARED_SLICES = (TS == 8 && MAXL >= 8) || (TS == 16 && MAXL == 8);
 template <int TS, int MAXL>
 constexpr size_t FINE_SMEM = sizeof(FineSmem<TS>) + (FINE_SHARED_SLICES<TS, MAXL> ? MAXL * TS * TS * sizeof(float4) : 0);
 
-// q + kk * acc with kk = 1 - q.a, the colours with one rounding; alpha, which decides when a pixel is
-// done, with the two of the reference's product and sum
+// q + kk * acc with kk = 1 - q.a.  The colours take one rounding (fused) where the reference's product
+// and sum take two: no bit of the lists or of coverage depends on them, and a colour is off by less.
+// Alpha, which decides when a pixel is done, takes the reference's two.
 __device__ __forceinline__ void blendOver(f4& acc, const f4 q, float kk) {
   acc.x = __fmaf_rn(kk, acc.x, q.x);
   acc.y = __fmaf_rn(kk, acc.y, q.y);

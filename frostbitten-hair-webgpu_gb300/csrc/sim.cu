@@ -945,8 +945,8 @@ cudaError_t launchSimIntegrate(HfbCtx* c, const HfbSimUniforms& u, const HfbHair
                                const int32_t* dv, const float* gw, const float* sdf, uint32_t sdfDims) {
   HFB_CHECK_BIND(c);
   const uint32_t S = h.strandsCount, P = h.pointsPerStrand;
-  // one instance alone rarely fills the GPU: its blocks take fewer strands
-  // (down to 8) until there are two per SM, so that more chains run at once
+  // one instance alone rarely fills the GPU: its blocks take fewer strands (down to
+  // 4), in whole waves of three blocks per SM, so that more chains run at once
   const uint32_t NB = simStrandsPerBlockFor(S, P, (uint32_t)c->smCount);
   const size_t smem = (size_t)NB * (P + 1u) * sizeof(float4) + (size_t)P * 4u;
   cudaError_t e = simSmemLimit((const void*)simIntegrateKernel, 0);

@@ -6,7 +6,8 @@ Each translation unit is compiled for sm_103a only, in parallel, then linked
 into ``hairfb/_lib/libhairfb.so``.  The library is compiled with
 ``-fmad=false -prec-div=true -prec-sqrt=true``: every kernel evaluates its
 fp32 expressions one IEEE operation at a time, which is what makes the
-integer outputs of the passes (tile lists, depth bounds, grids) reproducible.
+integer outputs of the passes (tile lists, depth bounds, grids) reproducible;
+multiply-adds are fused only where the source says so (hfb_math.cuh).
 """
 from __future__ import annotations
 
