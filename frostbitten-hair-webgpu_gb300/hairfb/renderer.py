@@ -129,7 +129,8 @@ class Renderer:
         if self.hair_depth is not None:
             self.hw_hair.cmd_draw_hair_depth(self.uniforms, self.hair, self.scene_depth, self.hair_depth, self.rb)
         if self.normals is not None:
-            self.normals.zero_()  # CONFIG.clearNormals
+            # CONFIG.clearNormals, on the context's stream like the passes around it
+            self.ctx.call("hfb_buffer_clear", ptr(self.normals), self.normals.numel() * 4)
             self.hw_hair.cmd_draw_hair_normals(self.uniforms, self.hair, self.hair_depth, self.normals, self.rb,
                                                self.winner)
             self.ao = AoPass(self.ctx).cmd_calc_ao(self.uniforms, self.hair_depth, self.normals,

@@ -156,3 +156,28 @@ def test_frames_captured_by_the_caller():
     want.frame()
     for a, b in zip(_state(got)[0], _state(want)[0]):
         assert np.array_equal(a, b)
+
+
+def test_normals_are_cleared_on_the_contexts_stream():
+    """A frame with AO on the context's own stream while torch's stream is busy: the normals are
+    cleared in turn with the passes, not whenever torch's stream gets to it."""
+    inst = small_instance()
+
+    def frames(busy):
+        ctx = Context(inst.cfg.to_c(), 0)
+        r = Renderer(inst, 0, ctx=ctx, hair_depth=True, ao=True)
+        torch.cuda.synchronize()
+        r.before_first_frame()
+        ctx.sync()
+        torch.cuda.synchronize()
+        if busy:
+            torch.cuda._sleep(100_000_000)  # about 50 ms
+        r.frame()
+        ctx.sync()
+        torch.cuda.synchronize()
+        return r.normals.cpu().numpy(), r.ao.cpu().numpy(), r.hair.shading.cpu().numpy()
+
+    want, got = frames(False), frames(True)
+    assert (want[0] != 0).any()
+    for a, b in zip(want, got):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
